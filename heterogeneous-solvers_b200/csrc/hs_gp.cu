@@ -130,9 +130,9 @@ hs_status cholesky_adjoint_impl(hs_ctx ctx, const double* L, double* Abar, const
     const int valid_last = (int)(ctx->N - (int64_t)(nb - 1) * bsz);
     hs_status st = launch_zero_diag_upper(ctx, Abar, s);
     if (st != HS_OK) return st;
-    // Y_k = L_kk^-T for every k in one batched substitution (the last block against a
-    // copy with a unit diagonal on its padding rows)
-    if ((st = launch_diag_inverses(ctx, L, w.Y, w.Dp, s)) != HS_OK) return st;
+    // Y_k = L_kk^-T for every k in one batched launch (identity on padding rows); w.T is
+    // free until the sweep
+    if ((st = launch_diag_inverses(ctx, L, w.Y, w.T, s)) != HS_OK) return st;
     for (int k = nb - 1; k >= 0; --k) {
         const int m = nb - k - 1;
         const int64_t dk = block_id(k, k, nb);

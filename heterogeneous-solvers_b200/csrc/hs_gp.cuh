@@ -49,8 +49,6 @@ hs_status launch_pad_unit_diag(hs_ctx ctx, const double* D, double* Dp, int vali
 hs_status launch_zero_diag_upper(hs_ctx ctx, double* Abar, cudaStream_t s);
 hs_status launch_identity(hs_ctx ctx, double* Y, cudaStream_t s);
 hs_status launch_sym_tril_half(hs_ctx ctx, const double* G, double* M, cudaStream_t s);
-// B <- B L^-T for `items` contiguous bsz x bsz blocks (k_factor.cu)
-hs_status launch_trsm_on(hs_ctx ctx, const double* L, int n, double* B, int items, cudaStream_t s);
 
 // workspace of the reverse sweep
 struct AdjointWork {

@@ -185,18 +185,48 @@ hs_status launch_update(hs_ctx ctx, double* A, int blockID, int blockRow, int sy
 // (SYRK on their diagonal blocks, GEMM below them)
 hs_status launch_update_cols(hs_ctx ctx, double* A, int blockID, int blockRow, int colStart, int colEnd,
                              cudaStream_t s);
+// one diagonal block of bsz 128 or 256 (k_diag.cu): L and its inverse in one launch
+struct DiagFactor {
+    const double* in64 = nullptr;  // the block, or
+    const float* in32 = nullptr;   // the same in FP32
+    double* L = nullptr;           // factor out
+    int in_place = 0;              // L is the packed matrix's own block: zeros above the diagonal, padding rows kept
+    int zeros = 1;                 // in place: also the zeros above the 32 x 32 diagonal blocks (0: the panel TRSM's)
+    double* Y = nullptr;           // L^-T, row major
+    int y_full = 0;                // Y: every zero below the diagonal (else those of its 64 x 64 diagonal blocks)
+    double* T = nullptr;           // bsz 256: 128 x 128 doubles of scratch
+    float *invHi = nullptr, *invLo = nullptr;  // L^-1 in FP32 and its low part under TF32
+    int zero_upper = 0;            // invHi / invLo: also the zeros above the diagonal
+    int record_neg = 0;            // record the most negative failing pivot in d_info[1]
+    int64_t row_base = 0;          // first global row of the block
+    int ctas = 8;                  // bsz 256: CTAs (one cluster) that share its products
+};
+hs_status launch_diag_factor(hs_ctx ctx, const DiagFactor& f, cudaStream_t s);
+// the factor's and the operators' form: in place, Y and T in the context's scratch
+// (kDiagScratchBlocks blocks from kSmallScratch: Y, then T)
+constexpr size_t kDiagScratchBlocks = 2;
+inline DiagFactor diag_factor_in_place(hs_ctx ctx, double* blk) {
+    DiagFactor f;
+    const size_t bb = (size_t)ctx->bsz * ctx->bsz;
+    f.in64 = f.L = blk;
+    f.in_place = 1;
+    f.Y = reinterpret_cast<double*>(static_cast<char*>(ctx->scratch) + kSmallScratch);
+    f.T = f.Y + bb;
+    return f;
+}
 // Y_k = L_kk^-T for all nb diagonal blocks of the packed factor L (Y: nb consecutive
-// blocks; pad: one block of scratch for a last block with padding rows)
-hs_status launch_diag_inverses(hs_ctx ctx, const double* L, double* Y, double* pad, cudaStream_t s);
+// blocks; T: 128 x 128 doubles of scratch a block, used for bsz 256)
+hs_status launch_diag_inverses(hs_ctx ctx, const double* L, double* Y, double* T, cudaStream_t s);
 // a whole forward (L^-1 in) or backward (L^-T in) sweep over the FP64 packed factor in
 // one cooperative launch, given Y_k = L_kk^-T (k_vector.cu)
 hs_status launch_sweep_whole_f64(hs_ctx ctx, const double* L, const double* Y, const double* in, double* out,
                                  int forward, unsigned epoch, unsigned* flags, int* err, cudaStream_t s);
-// X = L^-1 (row major) of one lower-triangular bsz x bsz block; Y is a block of scratch
-hs_status launch_diag_inverse(hs_ctx ctx, const double* Lkk, double* Y, double* X, cudaStream_t s);
-// B <- B X^T in place for blockCount consecutive blocks from firstBlock (bsz 128 or 256):
-// the panel TRSM on the FP64 tensor pipe, given X = L_kk^-1
-hs_status launch_trsm_dmma(hs_ctx ctx, double* A, int64_t firstBlock, int blockCount, const double* X,
+// Y = L^-T (row major) of one lower-triangular block (bsz 128 or 256; T: 128 x 128 of scratch)
+hs_status launch_diag_inverse(hs_ctx ctx, const double* Lkk, double* Y, double* T, cudaStream_t s);
+// B <- B Y in place for blockCount consecutive blocks from firstBlock (bsz 128 or 256):
+// the panel TRSM on the FP64 tensor pipe, given Y = L_kk^-T.  Lkk non-null: also writes
+// the zeros above that block's 32 x 32 diagonal blocks
+hs_status launch_trsm_dmma(hs_ctx ctx, double* A, int64_t firstBlock, int blockCount, const double* Y, double* Lkk,
                            cudaStream_t s);
 hs_status launch_symv(hs_ctx ctx, const double* A, const double* b, double* result, int bi0, int bj0, int nbi,
                       int nbj, int reset, double* dot_with /*nullable: also dot(result, dot_with) */,

@@ -112,11 +112,14 @@ __global__ void maxdiag_kernel(const double* __restrict__ A, int bsz, int nb, in
     }
 }
 
-// out[i] = float(in[i]), n even
-__global__ void f64_to_f32_copy_kernel(const double* __restrict__ in, float* __restrict__ out, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n / 2; i += (int64_t)gridDim.x * blockDim.x) {
-        const double2 v = reinterpret_cast<const double2*>(in)[i];
-        reinterpret_cast<float2*>(out)[i] = make_float2((float)v.x, (float)v.y);
+// FP32 copies of nb upper-triangular blocks (what is stored below the diagonal is not
+// read: zeros there)
+__global__ void upper_f32_copy_kernel(const double* __restrict__ in, float* __restrict__ out, int bsz, int nb) {
+    const int64_t n2 = (int64_t)nb * bsz * bsz / 2;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n2; i += (int64_t)gridDim.x * blockDim.x) {
+        const int e = (int)(2 * i % ((int64_t)bsz * bsz)), r = e / bsz, c = e % bsz;
+        const double2 v = c + 1 >= r ? reinterpret_cast<const double2*>(in)[i] : make_double2(0.0, 0.0);
+        reinterpret_cast<float2*>(out)[i] = make_float2(c >= r ? (float)v.x : 0.f, (float)v.y);
     }
 }
 
@@ -263,8 +266,8 @@ hs_status mixed_solve_impl(hs_ctx ctx, const double* K, const double* b, double*
     // the factor's own error), from the 16-bit panel area the factor no longer needs
     w.Y32 = reinterpret_cast<float*>(w.P16);
     ctx->launches += 1;
-    f64_to_f32_copy_kernel<<<grid_n((int64_t)nb * bsz * bsz / 2, ctx->num_sms), kThreads, 0, s>>>(
-        w.Yinv, w.Y32, (int64_t)nb * bsz * bsz);
+    upper_f32_copy_kernel<<<grid_n((int64_t)nb * bsz * bsz / 2, ctx->num_sms), kThreads, 0, s>>>(w.Yinv, w.Y32, bsz,
+                                                                                               nb);
     HS_CHECK_LAUNCH("Y32");
     {
         const int fg = mixed_fro_grid(total_blocks(nb));

@@ -15,7 +15,7 @@ struct MixedWork {
     float* LO = nullptr;    // low parts of two panel groups (slot set p: slots p nb..), then L_kk^-1 hi / lo
     double* Ld = nullptr;   // FP64 diagonal blocks of L (nb blocks; the lower triangle is written)
     double* Yinv = nullptr; // FP64 inverse diagonal blocks, Y_k = L_kk^-T (nb blocks)
-    double* S = nullptr;    // FP64 scratch block (POTRF)
+    double* T = nullptr;    // 128 x 128 doubles of scratch of the diagonal block at work
     __nv_bfloat16* P16 = nullptr;  // 16-bit (BF16 or FP16) split of two panel groups: set p hi blocks 2p nb.., lo (2p+1) nb..
     int* err = nullptr;     // [0] tensor-core tile timeout, [1] triangular-sweep timeout
     unsigned long long* tile_ctr = nullptr;  // tile counters of the trailing-update launches (zeroed per factor)
@@ -50,9 +50,6 @@ hs_status mixed_apply(hs_ctx ctx, MixedWork& w, double* b, double* tmp, cudaStre
 hs_status mixed_solve_impl(hs_ctx ctx, const double* K, const double* b, double* x, int precision, double tol,
                            int max_steps, hs_mixed_report* out, int acc_panels = 0);
 
-// TRSM of `items` bsz x bsz FP64 blocks stored contiguously at B against the
-// lower triangle L (bsz x bsz): B <- B L^-T
-hs_status launch_trsm_on(hs_ctx ctx, const double* L, int n, double* B, int items, cudaStream_t s);
 // a whole forward / backward sweep in one cooperative launch: out = L^-1 in or
 // L^-T in (block rows published through flags[] with value `epoch`; *err = 2 on a
 // wait that timed out)

@@ -107,23 +107,25 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
         return HS_OK;
     }
     // Tensor-core form with lookahead.  The panel TRSM is a product with
-    // X = L_kk^-1.  Per column k the trailing update runs in two launches: column
-    // k+1 first; then, while the rest of the update runs, POTRF(k+1), X and the
+    // Y = L_kk^-T.  Per column k the trailing update runs in two launches: column
+    // k+1 first; then, while the rest of the update runs, POTRF(k+1), Y and the
     // TRSM of column k+1 run on the high-priority side stream.  Every block sees
     // the same operations in the same order as without lookahead.
     const size_t bb = (size_t)bsz * bsz;
-    hs_status st = ensure_scratch(ctx, kSmallScratch + 2 * bb * sizeof(double));
+    hs_status st = ensure_scratch(ctx, kSmallScratch + kDiagScratchBlocks * bb * sizeof(double));
     if (st != HS_OK) return st;
-    double* Y = reinterpret_cast<double*>(static_cast<char*>(ctx->scratch) + kSmallScratch);
-    double* X = Y + bb;
     auto diag = [&](int k, cudaStream_t q) -> hs_status {
         const int blockID = diag_id(k);
-        hs_status s2 = launch_potrf(ctx, A, blockID, k, q);
+        DiagFactor f = diag_factor_in_place(ctx, A + (size_t)blockID * bb);
+        f.row_base = (int64_t)k * bsz;
+        f.zeros = k == nb - 1;
+        prof_begin(ctx, q, HS_KERNEL_POTRF);
+        hs_status s2 = launch_diag_factor(ctx, f, q);
         if (s2 != HS_OK) return s2;
+        const double n = bsz;
+        prof_end(ctx, q, HS_KERNEL_POTRF, n * n * n / 3.0, 2.0 * n * n * 8.0);
         const int cnt = nb - (k + 1);
-        if (cnt <= 0) return HS_OK;
-        if ((s2 = launch_diag_inverse(ctx, A + (size_t)blockID * bb, Y, X, q)) != HS_OK) return s2;
-        return launch_trsm_dmma(ctx, A, (int64_t)blockID + 1, cnt, X, q);
+        return launch_trsm_dmma(ctx, A, (int64_t)blockID + 1, cnt, f.Y, f.L, q);
     };
     if ((st = diag(0, s)) != HS_OK) return st;
     for (int k = 0; k + 1 < nb; ++k) {
@@ -155,15 +157,16 @@ hs_status solve_driver(hs_ctx ctx, const double* L, double* b) {
         // 2 nb dependent launches a sweep are latency-bound
         const size_t bb = (size_t)ctx->bsz * ctx->bsz;
         const int64_t n = (int64_t)nb * ctx->bsz;
-        const size_t ybytes = ((size_t)nb * bb + bb + (size_t)n) * sizeof(double);
+        const size_t tq = (size_t)nb * 128 * 128;  // a quadrant a block
+        const size_t ybytes = ((size_t)nb * bb + tq + (size_t)n) * sizeof(double);
         hs_status st = ensure_solvews(ctx, ybytes + 256 + (((size_t)nb * sizeof(unsigned) + 255) & ~size_t(255)));
         if (st != HS_OK) return st;
         double* Y = static_cast<double*>(ctx->solvews);
-        double* pad = Y + (size_t)nb * bb;
-        double* tmp = pad + bb;
+        double* T = Y + (size_t)nb * bb;
+        double* tmp = T + tq;
         int* err = reinterpret_cast<int*>(static_cast<char*>(ctx->solvews) + ybytes);
         unsigned* flags = reinterpret_cast<unsigned*>(static_cast<char*>(ctx->solvews) + ybytes + 256);
-        if ((st = launch_diag_inverses(ctx, L, Y, pad, s)) != HS_OK) return st;
+        if ((st = launch_diag_inverses(ctx, L, Y, T, s)) != HS_OK) return st;
         HS_CUDA(cudaMemsetAsync(flags, 0, (size_t)nb * sizeof(unsigned), s));
         HS_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
         if ((st = launch_sweep_whole_f64(ctx, L, Y, b, tmp, 1, 1u, flags, err, s)) != HS_OK) return st;

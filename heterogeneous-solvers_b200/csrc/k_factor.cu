@@ -8,11 +8,12 @@
 //   MatrixMatrixOperations.cpp:364-906  matrixMatrixStep{,...}
 //
 // The trailing update is the only O(N^3) part.  For bsz a multiple of 128 it
-// runs on the FP64 tensor pipe (DMMA, mma.sync m8n8k4 f64): 128x128 output
-// tiles per CTA, K streamed in 16-wide slabs through a 4-stage cp.async ring in
+// runs on the FP64 tensor pipe (DMMA, mma.sync m8n8k4 f64): 128x64 output tiles,
+// two CTAs an SM, K streamed in 16-wide slabs through a 3-stage cp.async ring in
 // shared memory, accumulators held in registers and initialised with -C so the
 // result is C - sum_k a_ik b_jk accumulated in k order.  Other block sizes use
-// a scalar fallback with the reference's accumulation order.
+// a scalar fallback with the reference's accumulation order.  The diagonal block
+// of bsz 128 and 256 is k_diag.cu's.
 #include "hs_internal.cuh"
 #include "hs_mixed.cuh"
 
@@ -86,11 +87,6 @@ __global__ void __launch_bounds__(1024) potrf_global_kernel(double* __restrict__
     }
 }
 
-__global__ void zero_tile_kernel(double* __restrict__ P, int ld, int rows, int cols) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * cols; e += gridDim.x * blockDim.x)
-        P[(size_t)(e / cols) * ld + (e % cols)] = 0.0;
-}
-
 // ------------------------------------------------------------------ TRSM
 // B <- B L^-T for slabs of up to 64 rows: each CTA keeps its slab in shared
 // memory and walks the columns in 32-wide chunks: solve the chunk against the
@@ -106,13 +102,10 @@ struct TrsmArgs {
     int n;             // triangle size = columns of B
     double* A;         // base for B items
     int ldB;
-    int64_t item0;     // panel mode: first B block id; sub mode: ignored
+    int64_t item0;     // first B block id
     int slabs;         // slabs per B item
-    int rows_last;     // rows in each item (bsz or sub-block rows)
-    int64_t block_elems;  // panel mode: stride between B blocks (elements); 0: single item at A
-    int l_diag_nb;        // > 0: item q solves against its own triangle, the diagonal block q of the
-                          // packed matrix at L with this many block columns (L = its base)
-    int slab_rows;        // rows of B a CTA solves (0: kTrsmRows); fewer rows, more CTAs an item
+    int rows_last;     // rows in each item
+    int64_t block_elems;  // stride between B blocks (elements)
 };
 
 __global__ void __launch_bounds__(256) trsm_kernel(TrsmArgs a) {
@@ -124,10 +117,9 @@ __global__ void __launch_bounds__(256) trsm_kernel(TrsmArgs a) {
     double* Lp = Tc + kTrsmCh * (kTrsmCh + 1);        // n x (kTrsmCh+1)
     const int item = blockIdx.x / a.slabs;
     const int slab = blockIdx.x % a.slabs;
-    const double* Lt = a.l_diag_nb > 0 ? a.L + (size_t)column_start(item, a.l_diag_nb) * n * n : a.L;
-    const int sr = a.slab_rows > 0 ? a.slab_rows : kTrsmRows;
-    double* B = a.A + (a.block_elems ? (size_t)(a.item0 + item) * a.block_elems : 0) + (size_t)slab * sr * a.ldB;
-    const int rows = min(sr, a.rows_last - slab * sr);
+    const double* Lt = a.L;
+    double* B = a.A + (size_t)(a.item0 + item) * a.block_elems + (size_t)slab * kTrsmRows * a.ldB;
+    const int rows = min(kTrsmRows, a.rows_last - slab * kTrsmRows);
     for (int e = threadIdx.x; e < rows * n; e += blockDim.x) {
         const int r = e / n, c = e % n;
         Bs[r * bld + c] = B[(size_t)r * a.ldB + c];
@@ -179,9 +171,7 @@ size_t trsm_smem(int n) {
 }
 
 // ------------------------------------------------------------------ DMMA tile
-constexpr int BM = 128, BN = 128, BK = 16, STAGES = 4, SPAD = 20;
-constexpr int kTileSmem = 2 * STAGES * BM * SPAD * (int)sizeof(double);  // 160 KB
-
+constexpr int BK = 16, SPAD = 20;
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -191,87 +181,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// C (128 x 128, ldc) -= A (128 x K, lda) * B (128 x K, ldb)^T; `lower`: only
-// entries with row >= col are written (diagonal tile of a diagonal block).
-__device__ __forceinline__ void dmma_tile(double* __restrict__ C, int64_t ldc, const double* __restrict__ Ag,
-                                          int64_t lda, const double* __restrict__ Bg, int64_t ldb, int K,
-                                          bool lower, double* smem) {
-    double* As = smem;                         // [STAGES][BM][SPAD]
-    double* Bs = smem + STAGES * BM * SPAD;    // [STAGES][BN][SPAD]
-    const int tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int wm = warp >> 2, wn = warp & 3;
-    const int g = lane >> 2, t = lane & 3;
-
-    double acc[8][4][2];
-#pragma unroll
-    for (int mi = 0; mi < 8; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-            const int r = wm * 64 + mi * 8 + g;
-            const int c = wn * 32 + ni * 8 + 2 * t;
-            const double2 v = *reinterpret_cast<const double2*>(C + (size_t)r * ldc + c);
-            acc[mi][ni][0] = -v.x;
-            acc[mi][ni][1] = -v.y;
-        }
-
-    const int ktiles = K / BK;
-    auto load_stage = [&](int stage, int kt) {
-        const int kc = kt * BK;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = tid + 256 * q;
-            const int row = e >> 3, ch = e & 7;
-            cp_async16(As + (stage * BM + row) * SPAD + ch * 2, Ag + (size_t)row * lda + kc + ch * 2);
-            cp_async16(Bs + (stage * BN + row) * SPAD + ch * 2, Bg + (size_t)row * ldb + kc + ch * 2);
-        }
-    };
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < ktiles) load_stage(s, s);
-        cp_async_commit();
-    }
-    for (int kt = 0; kt < ktiles; ++kt) {
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();
-        {
-            const int nk = kt + STAGES - 1;
-            if (nk < ktiles) load_stage(nk % STAGES, nk);
-            cp_async_commit();
-        }
-        const double* as = As + (kt % STAGES) * BM * SPAD + (wm * 64 + g) * SPAD + t;
-        const double* bs = Bs + (kt % STAGES) * BN * SPAD + (wn * 32 + g) * SPAD + t;
-#pragma unroll
-        for (int kk = 0; kk < BK / 4; ++kk) {
-            double a[8], b[4];
-#pragma unroll
-            for (int mi = 0; mi < 8; ++mi) a[mi] = as[mi * 8 * SPAD + kk * 4];
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) b[ni] = bs[ni * 8 * SPAD + kk * 4];
-#pragma unroll
-            for (int mi = 0; mi < 8; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
-        }
-    }
-    cp_async_wait<0>();
-    __syncthreads();  // the ring is reused by the CTA's next tile
-#pragma unroll
-    for (int mi = 0; mi < 8; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-            const int r = wm * 64 + mi * 8 + g;
-            const int c = wn * 32 + ni * 8 + 2 * t;
-            double* p = C + (size_t)r * ldc + c;
-            if (!lower || c + 1 <= r) {
-                *reinterpret_cast<double2*>(p) = make_double2(-acc[mi][ni][0], -acc[mi][ni][1]);
-            } else if (c <= r) {
-                p[0] = -acc[mi][ni][0];
-            }
-        }
-}
-
-// ------------------------------------------------------ templated DMMA tiles
 // A CTA computes a TM x TN output tile with (TM/WM) x (TN/WN) warps of WM x WN
 // (m8n8k4 sub-tiles), K streamed in 16-wide slabs through an ST-stage cp.async
 // ring with rows padded to SPAD doubles (row stride 40 banks: the eight rows a
@@ -281,7 +190,9 @@ struct DTile {
     static constexpr int kWarpsN = TN / WN;
     static constexpr int kThreads = 32 * (TM / WM) * (TN / WN);
     static constexpr int kMi = WM / 8, kNi = WN / 8;
-    static constexpr int kSmem = ST * (TM + TN) * SPAD * (int)sizeof(double);
+    static constexpr int kBRow = TN + 4;  // PRODUCT: B k-major, rows of 4 k 32 bytes apart modulo 128
+    static constexpr int kBStage = TN * SPAD > BK * kBRow ? TN * SPAD : BK * kBRow;
+    static constexpr int kSmem = ST * (TM * SPAD + kBStage) * (int)sizeof(double);
     static constexpr int kChunks = (TM + TN) * (BK / 2);  // 16-byte copies a stage
     static_assert(kChunks % kThreads == 0, "copies must split evenly over the threads");
     static_assert((TM * (BK / 2)) % 32 == 0, "A and B copies must not share a warp");
@@ -290,9 +201,10 @@ struct DTile {
 // PRODUCT = false: C (TM x TN, ldc) <- C - A (TM x K, lda) B (TN x K, ldb)^T,
 //   accumulated from -C in k order; with `lower`, entry (r, c) is written only
 //   if c + shift <= r (a tile that crosses the diagonal of a diagonal block).
-// PRODUCT = true: C <- A B^T with B lower triangular by rows (B[c][k] = 0 for
-//   k > c): a warp skips the K slabs past its last column.  C may be A itself:
-//   every load of A completes before the first store.
+// PRODUCT = true: C <- A B with B (K x TN, ldb) upper triangular (B[k][c] = 0 for
+//   k > c): a warp skips the K slabs past its last column, and what B holds below its
+//   WN x WN diagonal blocks is not used.  C may be A itself: every load of A completes
+//   before the first store.
 template <int TM, int TN, int WM, int WN, int ST, bool PRODUCT>
 __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double* Ag, int64_t lda,
                                             const double* __restrict__ Bg, int64_t ldb, int K, bool lower, int shift,
@@ -322,7 +234,7 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
         }
 
     const int ktiles = K / BK;
-    // PRODUCT: rows wn*WN .. wn*WN+WN-1 of B vanish past column wn*WN+WN-1
+    // PRODUCT: columns wn*WN .. wn*WN+WN-1 of B vanish past row wn*WN+WN-1
     const int kt_warp = PRODUCT ? min(ktiles, (wn * WN + WN + BK - 1) / BK) : ktiles;
     auto load_stage = [&](int stage, int kt) {
         const int kc = kt * BK;
@@ -330,10 +242,15 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
         for (int q = 0; q < D::kChunks / D::kThreads; ++q) {
             const int e = tid + D::kThreads * q;
             const int row = e >> 3, ch = e & 7;
-            if (row < TM)
+            if (row < TM) {
                 cp_async16(As + (stage * TM + row) * SPAD + ch * 2, Ag + (size_t)row * lda + kc + ch * 2);
-            else
-                cp_async16(Bs + (stage * TN + row - TM) * SPAD + ch * 2, Bg + (size_t)(row - TM) * ldb + kc + ch * 2);
+            } else if (PRODUCT) {
+                const int eb = e - TM * (BK / 2), kr = eb / (TN / 2), cc = 2 * (eb % (TN / 2));
+                cp_async16(Bs + stage * D::kBStage + kr * D::kBRow + cc, Bg + (size_t)(kc + kr) * ldb + cc);
+            } else {
+                cp_async16(Bs + stage * D::kBStage + (row - TM) * SPAD + ch * 2,
+                           Bg + (size_t)(row - TM) * ldb + kc + ch * 2);
+            }
         }
     };
 #pragma unroll
@@ -351,14 +268,15 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
         }
         if (kt < kt_warp) {
             const double* as = As + (kt % ST) * TM * SPAD + (wm * WM + g) * SPAD + t;
-            const double* bs = Bs + (kt % ST) * TN * SPAD + (wn * WN + g) * SPAD + t;
+            const double* bs = Bs + (kt % ST) * D::kBStage +
+                               (PRODUCT ? t * D::kBRow + wn * WN + g : (wn * WN + g) * SPAD + t);
 #pragma unroll
             for (int kk = 0; kk < BK / 4; ++kk) {
                 double a[D::kMi], b[D::kNi];
 #pragma unroll
                 for (int mi = 0; mi < D::kMi; ++mi) a[mi] = as[mi * 8 * SPAD + kk * 4];
 #pragma unroll
-                for (int ni = 0; ni < D::kNi; ++ni) b[ni] = bs[ni * 8 * SPAD + kk * 4];
+                for (int ni = 0; ni < D::kNi; ++ni) b[ni] = PRODUCT ? bs[kk * 4 * D::kBRow + ni * 8] : bs[ni * 8 * SPAD + kk * 4];
 #pragma unroll
                 for (int mi = 0; mi < D::kMi; ++mi)
 #pragma unroll
@@ -451,42 +369,32 @@ __global__ void __launch_bounds__(UTile::kThreads, 2) update_dmma_kernel(UpdateA
     dmma_tile_t<kUTM, kUTN, kUWM, kUWN, kUST, false>(C, a.bsz, Ag, a.bsz, Bg, a.bsz, a.bsz, lower, shift, smem);
 }
 
-// Panel TRSM as a tensor-core product: B <- B X^T with X = L_kk^-1 (row major,
-// lower triangular), in place; one CTA per 64 rows of a panel block.
+// Panel TRSM as a tensor-core product: B <- B Y with Y = L_kk^-T (row major, upper
+// triangular), in place; one CTA per 64 rows of a panel block.
 template <int BSZ>
 struct TrsmTile {
     using T = DTile<64, BSZ, 32, BSZ / 4, 3>;
 };
 
 template <int BSZ>
-__global__ void __launch_bounds__(256, 1) trsm_dmma_kernel(double* A, int64_t firstBlock, const double* __restrict__ X) {
+__global__ void __launch_bounds__(256, 1) trsm_dmma_kernel(double* A, int64_t firstBlock, const double* __restrict__ Y,
+                                                           double* Lkk) {
     extern __shared__ __align__(16) double smem[];
+    if (Lkk) {
+        // the zeros above the 32 x 32 diagonal blocks of L_kk, off the chain that produced it
+        constexpr int kT = BSZ / 32, kPairs = kT * (kT - 1) / 2;
+        for (int u = blockIdx.x; u < kPairs; u += gridDim.x) {
+            const int c = tri_root(u) + 1, r = u - c * (c - 1) / 2;  // r < c
+            for (int e = threadIdx.x; e < 512; e += 256)
+                *reinterpret_cast<double2*>(Lkk + (size_t)(32 * r + e / 16) * BSZ + 32 * c + 2 * (e % 16)) =
+                    make_double2(0.0, 0.0);
+        }
+    }
     constexpr int kSlabs = BSZ / 64;
     const int64_t item = blockIdx.x / kSlabs;
     const int slab = blockIdx.x % kSlabs;
     double* B = A + (size_t)(firstBlock + item) * BSZ * BSZ + (size_t)slab * 64 * BSZ;
-    dmma_tile_t<64, BSZ, 32, BSZ / 4, 3, true>(B, BSZ, B, BSZ, X, BSZ, BSZ, false, 0, smem);
-}
-
-__global__ void identity_block_kernel(double* __restrict__ Y, int n) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x)
-        Y[e] = (e / n == e % n) ? 1.0 : 0.0;
-}
-
-// X = Y^T for one n x n block (32 x 32 tiles through shared memory)
-__global__ void transpose_block_kernel(const double* __restrict__ Y, double* __restrict__ X, int n) {
-    __shared__ double tile[32][33];
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) tile[i][threadIdx.x] = Y[(size_t)(by + i) * n + bx + threadIdx.x];
-    __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) X[(size_t)(bx + i) * n + by + threadIdx.x] = tile[threadIdx.x][i];
-}
-
-// single-tile form used inside the blocked POTRF of a 256 block
-__global__ void __launch_bounds__(256, 1) tile_update_kernel(double* C, int ldc, const double* Ag, const double* Bg,
-                                                             int ld, int K, int lower) {
-    extern __shared__ __align__(16) double smem[];
-    dmma_tile(C, ldc, Ag, ld, Bg, ld, K, lower != 0, smem);
+    dmma_tile_t<64, BSZ, 32, BSZ / 4, 3, true>(B, BSZ, B, BSZ, Y, BSZ, BSZ, false, 0, smem);
 }
 
 // scalar fallback (any bsz): one thread per output element; SYRK follows
@@ -526,7 +434,6 @@ hs_status set_attrs() {
                                  TrsmTile<128>::T::kSmem));
     HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  TrsmTile<256>::T::kSmem));
-    HS_CUDA(cudaFuncSetAttribute(tile_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem));
     HS_CUDA(cudaFuncSetAttribute(trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(256)));
     HS_CUDA(cudaFuncSetAttribute(potrf_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(128 * 129 * sizeof(double))));
@@ -561,33 +468,15 @@ static hs_status potrf_impl(hs_ctx ctx, double* A, int blockID, int blockRow, cu
     const long long row_base = (long long)blockRow * bsz;
     const int64_t rem = ctx->N - row_base;
     const int valid = rem <= 0 ? 0 : (rem < bsz ? (int)rem : bsz);
-    if (bsz <= 128) return potrf_small(ctx, blk, bsz, bsz, valid, row_base, s);
-    if (bsz == 256) {
-        // [A11 . ; A21 A22] with 128 x 128 quadrants: POTRF(A11), A21 <- A21 L11^-T,
-        // A22 -= A21 A21^T (lower, DMMA tile), POTRF(A22), zero the upper-right quadrant
-        const int n1 = 128, n2 = 128;
-        st = potrf_small(ctx, blk, bsz, n1, min(valid, n1), row_base, s);
+    if (bsz == 128 || bsz == 256) {
+        const size_t bb = (size_t)bsz * bsz;
+        st = ensure_scratch(ctx, kSmallScratch + kDiagScratchBlocks * bb * sizeof(double));
         if (st != HS_OK) return st;
-        double* A21 = blk + (size_t)n1 * bsz;
-        double* A22 = A21 + n1;
-        if (valid > n1) {
-            TrsmArgs ta{blk, bsz, n1, A21, bsz, 0, n2 / kTrsmRows, n2, 0};
-            st = launch_trsm_args(ctx, ta, 1, s);
-            if (st != HS_OK) return st;
-            ctx->launches += 1;
-            tile_update_kernel<<<1, 256, kTileSmem, s>>>(A22, bsz, A21, A21, bsz, n1, 1);
-            HS_CHECK_LAUNCH("potrf syrk");
-            st = potrf_small(ctx, A22, bsz, n2, valid - n1, row_base + n1, s);
-        } else {
-            // rows >= 128 are padding; the reference still writes sqrt(0) on their diagonal
-            st = potrf_small(ctx, A22, bsz, n2, 0, row_base + n1, s);
-        }
-        if (st != HS_OK) return st;
-        ctx->launches += 1;
-        zero_tile_kernel<<<16, 256, 0, s>>>(blk + n1, bsz, min(valid, n1), n2);
-        HS_CHECK_LAUNCH("potrf zero");
-        return HS_OK;
+        DiagFactor f = diag_factor_in_place(ctx, blk);
+        f.row_base = row_base;
+        return launch_diag_factor(ctx, f, s);
     }
+    if (bsz <= 128) return potrf_small(ctx, blk, bsz, bsz, valid, row_base, s);
     ctx->launches += 1;
     potrf_global_kernel<<<1, 1024, 0, s>>>(blk, bsz, valid, ctx->d_info, row_base);
     HS_CHECK_LAUNCH("potrf");
@@ -602,69 +491,7 @@ hs_status launch_potrf(hs_ctx ctx, double* A, int blockID, int blockRow, cudaStr
     return st;
 }
 
-hs_status launch_diag_inverse(hs_ctx ctx, const double* Lkk, double* Y, double* X, cudaStream_t s) {
-    // Y = I L^-T by the substitution kernel, X = Y^T = L^-1 (row major, lower triangular:
-    // every entry above the diagonal of Y comes out exactly zero)
-    const int n = ctx->bsz;
-    ctx->launches += 1;
-    identity_block_kernel<<<64, 256, 0, s>>>(Y, n);
-    HS_CHECK_LAUNCH("identity");
-    // one block on the critical path of the factor: 16 rows of Y a CTA (16 CTAs for
-    // bsz 256) instead of 64, the trailing products of a chunk spread 4x wider
-    constexpr int kRows = 16;
-    TrsmArgs ta{Lkk, n, n, Y, n, 0, (n + kRows - 1) / kRows, n, (int64_t)n * n, 0, kRows};
-    hs_status st = launch_trsm_args(ctx, ta, 1, s);
-    if (st != HS_OK) return st;
-    ctx->launches += 1;
-    transpose_block_kernel<<<dim3(n / 32, n / 32), dim3(32, 8), 0, s>>>(Y, X, n);
-    HS_CHECK_LAUNCH("transpose");
-    return HS_OK;
-}
-
-__global__ void identity_blocks_kernel(double* __restrict__ Y, int n, int64_t blocks) {
-    const int64_t total = (int64_t)n * n * blocks;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t w = e % ((int64_t)n * n);
-        Y[e] = (w / n == w % n) ? 1.0 : 0.0;
-    }
-}
-
-// P = the last diagonal block with a unit diagonal on its padding rows (valid < n)
-__global__ void pad_unit_block_kernel(const double* __restrict__ D, double* __restrict__ P, int n, int valid) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
-        const int i = e / n, j = e % n;
-        P[e] = (i < valid && j < valid) ? D[e] : (i == j ? 1.0 : 0.0);
-    }
-}
-
-hs_status launch_diag_inverses(hs_ctx ctx, const double* L, double* Y, double* pad, cudaStream_t s) {
-    // Y_k = L_kk^-T for every diagonal block: the substitution kernel on identity blocks,
-    // every item against its own triangle; the last block, when it has padding rows,
-    // against a copy with a unit diagonal there (its padding rows are never used)
-    hs_status st = set_attrs();
-    if (st != HS_OK) return st;
-    const int n = ctx->bsz, nb = ctx->nb;
-    const int64_t bb = (int64_t)n * n;
-    const int valid = (int)(ctx->N - (int64_t)(nb - 1) * n);
-    ctx->launches += 1;
-    identity_blocks_kernel<<<4 * ctx->num_sms, 256, 0, s>>>(Y, n, nb);
-    HS_CHECK_LAUNCH("identity blocks");
-    const int full = valid < n ? nb - 1 : nb;
-    if (full > 0) {
-        TrsmArgs ta{L, n, n, Y, n, 0, (n + kTrsmRows - 1) / kTrsmRows, n, bb, nb};
-        if ((st = launch_trsm_args(ctx, ta, full, s)) != HS_OK) return st;
-    }
-    if (full < nb) {
-        ctx->launches += 1;
-        pad_unit_block_kernel<<<64, 256, 0, s>>>(L + (size_t)column_start(nb - 1, nb) * bb, pad, n, valid);
-        HS_CHECK_LAUNCH("pad block");
-        TrsmArgs ta{pad, n, n, Y + (size_t)(nb - 1) * bb, n, 0, (n + kTrsmRows - 1) / kTrsmRows, n, bb, 0};
-        if ((st = launch_trsm_args(ctx, ta, 1, s)) != HS_OK) return st;
-    }
-    return HS_OK;
-}
-
-hs_status launch_trsm_dmma(hs_ctx ctx, double* A, int64_t firstBlock, int blockCount, const double* X,
+hs_status launch_trsm_dmma(hs_ctx ctx, double* A, int64_t firstBlock, int blockCount, const double* Y, double* Lkk,
                            cudaStream_t s) {
     if (blockCount <= 0) return HS_OK;
     hs_status st = set_attrs();
@@ -676,9 +503,9 @@ hs_status launch_trsm_dmma(hs_ctx ctx, double* A, int64_t firstBlock, int blockC
     ctx->launches += 1;
     const unsigned grid = (unsigned)((int64_t)blockCount * (bsz / 64));
     if (bsz == 256)
-        trsm_dmma_kernel<256><<<grid, 256, TrsmTile<256>::T::kSmem, s>>>(A, firstBlock, X);
+        trsm_dmma_kernel<256><<<grid, 256, TrsmTile<256>::T::kSmem, s>>>(A, firstBlock, Y, Lkk);
     else
-        trsm_dmma_kernel<128><<<grid, 256, TrsmTile<128>::T::kSmem, s>>>(A, firstBlock, X);
+        trsm_dmma_kernel<128><<<grid, 256, TrsmTile<128>::T::kSmem, s>>>(A, firstBlock, Y, Lkk);
     HS_CHECK_LAUNCH("trsm_dmma");
     // algorithmic work: the triangular solve's n^3 flops a block
     prof_end(ctx, s, HS_KERNEL_TRSM, blockCount * n * n * n, (2.0 * blockCount + 1.0) * n * n * 8.0);
@@ -694,14 +521,13 @@ hs_status launch_trsm(hs_ctx ctx, double* A, int blockID, int blockRow, int bloc
     HS_REQUIRE(bsz <= 256, "TRSM supports matrixBlockSize up to 256");
     const size_t bb = (size_t)bsz * bsz;
     if (bsz == 128 || bsz == 256) {
-        // on the FP64 tensor pipe: X = L_kk^-1 once, then B <- B X^T block by block
-        st = ensure_scratch(ctx, kSmallScratch + 2 * bb * sizeof(double));
+        // on the FP64 tensor pipe: Y = L_kk^-T once, then B <- B Y block by block
+        st = ensure_scratch(ctx, kSmallScratch + kDiagScratchBlocks * bb * sizeof(double));
         if (st != HS_OK) return st;
         double* Y = reinterpret_cast<double*>(static_cast<char*>(ctx->scratch) + kSmallScratch);
-        double* X = Y + bb;
-        st = launch_diag_inverse(ctx, A + (size_t)blockID * bb, Y, X, s);
+        st = launch_diag_inverse(ctx, A + (size_t)blockID * bb, Y, Y + bb, s);
         if (st != HS_OK) return st;
-        return launch_trsm_dmma(ctx, A, (int64_t)blockID + (blockStart - blockRow), blockCount, X, s);
+        return launch_trsm_dmma(ctx, A, (int64_t)blockID + (blockStart - blockRow), blockCount, Y, nullptr, s);
     }
     TrsmArgs ta{A + (size_t)blockID * bb, bsz, bsz, A, bsz, (int64_t)blockID + (blockStart - blockRow),
                 (bsz + kTrsmRows - 1) / kTrsmRows, bsz, (int64_t)bb};
@@ -710,13 +536,6 @@ hs_status launch_trsm(hs_ctx ctx, double* A, int blockID, int blockRow, int bloc
     st = launch_trsm_args(ctx, ta, blockCount, s);
     prof_end(ctx, s, HS_KERNEL_TRSM, blockCount * n * n * n, (2.0 * blockCount + 1.0) * n * n * 8.0);
     return st;
-}
-
-hs_status launch_trsm_on(hs_ctx ctx, const double* L, int n, double* B, int items, cudaStream_t s) {
-    hs_status st = set_attrs();
-    if (st != HS_OK) return st;
-    TrsmArgs ta{L, n, n, B, n, 0, (n + kTrsmRows - 1) / kTrsmRows, n, (int64_t)n * n};
-    return launch_trsm_args(ctx, ta, items, s);
 }
 
 namespace {

@@ -805,371 +805,6 @@ __global__ void lo_part_kernel(const float* __restrict__ a, float* __restrict__ 
     }
 }
 
-// ------------------------------------------------------------------ diagonal chain
-// The FP64 work on one diagonal block in a single CTA: Cholesky of the FP32 block
-// (lower triangle; rows / columns >= valid replaced by the identity) together with
-// X = L^-1, by one right-looking sweep over 32-column panels p:
-//   - the panel's 32 x 32 diagonal block D_p is factored by warp 0 in registers,
-//     column by column, and inverted in the same pass (lane = row of L_pp and
-//     column of X_pp = L_pp^-1; each column of L_pp is broadcast once for both);
-//   - block row p of X is X_pp B_p (B = the identity less the updates below) and
-//     the panel rows below the diagonal block become row X_pp^T;
-//   - rank-32 updates in 32 x 32 warp tiles on the FP64 tensor pipe (DMMA): the
-//     trailing lower triangle, S_rc -= L_rp L_cp^T, and the rows of B below,
-//     B_r -= L_rp X_p.  Warp 1 first computes the diagonal block of panel p+1 (the
-//     corner of the trailing triangle) and hands it to warp 0, which factors it
-//     while warps 1..7 update the rest.
-// S (the working matrix) and B (held transposed in Y, which ends as X^T) stay in
-// global memory (L2-resident; S is read from the FP32 block directly at panel 0);
-// the panel is staged in shared memory k-major, block row p of B / X as [a][c].
-// Outputs: L's lower triangle in FP64 in Ld (the solves read its diagonal for log|K|,
-// the mixed NLML the whole block; the FP32 block keeps its input), Y = X^T,
-// invHi = float(X), invLo = invHi - tf32(invHi).
-// A pivot that is not > 0 on a valid row records its global row in *info.
-constexpr int kChainThreads = 256;
-
-template <int BSZ>
-struct ChainSmem {
-    static constexpr int kP = BSZ / 32;       // panels
-    static constexpr int kLt = BSZ - 32 + 4;  // k-major panel stride (rows below the diagonal block)
-    static constexpr int kXr = BSZ + 4;       // block-row stride
-    static constexpr int kD = 33;             // diagonal block / inverse stride
-    static constexpr size_t kBytes = (size_t)(32 * kLt + 32 * kXr + 2 * 32 * kD + 64) * sizeof(double);
-};
-
-// two / four consecutive entries (r, c..) of the working matrix: the FP32 block with
-// the identity outside the valid range (panel 0), else S
-template <int BSZ>
-__device__ __forceinline__ void chain_src4(const float* __restrict__ blk, const double* __restrict__ S, bool first,
-                                           int valid, int r, int c, double v[4]) {
-    if (first) {
-        const float4 f = *reinterpret_cast<const float4*>(blk + (size_t)r * BSZ + c);
-        const float fv[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = (r >= valid || c + q >= valid) ? (r == c + q ? 1.0 : 0.0) : (double)fv[q];
-    } else {
-        const double2 a = *reinterpret_cast<const double2*>(S + (size_t)r * BSZ + c);
-        const double2 b = *reinterpret_cast<const double2*>(S + (size_t)r * BSZ + c + 2);
-        v[0] = a.x;
-        v[1] = a.y;
-        v[2] = b.x;
-        v[3] = b.y;
-    }
-}
-
-template <int BSZ>
-__device__ __forceinline__ double2 chain_src2(const float* __restrict__ blk, const double* __restrict__ S, bool first,
-                                              int valid, int r, int c) {
-    if (first) {
-        const float2 f = *reinterpret_cast<const float2*>(blk + (size_t)r * BSZ + c);
-        return make_double2((r >= valid || c >= valid) ? (r == c ? 1.0 : 0.0) : (double)f.x,
-                            (r >= valid || c + 1 >= valid) ? (r == c + 1 ? 1.0 : 0.0) : (double)f.y);
-    }
-    return *reinterpret_cast<const double2*>(S + (size_t)r * BSZ + c);
-}
-
-// warp 0: D (32 x 32, stride kD, lower triangle read) -> L_pp in D (upper part
-// zero) and Xp = L_pp^-1.  d0 = the block's first row within the diagonal block
-// of the matrix.
-__device__ __forceinline__ void chain_diag(double* __restrict__ D, double* __restrict__ Xp,
-                                           double* __restrict__ colb, int lane, int d0, int valid,
-                                           long long* __restrict__ info, long long row_base) {
-    constexpr int kD = 33;
-    double x[32], z[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        x[j] = j <= lane ? D[lane * kD + j] : 0.0;
-        z[j] = j == lane ? 1.0 : 0.0;
-    }
-    // the pivot of step k+1 is taken from lane k+1 as soon as that lane has its own
-    // L[k+1][k], ahead of the column broadcast through shared memory
-    double piv = __shfl_sync(0xffffffffu, x[0], 0);
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-        if (lane == 0 && d0 + k < valid && !(piv > 0.0)) {
-            atomicMin(info, row_base + d0 + k);
-            // info[1]: the most negative failing pivot (bit pattern of a negative double;
-            // a larger signed pattern is a larger magnitude); NaN and zero pivots are not
-            // recorded
-            if (piv < 0.0) atomicMax(info + 1, __double_as_longlong(piv));
-        }
-        const double ri = rsqrt(piv);
-        const double lk = lane == k ? piv * ri : (lane > k ? x[k] * ri : 0.0);  // L[lane][k]
-        const double zk = z[k] * ri;                                            // X[k][lane]
-        x[k] = lk;
-        z[k] = zk;
-        if (k + 1 < 32) piv = __shfl_sync(0xffffffffu, x[k + 1] - lk * lk, k + 1);
-        double* cb = colb + 32 * (k & 1);
-        cb[lane] = lk;
-        __syncwarp();
-#pragma unroll
-        for (int j = k + 1; j < 32; ++j) {
-            const double ljk = cb[j];
-            x[j] = x[j] - lk * ljk;
-            z[j] = z[j] - ljk * zk;
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        D[lane * kD + j] = x[j];
-        Xp[j * kD + lane] = z[j];
-    }
-}
-
-// one 32 x 32 warp tile of sum_k A[m][k] B[k][n] over K = 32 on the FP64 tensor
-// pipe: A[m][k] = pa[k * lda + m], B[k][n] = pb[k * ldb + n]; lane holds rows
-// 8 mi + lane/4, columns 8 ni + 2 (lane%4) + {0, 1}
-__device__ __forceinline__ void chain_wtile(const double* __restrict__ pa, int lda, const double* __restrict__ pb,
-                                            int ldb, int lane, double (&acc)[4][4][2]) {
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
-#pragma unroll
-    for (int k0 = 0; k0 < 32; k0 += 4) {
-        double a[4], b[4];
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi) a[mi] = pa[(k0 + t) * lda + 8 * mi + g];
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) b[ni] = pb[(k0 + t) * ldb + 8 * ni + g];
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
-    }
-}
-
-__device__ __forceinline__ void chain_bar(int id, int count) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-
-// block row p of X from shared memory -> Y (transposed; zero before column c0 in
-// the panel's rows of Y) and invHi / invLo (zero after column w when `zero_upper`:
-// the planes are shared by all diagonal blocks and only the first writes the part
-// above the block diagonal).  Threads `t0`, `t0 + nt`, ... take part.
-template <int BSZ>
-__device__ __forceinline__ void chain_outputs(double* __restrict__ Y, float* __restrict__ invHi,
-                                              float* __restrict__ invLo, const double* __restrict__ Xr, int c0,
-                                              bool zero_upper, int t0, int nt) {
-    using CS = ChainSmem<BSZ>;
-    constexpr int n = BSZ, kXr = CS::kXr;
-    const int w = c0 + 32;
-    for (int e = t0; e < w * 8; e += nt) {
-        const int c = e % w, a4 = e / w;
-        double v[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = Xr[(4 * a4 + q) * kXr + c];
-        *reinterpret_cast<double2*>(Y + (size_t)c * n + c0 + 4 * a4) = make_double2(v[0], v[1]);
-        *reinterpret_cast<double2*>(Y + (size_t)c * n + c0 + 4 * a4 + 2) = make_double2(v[2], v[3]);
-    }
-    for (int e = t0; e < 32 * c0 / 2; e += nt) {
-        const int c = c0 + (2 * e) / c0, r = (2 * e) % c0;
-        *reinterpret_cast<double2*>(Y + (size_t)c * n + r) = make_double2(0.0, 0.0);
-    }
-    const int cw = zero_upper ? n : w;  // columns written
-    for (int e = t0; e < 8 * cw; e += nt) {
-        const int a = e / (cw / 4), c = 4 * (e % (cw / 4));
-        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < w) {
-            const double* xr = Xr + a * kXr + c;
-            f = make_float4((float)xr[0], (float)xr[1], (float)xr[2], (float)xr[3]);
-        }
-        const size_t o = (size_t)(c0 + a) * n + c;
-        *reinterpret_cast<float4*>(invHi + o) = f;
-        *reinterpret_cast<float4*>(invLo + o) =
-            make_float4(f.x - tf32_trunc(f.x), f.y - tf32_trunc(f.y), f.z - tf32_trunc(f.z), f.w - tf32_trunc(f.w));
-    }
-}
-
-template <int BSZ>
-__global__ void __launch_bounds__(kChainThreads, 1)
-    diag_chain_kernel(const float* __restrict__ blk, double* __restrict__ S, double* __restrict__ Y,
-                      double* __restrict__ Ld, float* __restrict__ invHi, float* __restrict__ invLo, int valid,
-                      int zero_upper, long long* __restrict__ info, long long row_base) {
-    using CS = ChainSmem<BSZ>;
-    constexpr int n = BSZ, kLt = CS::kLt, kXr = CS::kXr, kD = CS::kD;
-    constexpr int kIt = (n * 8 + kChainThreads - 1) / kChainThreads;  // staging steps a thread
-    extern __shared__ double csm[];
-    double* PsT = csm;               // [k][rr - 32]: panel rows below the diagonal block
-    double* Xr = PsT + 32 * kLt;     // [a][c]: block row p of B, then of X
-    double* D = Xr + 32 * kXr;       // diagonal block of the current panel (L after warp 0)
-    double* Xp = D + 32 * kD;        // its inverse
-    double* colb = Xp + 32 * kD;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-    if (warp == 0) {  // D_0 from the FP32 block
-#pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-            double v[4];
-            chain_src4<BSZ>(blk, S, true, valid, lane, 4 * j4, v);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) D[lane * kD + 4 * j4 + q] = v[q];
-        }
-        __syncwarp();
-        chain_diag(D, Xp, colb, lane, 0, valid, info, row_base);
-    }
-    __syncthreads();
-
-    for (int p = 0; p < CS::kP; ++p) {
-        const int c0 = 32 * p, mb = n - c0 - 32, w = c0 + 32;
-        const bool first = p == 0;
-        {
-            // panel rows below the diagonal block, four columns a step (rows fastest),
-            // all loads of a thread in flight before the shared stores
-            double v[kIt][4];
-#pragma unroll
-            for (int u = 0; u < kIt; ++u) {
-                const int e = tid + u * kChainThreads;
-                if (e < mb * 8) chain_src4<BSZ>(blk, S, first, valid, c0 + 32 + e % mb, c0 + 4 * (e / mb), v[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < kIt; ++u) {
-                const int e = tid + u * kChainThreads;
-                if (e < mb * 8) {
-                    const int rr = e % mb, k4 = e / mb;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) PsT[(4 * k4 + q) * kLt + rr] = v[u][q];
-                }
-            }
-            // B_p[a][c]: columns before the panel from Y[c][c0 + a], the panel's own the identity
-#pragma unroll
-            for (int u = 0; u < kIt; ++u) {
-                const int e = tid + u * kChainThreads;
-                const int c = e % w, a4 = e / w;
-                if (e < w * 8) {
-                    if (c < c0) {
-                        const double2 x0 = *reinterpret_cast<const double2*>(Y + (size_t)c * n + c0 + 4 * a4);
-                        const double2 x1 = *reinterpret_cast<const double2*>(Y + (size_t)c * n + c0 + 4 * a4 + 2);
-                        v[u][0] = x0.x;
-                        v[u][1] = x0.y;
-                        v[u][2] = x1.x;
-                        v[u][3] = x1.y;
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) v[u][q] = (c - c0 == 4 * a4 + q) ? 1.0 : 0.0;
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kIt; ++u) {
-                const int e = tid + u * kChainThreads;
-                if (e < w * 8) {
-                    const int c = e % w, a4 = e / w;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) Xr[(4 * a4 + q) * kXr + c] = v[u][q];
-                }
-            }
-        }
-        __syncthreads();
-        if (tid < w) {
-            // column tid of block row p: X_p = X_pp B_p
-            double b[32], v[32];
-#pragma unroll
-            for (int a = 0; a < 32; ++a) {
-                b[a] = Xr[a * kXr + tid];
-                v[a] = 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < 32; ++q)
-#pragma unroll
-                for (int a = q; a < 32; ++a) v[a] = fma(Xp[a * kD + q], b[q], v[a]);
-#pragma unroll
-            for (int a = 0; a < 32; ++a) Xr[a * kXr + tid] = v[a];
-        } else if (tid < w + mb) {
-            // panel row below the diagonal block: row X_pp^T
-            const int rr = tid - w;
-            double x[32], v[32];
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-                x[k] = PsT[k * kLt + rr];
-                v[k] = 0.0;
-            }
-#pragma unroll
-            for (int k = 0; k < 32; ++k)
-#pragma unroll
-                for (int j = k; j < 32; ++j) v[j] = fma(x[k], Xp[j * kD + k], v[j]);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) PsT[j * kLt + rr] = v[j];
-        }
-        __syncthreads();
-        // panel p of L -> Ld in FP64 (its diagonal block from D, lower triangle, and the
-        // rows below from PsT; D is rewritten below); block row p of X goes out during
-        // the updates
-        for (int e = tid; e < 32 * 32; e += kChainThreads) {
-            const int i = e >> 5, j = e & 31;
-            if (j <= i) Ld[(size_t)(c0 + i) * n + c0 + j] = D[i * kD + j];
-        }
-        for (int e = tid; e < mb * 32; e += kChainThreads) {
-            const int k = e & 31, rr = e >> 5;
-            Ld[(size_t)(c0 + 32 + rr) * n + c0 + k] = PsT[k * kLt + rr];
-        }
-        if (mb == 0) {
-            chain_outputs<BSZ>(Y, invHi, invLo, Xr, c0, zero_upper != 0, tid, kChainThreads);
-            break;
-        }
-        __syncthreads();  // D, Xp are rewritten below
-        if (warp == 0) {
-            chain_bar(1, 64);  // warp 1 has written D of panel p+1
-            chain_diag(D, Xp, colb, lane, c0 + 32, valid, info, row_base);
-        } else {
-            // 32 x 32 warp tiles over warps 1..7: the trailing lower triangle (its
-            // corner, the diagonal block of panel p+1, first and into D), then the rows
-            // of B below block row p (in Y[c][r]; the panel's own columns are written
-            // for the first time)
-            const int g = lane >> 2, t = lane & 3;
-            const int q = mb >> 5, wq = w >> 5;
-            const int ntri = q * (q + 1) / 2;
-            const int ntiles = ntri + q * wq;
-            // warp 4 shares warp 0's scheduler and stays off the tile work
-            constexpr int kTw = kChainThreads / 32 - 2;
-            const int tw = warp < 4 ? warp - 1 : warp - 2;
-            double acc[4][4][2];
-            for (int u = tw; u < ntiles && warp != 4; u += kTw) {
-                if (u < ntri) {
-                    int R = (int)((sqrtf(8.0f * u + 1.0f) - 1.0f) * 0.5f);
-                    while (R * (R + 1) / 2 > u) --R;
-                    while ((R + 1) * (R + 2) / 2 <= u) ++R;
-                    const int C = u - R * (R + 1) / 2;
-                    chain_wtile(PsT + 32 * R, kLt, PsT + 32 * C, kLt, lane, acc);
-                    const int r0 = c0 + 32 + 32 * R, cc0 = c0 + 32 + 32 * C;
-#pragma unroll
-                    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                        for (int ni = 0; ni < 4; ++ni) {
-                            const int r = r0 + 8 * mi + g, c = cc0 + 8 * ni + 2 * t;
-                            const double2 sv = chain_src2<BSZ>(blk, S, first, valid, r, c);
-                            const double2 o = make_double2(sv.x - acc[mi][ni][0], sv.y - acc[mi][ni][1]);
-                            if (u == 0) {
-                                D[(r - r0) * kD + (c - cc0)] = o.x;
-                                D[(r - r0) * kD + (c - cc0) + 1] = o.y;
-                            } else {
-                                *reinterpret_cast<double2*>(S + (size_t)r * n + c) = o;
-                            }
-                        }
-                    if (u == 0) chain_bar(1, 64);  // D of panel p+1 is ready for warp 0
-                } else {
-                    const int R = (u - ntri) % q, C = (u - ntri) / q;
-                    chain_wtile(PsT + 32 * R, kLt, Xr + 32 * C, kXr, lane, acc);
-                    const bool fresh = C == p;
-                    const int r0 = c0 + 32 + 32 * R;
-#pragma unroll
-                    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                double* o = Y + (size_t)(32 * C + 8 * ni + 2 * t + i) * n + r0 + 8 * mi + g;
-                                *o = (fresh ? 0.0 : *o) - acc[mi][ni][i];
-                            }
-                }
-            }
-            chain_outputs<BSZ>(Y, invHi, invLo, Xr, c0, zero_upper != 0, tid - 32, kChainThreads - 32);
-        }
-        __syncthreads();
-    }
-}
-
 __global__ void set_int_kernel(int* p, int v) { *p = v; }
 
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
@@ -1261,8 +896,6 @@ hs_status tc_attrs() {
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, UpdSmem<BSZ>::kBytes));
     HS_CUDA(cudaFuncSetAttribute(tc_update_kernel<BSZ, HS_PRECISION_F16X3>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, UpdSmem<BSZ>::kBytes));
-    HS_CUDA(cudaFuncSetAttribute(diag_chain_kernel<BSZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ChainSmem<BSZ>::kBytes));
     if (dev < 64) g_tc_attr[dev][slot] = true;
     return HS_OK;
 }
@@ -1285,7 +918,7 @@ size_t mixed_workspace_bytes(int64_t N, int bsz) {
     bytes += (size_t)nb * bb * 8;        // Ldiag64
     bytes += (size_t)nb * bb * 8;        // Yinv
     bytes += (size_t)2 * kSets * nb * bb * 2;  // 16-bit split of two groups' panels (hi / lo each)
-    bytes += bb * 8;                     // S
+    bytes += 128 * 128 * 8;              // T
     bytes += 1024;                       // error flags
     bytes += ((size_t)tile_counters(nb) * 8 + 255) & ~size_t(255);  // tile counters of the updates
     bytes += ((size_t)nb * 4 + 255) & ~size_t(255);  // sweep publication flags
@@ -1307,8 +940,8 @@ hs_status mixed_bind(hs_ctx ctx, void* ws, MixedWork* w) {
     p += (size_t)nb * bb * 8;
     w->P16 = reinterpret_cast<__nv_bfloat16*>(p);
     p += (size_t)2 * kSets * nb * bb * 2;
-    w->S = reinterpret_cast<double*>(p);
-    p += bb * 8;
+    w->T = reinterpret_cast<double*>(p);
+    p += 128 * 128 * 8;
     w->err = reinterpret_cast<int*>(p);
     p += 1024;
     w->tile_ctr = reinterpret_cast<unsigned long long*>(p);
@@ -1352,27 +985,27 @@ hs_status mixed_factor(hs_ctx ctx, const double* K64, MixedWork& w, cudaStream_t
         shift_diag_kernel<<<64, 256, 0, s>>>(w.A32, bsz, nb, ctx->N, (float)shift);
         HS_CHECK_LAUNCH("shift_diag");
     }
-    // diagonal block k in FP64 (one CTA): L_kk, its FP32 copy in place, Y_k = L_kk^-T
-    // and the split L_kk^-1 for the panel TRSM
-    auto diag_chain = [&](int k, cudaStream_t st_) -> hs_status {
+    // diagonal block k in FP64: L_kk, Y_k = L_kk^-T and the split L_kk^-1 for the panel
+    // TRSM.  `ctas`: 8 where the GPU has eight neighbouring SMs to spare, 1 beside a
+    // trailing update that leaves only scattered ones
+    auto diag_chain = [&](int k, cudaStream_t st_, int ctas) -> hs_status {
         const int64_t id = T - (int64_t)(nb - k) * (nb - k + 1) / 2;
-        float* dblk = w.A32 + (size_t)id * bb;
-        const int64_t rem = ctx->N - (int64_t)k * bsz;
-        const int valid = rem < bsz ? (int)rem : bsz;
-        float* invHi = w.LO + (size_t)kSets * nb * bb;
+        DiagFactor f;
+        f.in32 = w.A32 + (size_t)id * bb;
+        f.L = w.Ld + (size_t)k * bb;
+        f.Y = w.Yinv + (size_t)k * bb;
+        f.T = w.T;
+        f.invHi = w.LO + (size_t)kSets * nb * bb;
+        f.invLo = f.invHi + bb;
+        f.zero_upper = k == 0;  // the planes are shared by all diagonal blocks
+        f.record_neg = 1;
+        f.row_base = (int64_t)k * bsz;
+        f.ctas = ctas;
         prof_begin(ctx, st_, HS_KERNEL_POTRF);
-        ctx->launches += 1;
-        if (bsz == 256)
-            diag_chain_kernel<256><<<1, kChainThreads, ChainSmem<256>::kBytes, st_>>>(
-                dblk, w.S, w.Yinv + (size_t)k * bb, w.Ld + (size_t)k * bb, invHi, invHi + bb, valid, k == 0,
-                ctx->d_info, (long long)k * bsz);
-        else
-            diag_chain_kernel<128><<<1, kChainThreads, ChainSmem<128>::kBytes, st_>>>(
-                dblk, w.S, w.Yinv + (size_t)k * bb, w.Ld + (size_t)k * bb, invHi, invHi + bb, valid, k == 0,
-                ctx->d_info, (long long)k * bsz);
-        HS_CHECK_LAUNCH("diag_chain");
+        hs_status r = launch_diag_factor(ctx, f, st_);
+        if (r != HS_OK) return r;
         const double nn = bsz;
-        prof_end(ctx, st_, HS_KERNEL_POTRF, 2.0 * nn * nn * nn / 3.0, nn * nn * (4.0 + 8.0 * 4.0 + 4.0 + 4.0));
+        prof_end(ctx, st_, HS_KERNEL_POTRF, 2.0 * nn * nn * nn / 3.0, nn * nn * (4.0 + 8.0 * 2.0 + 4.0 + 4.0));
         return HS_OK;
     };
     // Panels are factored in groups of up to kPanelGroup (k .. k+g-1) and the columns
@@ -1485,12 +1118,12 @@ hs_status mixed_factor(hs_ctx ctx, const double* K64, MixedWork& w, cudaStream_t
             if ((r = panel(k + i, kPanelGroup * bank + i, st_)) != HS_OK) return r;
             if (i + 1 < g) {
                 if ((r = update(k, i + 1, k + i + 1, 1, 1, kPanelGroup * bank, st_, cap, -1)) != HS_OK) return r;
-                if ((r = diag_chain(k + i + 1, st_)) != HS_OK) return r;
+                if ((r = diag_chain(k + i + 1, st_, st_ == s ? 8 : 1)) != HS_OK) return r;
             }
         }
         return HS_OK;
     };
-    if ((st = diag_chain(0, s)) != HS_OK) return st;
+    if ((st = diag_chain(0, s, 8)) != HS_OK) return st;
     bool ready = false;  // the group at k has been factored ahead
     for (int k = 0, bank = 0; k < nb - 1; bank ^= 1) {
         // precondition: column k has seen every panel before it and its diagonal
@@ -1506,7 +1139,7 @@ hs_status mixed_factor(hs_ctx ctx, const double* K64, MixedWork& w, cudaStream_t
             if ((st = update(k, g, c0, 3, g2, set0, s, ctx->num_sms, -1)) != HS_OK) return st;
             HS_CUDA(cudaEventRecord(ctx->ev_a, s));
             HS_CUDA(cudaStreamWaitEvent(sd, ctx->ev_a, 0));
-            if ((st = diag_chain(c0, sd)) != HS_OK) return st;
+            if ((st = diag_chain(c0, sd, 1)) != HS_OK) return st;
             if ((st = in_group(c0, g2, bank ^ 1, sd, side_sms)) != HS_OK) return st;
             const int ctr = next_ctr++;
             if ((st = update(k, g, c0 + g2, 0, 0, set0, s, ctx->num_sms - side_sms, ctr)) != HS_OK) return st;
@@ -1521,7 +1154,7 @@ hs_status mixed_factor(hs_ctx ctx, const double* K64, MixedWork& w, cudaStream_t
             if (side) {
                 HS_CUDA(cudaEventRecord(ctx->ev_a, s));
                 HS_CUDA(cudaStreamWaitEvent(sd, ctx->ev_a, 0));
-                if ((st = diag_chain(c0, sd)) != HS_OK) return st;
+                if ((st = diag_chain(c0, sd, 1)) != HS_OK) return st;
                 HS_CUDA(cudaEventRecord(ctx->ev_b, sd));
             }
             if (more && (st = update(k, g, c0, 2, 0, set0, s, side ? ctx->num_sms - kFree : ctx->num_sms, -1)) !=
@@ -1529,7 +1162,7 @@ hs_status mixed_factor(hs_ctx ctx, const double* K64, MixedWork& w, cudaStream_t
                 return st;
             if (side) {
                 HS_CUDA(cudaStreamWaitEvent(s, ctx->ev_b, 0));
-            } else if ((st = diag_chain(c0, s)) != HS_OK) {
+            } else if ((st = diag_chain(c0, s, 8)) != HS_OK) {
                 return st;
             }
             ready = false;
