@@ -217,10 +217,16 @@ inline DiagFactor diag_factor_in_place(hs_ctx ctx, double* blk) {
 // Y_k = L_kk^-T for all nb diagonal blocks of the packed factor L (Y: nb consecutive
 // blocks; T: 128 x 128 doubles of scratch a block, used for bsz 256)
 hs_status launch_diag_inverses(hs_ctx ctx, const double* L, double* Y, double* T, cudaStream_t s);
-// a whole forward (L^-1 in) or backward (L^-T in) sweep over the FP64 packed factor in
-// one cooperative launch, given Y_k = L_kk^-T (k_vector.cu)
-hs_status launch_sweep_whole_f64(hs_ctx ctx, const double* L, const double* Y, const double* in, double* out,
-                                 int forward, unsigned epoch, unsigned* flags, int* err, cudaStream_t s);
+// a whole forward (out = L^-1 in) or backward (out = L^-T in) sweep over a packed factor in
+// one launch, given Y_k = L_kk^-T (k_sweep.cu; out must not be in).  ws: workspace whose
+// flags sweep_reset has cleared; epoch: a value no sweep since has used; *err = 2 on a
+// wait that ran out
+size_t sweep_workspace_bytes(int nb, int bsz);
+hs_status sweep_reset(hs_ctx ctx, void* ws, cudaStream_t s);
+hs_status launch_sweep_f64(hs_ctx ctx, const double* L, const double* Y, const double* in, double* out, int forward,
+                           unsigned epoch, void* ws, int* err, cudaStream_t s);
+hs_status launch_sweep_f32(hs_ctx ctx, const float* L, const float* Y, const double* in, double* out, int forward,
+                           unsigned epoch, void* ws, int* err, cudaStream_t s);
 // Y = L^-T (row major) of one lower-triangular block (bsz 128 or 256; T: 128 x 128 of scratch)
 hs_status launch_diag_inverse(hs_ctx ctx, const double* Lkk, double* Y, double* T, cudaStream_t s);
 // B <- B Y in place for blockCount consecutive blocks from firstBlock (bsz 128 or 256):

@@ -138,13 +138,13 @@ int grid_n(int64_t n, int sms) {
 }  // namespace
 
 // b <- (L L^T)^-1 b with the mixed factor: FP32 off-diagonal blocks, FP64
-// inverse diagonal blocks; one cooperative launch a direction.  The forward sweep
+// inverse diagonal blocks; one launch a direction.  The forward sweep
 // reads b and writes L^-1 b into tmp; the backward sweep reads tmp and writes the
 // result into b.
 hs_status mixed_apply(hs_ctx ctx, MixedWork& w, double* b, double* tmp, cudaStream_t s) {
-    hs_status st = launch_mixed_sweep_whole(ctx, w.A32, w.Y32, b, tmp, 1, ++w.epoch, w.flags, w.err + 1, s);
+    hs_status st = launch_sweep_f32(ctx, w.A32, w.Y32, b, tmp, 1, ++w.epoch, w.sweep, w.err + 1, s);
     if (st != HS_OK) return st;
-    return launch_mixed_sweep_whole(ctx, w.A32, w.Y32, tmp, b, 0, ++w.epoch, w.flags, w.err + 1, s);
+    return launch_sweep_f32(ctx, w.A32, w.Y32, tmp, b, 0, ++w.epoch, w.sweep, w.err + 1, s);
 }
 
 namespace {
@@ -186,7 +186,7 @@ hs_status mixed_solve_impl(hs_ctx ctx, const double* K, const double* b, double*
     MixedWork w;
     st = mixed_bind(ctx, ctx->mixed, &w);
     if (st != HS_OK) return st;
-    HS_CUDA(cudaMemsetAsync(w.flags, 0, (size_t)nb * sizeof(unsigned), s));
+    if ((st = sweep_reset(ctx, w.sweep, s)) != HS_OK) return st;
     HS_CUDA(cudaMemsetAsync(w.err + 1, 0, sizeof(int), s));
     st = ensure_scratch(ctx, kSmallScratch + (size_t)nb * nb * bsz * sizeof(double));
     if (st != HS_OK) return st;

@@ -4,6 +4,7 @@
 
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cudaTypedefs.h>
 
 #include "hs_internal.cuh"
 
@@ -19,7 +20,7 @@ struct MixedWork {
     __nv_bfloat16* P16 = nullptr;  // 16-bit (BF16 or FP16) split of two panel groups: set p hi blocks 2p nb.., lo (2p+1) nb..
     int* err = nullptr;     // [0] tensor-core tile timeout, [1] triangular-sweep timeout
     unsigned long long* tile_ctr = nullptr;  // tile counters of the trailing-update launches (zeroed per factor)
-    unsigned* flags = nullptr;  // per block row: epoch of the sweep that published it
+    void* sweep = nullptr;      // the sweeps' workspace (sweep_workspace_bytes)
     unsigned epoch = 0;         // last sweep launched (flags are cleared when it restarts at 0)
     float* Y32 = nullptr;       // FP32 copy of Yinv for the sweeps, in the P16 area once the factor is done
     CUtensorMap mA128, mL128, mL32;      // 128-byte swizzle, 32-wide K boxes of 128 / 32 rows (TRSM)
@@ -50,13 +51,7 @@ hs_status mixed_apply(hs_ctx ctx, MixedWork& w, double* b, double* tmp, cudaStre
 hs_status mixed_solve_impl(hs_ctx ctx, const double* K, const double* b, double* x, int precision, double tol,
                            int max_steps, hs_mixed_report* out, int acc_panels = 0);
 
-// a whole forward / backward sweep in one cooperative launch: out = L^-1 in or
-// L^-T in (block rows published through flags[] with value `epoch`; *err = 2 on a
-// wait that timed out)
-hs_status launch_mixed_sweep_whole(hs_ctx ctx, const float* A32, const float* Y, const double* in, double* out,
-                                   int forward, unsigned epoch, unsigned* flags, int* err, cudaStream_t s);
-// column update reading FP32 blocks (accumulation in FP64)
-hs_status launch_column_update_f32(hs_ctx ctx, const float* A32, double* b, int blockStart, int blockCount,
-                                   int blockRow, int blockID, int transposed, cudaStream_t s);
+// the driver's cuTensorMapEncodeTiled
+hs_status tensor_map_encoder(PFN_cuTensorMapEncodeTiled_v12000* fn);
 
 }  // namespace hs

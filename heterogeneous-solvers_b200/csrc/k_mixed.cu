@@ -822,6 +822,16 @@ hs_status get_encoder() {
     return HS_OK;
 }
 
+}  // namespace
+
+hs_status tensor_map_encoder(PFN_cuTensorMapEncodeTiled_v12000* fn) {
+    hs_status st = get_encoder();
+    *fn = g_encode;
+    return st;
+}
+
+namespace {
+
 // 3-D FP32 map over `blocks` blocks of bsz x bsz, box = 32 columns x box_rows rows x 1 block
 hs_status make_map(CUtensorMap* m, void* base, int bsz, int64_t blocks, int box_rows, int box_k = kSlab,
                    int elem = 4) {
@@ -921,7 +931,7 @@ size_t mixed_workspace_bytes(int64_t N, int bsz) {
     bytes += 128 * 128 * 8;              // T
     bytes += 1024;                       // error flags
     bytes += ((size_t)tile_counters(nb) * 8 + 255) & ~size_t(255);  // tile counters of the updates
-    bytes += ((size_t)nb * 4 + 255) & ~size_t(255);  // sweep publication flags
+    bytes += sweep_workspace_bytes((int)nb, bsz);
     return bytes;
 }
 
@@ -946,7 +956,7 @@ hs_status mixed_bind(hs_ctx ctx, void* ws, MixedWork* w) {
     p += 1024;
     w->tile_ctr = reinterpret_cast<unsigned long long*>(p);
     p += ((size_t)tile_counters(nb) * 8 + 255) & ~size_t(255);
-    w->flags = reinterpret_cast<unsigned*>(p);
+    w->sweep = p;
     hs_status st = make_map(&w->mA128, w->A32, bsz, (int64_t)T, 128);
     if (st == HS_OK) st = make_map(&w->mL128, w->LO, bsz, kSets * nb + 2, 128);
     if (st == HS_OK) st = make_map(&w->mL32, w->LO, bsz, kSets * nb + 2, 32);

@@ -333,46 +333,10 @@ __global__ void __launch_bounds__(kThreads) column_update_kernel(const double* _
     for (int r = threadIdx.x; r < bsz; r += blockDim.x) bi[r] -= out[r];
 }
 
-// block-column update reading FP32 blocks (mixed-precision solves), FP64 sums
-template <int BSZ>
-__global__ void __launch_bounds__(kThreads) column_update_f32_kernel(const float* __restrict__ A,
-                                                                     double* __restrict__ b, int nb, int blockStart,
-                                                                     int blockRow, int64_t blockID, int transposed) {
-    __shared__ double smem[8 * BSZ];
-    __shared__ double out[BSZ];
-    const int g = blockIdx.x;
-    const size_t bb = (size_t)BSZ * BSZ;
-    const double* b0 = b + (size_t)blockRow * BSZ;
-    double* bi = b + (size_t)(blockStart + g) * BSZ;
-    if (!transposed) {
-        const float* M = A + (size_t)(blockID + (blockStart - blockRow + g)) * bb;
-        BlockApply<BSZ, float>::run(M, b0, nullptr, out, nullptr, 1, smem);
-    } else {
-        const float* M = A + (size_t)block_id(blockRow, blockStart + g, nb) * bb;
-        BlockApply<BSZ, float>::run(M, nullptr, b0, nullptr, out, 2, smem);
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < BSZ; r += blockDim.x) bi[r] -= out[r];
-}
-
-// Whole sweep in one launch.  CTA c owns block rows i = c, c + P, ... (P = grid)
-// and keeps their running right-hand sides in shared memory.  Forward (t = L^-1 b):
-// row i takes L_ij out_j off for j = 0 .. i-1 in that order, then its owner solves
-// out_i = Y_i^T t_i and publishes it; backward (L^-T) mirrors this with the
-// transposed blocks L_ji^T and descending columns.  Each row is reduced by one CTA
-// in column order, so the sums follow a fixed order.  Publication: the owner
-// stores out_i, fences, and sets flags[i] = epoch; readers wait for that value
-// (bounded: on timeout *err = 2 and the CTA stops) and read out_j past L1.
-// Needs all CTAs resident at once (cooperative launch).
-constexpr uint64_t kSweepWaitNs = 2000000000ull;
-
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ uint64_t sweep_clock_ns() {
     uint64_t t;
@@ -391,154 +355,6 @@ __global__ void bounded_wait_kernel(const unsigned* __restrict__ flag, unsigned 
             atomicExch(err, 1);
             return;
         }
-    }
-}
-
-// hint: bring `bytes` (a multiple of 16) at p (16-byte aligned) into L2
-__device__ __forceinline__ void sweep_prefetch_l2(const void* p, uint32_t bytes) {
-    const char* b = static_cast<const char*>(p);
-    for (uint32_t off = 0; off < bytes; off += 65536u) {
-        const uint32_t n = bytes - off < 65536u ? bytes - off : 65536u;
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b + off), "r"(n) : "memory");
-    }
-}
-// The bulk of a sweep's block products streams past L2 (evict-first loads) while
-// most CTAs work at once, so a row's last two block products — the one with the
-// block next to the diagonal, once the previous row is published, then the one
-// with its inverse diagonal block — run on the chain at a CTA's share of a busy
-// HBM.  Their blocks are hinted into L2 when the owner applies the column
-// kSweepAhead before the diagonal, so the chain reads them from L2.
-constexpr int kSweepAhead = 4;
-
-template <int BSZ, typename T>
-__global__ void __launch_bounds__(kThreads) mixed_sweep_whole_kernel(const T* __restrict__ A,
-                                                                     const T* __restrict__ Y,
-                                                                     const double* __restrict__ in,
-                                                                     double* __restrict__ out, int nb, int forward,
-                                                                     unsigned epoch, unsigned* __restrict__ flags,
-                                                                     int* __restrict__ err) {
-    extern __shared__ double ssm[];
-    const int P = gridDim.x, c = blockIdx.x, tid = threadIdx.x;
-    const int nown = (nb - c + P - 1) / P;  // rows c + P q, q < nown
-    double* smem = ssm;                     // 8 BSZ: BlockApply
-    double* xs = smem + 8 * BSZ;            // the published block of out
-    double* tmp = xs + BSZ;                 // one block product
-    double* wk = tmp + BSZ;                 // nown rows of running right-hand side
-    __shared__ int s_stop;
-    const size_t bb = (size_t)BSZ * BSZ;
-    for (int q = 0; q < nown; ++q)
-        for (int r = tid; r < BSZ; r += blockDim.x) wk[q * BSZ + r] = in[(size_t)(c + P * q) * BSZ + r];
-    if (tid == 0) s_stop = 0;
-    __syncthreads();
-
-    // the owner's diagonal solve of row i (running right-hand side in wk row q)
-    auto solve = [&](int i, int q) {
-        const T* Yi = Y + (size_t)i * bb;
-        if (forward)
-            BlockApply<BSZ, T>::run(Yi, nullptr, wk + q * BSZ, nullptr, out + (size_t)i * BSZ, 2, smem);
-        else
-            BlockApply<BSZ, T>::run(Yi, wk + q * BSZ, nullptr, out + (size_t)i * BSZ, nullptr, 1, smem);
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            st_release_u32(flags + i, epoch);
-        }
-    };
-    // wk row q -= (block (r, cc) or its transpose) xs
-    auto update = [&](int r, int cc, int q) {
-        const T* M = A + (size_t)block_id(r, cc, nb) * bb;
-        if (forward)
-            BlockApply<BSZ, T>::run(M, xs, nullptr, tmp, nullptr, 1, smem);
-        else
-            BlockApply<BSZ, T>::run(M, nullptr, xs, nullptr, tmp, 2, smem);
-        __syncthreads();
-        for (int e = tid; e < BSZ; e += blockDim.x) wk[q * BSZ + e] -= tmp[e];
-        __syncthreads();
-    };
-
-    // Greedy order: act on the CTA's smallest open row (forward; largest backward)
-    // that can progress: apply its next column once published, or solve it once
-    // every column is in.  Columns are published in order, so `known` (the last
-    // column seen published) settles most checks without a load.
-    int* nextc = reinterpret_cast<int*>(wk + nown * BSZ);  // per owned row: next column to apply
-    __shared__ int s_pick, s_col, s_known, s_xs;
-    if (tid == 0) {
-        for (int q = 0; q < nown; ++q) nextc[q] = forward ? 0 : nb - 1;
-        s_known = 0;  // columns seen published (forward: 0 .. known-1; backward: nb-known .. nb-1)
-        s_xs = -1;
-    }
-    __syncthreads();
-    int solved = 0;
-    while (solved < nown) {
-        if (tid == 0) {
-            int pick = -1, col = -1;
-            for (;;) {
-                bool open = false;
-                for (int qq = 0; qq < nown; ++qq) {
-                    const int q = forward ? qq : nown - 1 - qq;
-                    const int i = c + P * q;
-                    const int jn = nextc[q];
-                    if (jn < 0) continue;  // solved
-                    open = true;
-                    if (jn == i) {  // every column applied
-                        pick = q;
-                        col = -2;
-                        break;
-                    }
-                    if (forward ? (jn < s_known) : (jn > nb - 1 - s_known)) {
-                        pick = q;
-                        col = jn;
-                        break;
-                    }
-                }
-                if (pick >= 0 || !open) break;
-                // nothing to do: wait (bounded) for the next column in publication order
-                const int jw = forward ? s_known : nb - 1 - s_known;
-                const uint64_t deadline = sweep_clock_ns() + kSweepWaitNs;
-                while (ld_acquire_u32(flags + jw) != epoch) {
-                    if (sweep_clock_ns() > deadline || *reinterpret_cast<volatile int*>(err) != 0) {
-                        atomicExch(err, 2);
-                        s_stop = 1;
-                        break;
-                    }
-                }
-                if (s_stop) break;
-                ++s_known;
-            }
-            s_pick = pick;
-            s_col = col;
-            if (pick >= 0 && col >= 0) {
-                // row i's chain blocks: link block (i, i-1) forward, (i+1, i) backward
-                // (both exist: a row takes column picks only when it has a link), and Y_i
-                const int i = c + P * pick;
-                const int first = forward ? (i > kSweepAhead ? i - kSweepAhead : 0)
-                                          : (i + kSweepAhead < nb - 1 ? i + kSweepAhead : nb - 1);
-                if (col == first) {
-                    const int lr = forward ? i : i + 1, lc = lr - 1;
-                    sweep_prefetch_l2(A + (size_t)block_id(lr, lc, nb) * bb, (uint32_t)(bb * sizeof(T)));
-                    sweep_prefetch_l2(Y + (size_t)i * bb, (uint32_t)(bb * sizeof(T)));
-                }
-            }
-        }
-        __syncthreads();
-        if (s_stop || s_pick < 0) break;
-        const int q = s_pick, i = c + P * q, j = s_col;
-        if (j == -2) {
-            solve(i, q);
-            if (tid == 0) nextc[q] = -1;
-            ++solved;
-            __syncthreads();
-            continue;
-        }
-        if (s_xs != j) {
-            for (int e = tid; e < BSZ; e += blockDim.x) xs[e] = __ldcg(out + (size_t)j * BSZ + e);
-            __syncthreads();
-            if (tid == 0) s_xs = j;
-        }
-        if (forward) update(i, j, q);
-        else update(j, i, q);
-        if (tid == 0) nextc[q] = forward ? j + 1 : j - 1;
-        __syncthreads();
     }
 }
 
@@ -767,69 +583,6 @@ hs_status launch_bounded_wait_selftest(hs_ctx ctx, int64_t timeout_ns) {
                   "(expected: nothing sets its flag)");
         return HS_ERR_TIMEOUT;
     }
-    return HS_OK;
-}
-
-namespace {
-
-template <typename T>
-hs_status launch_sweep_whole(hs_ctx ctx, const T* A, const T* Y, const double* in, double* out, int forward,
-                             unsigned epoch, unsigned* flags, int* err, cudaStream_t s) {
-    const int bsz = ctx->bsz, nb = ctx->nb;
-    HS_REQUIRE(bsz == 128 || bsz == 256, "the whole-sweep solve supports matrixBlockSize 128 or 256");
-    int per_sm = 0;
-    const void* fn = bsz == 256 ? (const void*)mixed_sweep_whole_kernel<256, T>
-                                : (const void*)mixed_sweep_whole_kernel<128, T>;
-    // rows per CTA for the grid used (at least one row each); shared memory for them
-    auto smem_for = [&](int grid) {
-        const int nown = (nb + grid - 1) / grid;
-        return (size_t)(10 + nown) * bsz * sizeof(double) + (size_t)nown * sizeof(int);
-    };
-    int grid = nb < 2 * ctx->num_sms ? nb : 2 * ctx->num_sms;
-    HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, smem_for(grid)));
-    if (grid > per_sm * ctx->num_sms) grid = per_sm * ctx->num_sms;
-    HS_REQUIRE(grid >= 1, "the whole-sweep solve does not fit on the device");
-    const size_t smem = smem_for(grid);
-    HS_REQUIRE(smem <= 200 * 1024, "matrix too large for the single-launch sweep");
-    if (smem > 48 * 1024) HS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    void* args[] = {(void*)&A, (void*)&Y, (void*)&in, (void*)&out, (void*)&nb, (void*)&forward,
-                    (void*)&epoch, (void*)&flags, (void*)&err};
-    prof_begin(ctx, s, HS_KERNEL_COLUPD);
-    ctx->launches += 1;
-    HS_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, s));
-    const double Tb = (double)nb * (nb - 1) / 2.0;
-    prof_end(ctx, s, HS_KERNEL_COLUPD, 2.0 * (Tb + nb) * bsz * bsz, (Tb + nb) * sizeof(T) * bsz * bsz);
-    return HS_OK;
-}
-
-}  // namespace
-
-hs_status launch_mixed_sweep_whole(hs_ctx ctx, const float* A32, const float* Y, const double* in, double* out,
-                                   int forward, unsigned epoch, unsigned* flags, int* err, cudaStream_t s) {
-    return launch_sweep_whole<float>(ctx, A32, Y, in, out, forward, epoch, flags, err, s);
-}
-
-hs_status launch_sweep_whole_f64(hs_ctx ctx, const double* L, const double* Y, const double* in, double* out,
-                                 int forward, unsigned epoch, unsigned* flags, int* err, cudaStream_t s) {
-    return launch_sweep_whole<double>(ctx, L, Y, in, out, forward, epoch, flags, err, s);
-}
-
-hs_status launch_column_update_f32(hs_ctx ctx, const float* A32, double* b, int blockStart, int blockCount,
-                                   int blockRow, int blockID, int transposed, cudaStream_t s) {
-    if (blockCount <= 0) return HS_OK;
-    const int bsz = ctx->bsz;
-    HS_REQUIRE(bsz == 128 || bsz == 256, "FP32 column update supports matrixBlockSize 128 or 256");
-    prof_begin(ctx, s, HS_KERNEL_COLUPD);
-    ctx->launches += 1;
-    if (bsz == 256)
-        column_update_f32_kernel<256><<<blockCount, kThreads, 0, s>>>(A32, b, ctx->nb, blockStart, blockRow, blockID,
-                                                                     transposed);
-    else
-        column_update_f32_kernel<128><<<blockCount, kThreads, 0, s>>>(A32, b, ctx->nb, blockStart, blockRow, blockID,
-                                                                     transposed);
-    HS_CHECK_LAUNCH("column_update_f32");
-    prof_end(ctx, s, HS_KERNEL_COLUPD, 2.0 * blockCount * (double)bsz * bsz,
-             (double)blockCount * bsz * bsz * 4.0 + 24.0 * blockCount * bsz);
     return HS_OK;
 }
 
