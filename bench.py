@@ -695,7 +695,9 @@ def main():
                    "iterations": it.value, "ms": cg_ms, "ms_per_iteration": cg_ms / max(1, it.value),
                    "rel_residual": (dn.value / d0.value) ** 0.5 if d0.value else None,
                    "true_rel_residual": (torch.linalg.norm(r_cg - bd) / torch.linalg.norm(bd)).item(),
-                   "matvecs": symv["launches"], "matvec_ms": symv["ms"] / max(1, symv["launches"]),
+                   # the iterations run on the device: ms of a whole iteration, by matvec
+                   "matvecs": round(symv["bytes"] / (nb * (nb + 1) // 2 * bsz * bsz * 8.0 + 24.0 * nb * bsz)),
+                   "matvec_ms": symv["ms"] / max(1, it.value),
                    "matvec_gbs": symv["bytes"] / (symv["ms"] * 1e-3) / 1e9 if symv["ms"] else None,
                    "matvec_frac_of_hbm": None}
         if fp64 is not None:

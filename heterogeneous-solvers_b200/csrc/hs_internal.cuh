@@ -237,6 +237,9 @@ hs_status launch_trsm_dmma(hs_ctx ctx, double* A, int64_t firstBlock, int blockC
 hs_status launch_symv(hs_ctx ctx, const double* A, const double* b, double* result, int bi0, int bj0, int nbi,
                       int nbj, int reset, double* dot_with /*nullable: also dot(result, dot_with) */,
                       double* dot_out, cudaStream_t s);
+// CG with the iterations on the device (k_cg.cu; block sizes 128 and 256)
+hs_status cg_persistent(hs_ctx ctx, const double* A, const double* b, double* x, double eps, int64_t imax,
+                        int64_t* iters_out, double* dnew_out, double* d0_out);
 hs_status launch_trsv(hs_ctx ctx, const double* A, double* b, int blockRow, int blockID, int transposed,
                       cudaStream_t s);
 hs_status launch_column_update(hs_ctx ctx, const double* A, double* b, int blockStart, int blockCount,

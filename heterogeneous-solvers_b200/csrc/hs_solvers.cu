@@ -208,6 +208,8 @@ hs_status cg_driver(hs_ctx ctx, const double* A, const double* b, double* x, dou
     const int64_t n = (int64_t)nb * ctx->bsz;
     cudaStream_t s = ctx->stream;
     const bool ref = ctx->ref_chunks > 0;
+    if (!ref && (ctx->bsz == 128 || ctx->bsz == 256))
+        return cg_persistent(ctx, A, b, x, eps, imax, iters_out, dnew_out, d0_out);
     hs_status st = ensure_work(ctx, (size_t)3 * n * sizeof(double));
     if (st != HS_OK) return st;
     // size the scratch for the matvec partials now: pointers into it stay valid below
