@@ -107,10 +107,12 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
         return HS_OK;
     }
     // Tensor-core form with lookahead.  The panel TRSM is a product with
-    // Y = L_kk^-T.  Per column k the trailing update runs in two launches: column
-    // k+1 first; then, while the rest of the update runs, POTRF(k+1), Y and the
-    // TRSM of column k+1 run on the high-priority side stream.  Every block sees
-    // the same operations in the same order as without lookahead.
+    // Y = L_kk^-T.  The chain of columns (bring column k up to date with panel k-1, factor
+    // its diagonal block, TRSM) runs on the high-priority side stream, one launch after the
+    // other; the rest of panel k's update, columns k+2 on, runs beside it on the caller's
+    // stream.  Every block sees the same operations in the same order as without
+    // lookahead.  (With the column update on the caller's stream, the chain crossed streams
+    // twice a column.)
     const size_t bb = (size_t)bsz * bsz;
     hs_status st = ensure_scratch(ctx, kSmallScratch + kDiagScratchBlocks * bb * sizeof(double));
     if (st != HS_OK) return st;
@@ -127,21 +129,39 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
         const int cnt = nb - (k + 1);
         return launch_trsm_dmma(ctx, A, (int64_t)blockID + 1, cnt, f.Y, f.L, q);
     };
-    if ((st = diag(0, s)) != HS_OK) return st;
+    cudaStream_t c = ctx->side_hi;
+    HS_CUDA(cudaEventRecord(ctx->ev_a, s));
+    HS_CUDA(cudaStreamWaitEvent(c, ctx->ev_a, 0));
+    if ((st = diag(0, c)) != HS_OK) return st;
     for (int k = 0; k + 1 < nb; ++k) {
         const int blockID = diag_id(k);
-        if ((st = launch_update_cols(ctx, A, blockID, k, k + 1, k + 2, s)) != HS_OK) return st;
-        if (k + 2 < nb) {
-            HS_CUDA(cudaEventRecord(ctx->ev_a, s));
-            HS_CUDA(cudaStreamWaitEvent(ctx->side_hi, ctx->ev_a, 0));
-            if ((st = diag(k + 1, ctx->side_hi)) != HS_OK) return st;
-            HS_CUDA(cudaEventRecord(ctx->ev_b, ctx->side_hi));
-            if ((st = launch_update_cols(ctx, A, blockID, k, k + 2, nb, s)) != HS_OK) return st;
-            HS_CUDA(cudaStreamWaitEvent(s, ctx->ev_b, 0));
-        } else if ((st = diag(k + 1, s)) != HS_OK) {
-            return st;
+        const int64_t m = nb - k - 2;  // block columns of the rest of panel k's update
+        // A diagonal block's CTAs need whole SMs, and beside an update that fills the chip
+        // they wait for one to drain.  Where the chain is what the factor waits for, the
+        // update is therefore released only after column k+1's, just behind the diagonal
+        // block's launch; where the update takes several times the chain it starts at once
+        // (six waves of two 128 x 64 tiles an SM: about twice a column's chain).
+        const bool behind = m * (m + 1) / 2 * (bsz / 128) * (bsz / 64) <= 12LL * ctx->num_sms;
+        if (m > 0 && !behind) {
+            HS_CUDA(cudaEventRecord(ctx->ev_a, c));  // panel k
+            HS_CUDA(cudaStreamWaitEvent(s, ctx->ev_a, 0));
         }
+        // column k+1 has panels 0..k-1 once the rest of panel k-1's update is done
+        if (k > 0) HS_CUDA(cudaStreamWaitEvent(c, ctx->ev_b, 0));
+        if ((st = launch_update_cols(ctx, A, blockID, k, k + 1, k + 2, c)) != HS_OK) return st;
+        if (m > 0 && behind) {
+            HS_CUDA(cudaEventRecord(ctx->ev_a, c));
+            if ((st = diag(k + 1, c)) != HS_OK) return st;
+            HS_CUDA(cudaStreamWaitEvent(s, ctx->ev_a, 0));
+        }
+        if (m > 0) {
+            if ((st = launch_update_cols(ctx, A, blockID, k, k + 2, nb, s)) != HS_OK) return st;
+            HS_CUDA(cudaEventRecord(ctx->ev_b, s));
+        }
+        if (!(m > 0 && behind) && (st = diag(k + 1, c)) != HS_OK) return st;
     }
+    HS_CUDA(cudaEventRecord(ctx->ev_a, c));
+    HS_CUDA(cudaStreamWaitEvent(s, ctx->ev_a, 0));
     return HS_OK;
 }
 

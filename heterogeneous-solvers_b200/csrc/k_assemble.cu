@@ -82,32 +82,35 @@ __global__ void __launch_bounds__(256) rbf_assemble_kernel(double* __restrict__ 
 // Thread t takes columns 4 (t % G) .. +3 (G = bsz / 4 column groups) and rows
 // 4 (t / G) + R p .. +3 in pass p (R = 4 * 256 / G rows a pass); a warp shares its
 // rows (broadcast reads) and writes 32 x 32 contiguous bytes per row.  Per entry the
-// distance is summed over k ascending exactly as in rbf_assemble_kernel.
+// distance is summed over k ascending exactly as in rbf_assemble_kernel.  blockIdx.y:
+// which `rows` rows of the block (all of them when the blocks alone fill the chip; fewer
+// a CTA below that: N=500, bsz 128, 19 -> 8 us).
 __global__ void __launch_bounds__(256) rbf_assemble_tile_kernel(double* __restrict__ A,
                                                                 const double* __restrict__ X, int64_t N, int d,
                                                                 int bsz, int nb, int ard,
                                                                 const double* __restrict__ wsc, double sf2,
-                                                                double sn2, double iso_scale) {
+                                                                double sn2, double iso_scale, int rows) {
     extern __shared__ double sm[];
-    double* Xi = sm;                      // bsz x d
-    double* XjT = sm + (size_t)bsz * d;   // d x bsz
+    double* Xi = sm;                      // rows x d
+    double* XjT = sm + (size_t)rows * d;  // d x bsz
     __shared__ double w[kMaxD];
     int ib, jb;
     block_coords(blockIdx.x, nb, &ib, &jb);
-    const int64_t i0 = (int64_t)ib * bsz, j0 = (int64_t)jb * bsz;
+    const int r0 = blockIdx.y * rows;
+    const int64_t i0 = (int64_t)ib * bsz + r0, j0 = (int64_t)jb * bsz;
+    for (int e = threadIdx.x; e < rows * d; e += blockDim.x) Xi[e] = (i0 + e / d < N) ? X[i0 * d + e] : 0.0;
     for (int e = threadIdx.x; e < bsz * d; e += blockDim.x) {
         const int r = e / d, k = e % d;
-        Xi[e] = (i0 + r < N) ? X[(i0 + r) * d + k] : 0.0;
         XjT[(size_t)k * bsz + r] = (j0 + r < N) ? X[(j0 + r) * d + k] : 0.0;
     }
     if (threadIdx.x < d) w[threadIdx.x] = ard ? wsc[threadIdx.x] : 1.0;
     __syncthreads();
-    double* blk = A + (size_t)blockIdx.x * bsz * bsz;
+    double* blk = A + (size_t)blockIdx.x * bsz * bsz + (size_t)r0 * bsz;
     const int G = bsz >> 2;
     const int cg = threadIdx.x % G, rg = threadIdx.x / G;
     const int rows_pass = 4 * (256 / G);
     const int jl = 4 * cg;
-    for (int il0 = 4 * rg; il0 < bsz; il0 += rows_pass) {
+    for (int il0 = 4 * rg; il0 < rows; il0 += rows_pass) {
         double acc[4][4];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
@@ -207,8 +210,13 @@ hs_status launch_rbf_assemble(hs_ctx ctx, double* A, const double* X, int d, con
         if (smem > 48 * 1024)
             HS_CUDA(cudaFuncSetAttribute(rbf_assemble_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem));
-        rbf_assemble_tile_kernel<<<(unsigned)T, 256, smem, s>>>(A, X, ctx->N, d, bsz, nb, ard, wdev, sf2, sn2,
-                                                                iso_scale);
+        // rows a CTA: halved, down to one pass over them, while the CTAs are under two an SM
+        const int pass = 4 * (256 / (bsz / 4));
+        int rows = bsz;
+        while (rows % 2 == 0 && rows / 2 >= pass && rows / 2 % pass == 0 && T * (bsz / rows) < 2LL * ctx->num_sms)
+            rows /= 2;
+        rbf_assemble_tile_kernel<<<dim3((unsigned)T, (unsigned)(bsz / rows)), 256, (size_t)(bsz + rows) * d * sizeof(double),
+                                   s>>>(A, X, ctx->N, d, bsz, nb, ard, wdev, sf2, sn2, iso_scale, rows);
     } else if (bsz % 2 == 0 && smem <= 200 * 1024) {
         if (smem > 48 * 1024)
             HS_CUDA(cudaFuncSetAttribute(rbf_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

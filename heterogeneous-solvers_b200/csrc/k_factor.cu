@@ -214,7 +214,11 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
     double* Bs = smem + ST * TM * SPAD;  // [ST][TN][SPAD]
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const int wm = warp / D::kWarpsN, wn = warp % D::kWarpsN;
+    // PRODUCT: later columns have longer sums; warps w and w + 4 share a scheduler, so the
+    // second four take the columns in reverse
+    const int wm = warp / D::kWarpsN;
+    const int wn = PRODUCT && warp >= 4 ? D::kWarpsN - 1 - warp % 4 % D::kWarpsN : warp % D::kWarpsN;
+    static_assert(!PRODUCT || (D::kThreads == 256 && (D::kWarpsN == 4 || D::kWarpsN == 8)), "the mapping above");
     const int g = lane >> 2, t = lane & 3;
 
     double acc[D::kMi][D::kNi][2];
@@ -307,6 +311,10 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
 // Each CTA's C preload and store overlap the other CTA's tensor work.
 constexpr int kUTM = 128, kUTN = 64, kUWM = 32, kUWN = 32, kUST = 3;
 using UTile = DTile<kUTM, kUTN, kUWM, kUWN, kUST>;
+// An update too small to give every SM a tile is on the factor's critical path and takes
+// one tile's time: 32 x 32 tiles of four warps then (a column of 20 blocks of 128: 15 -> 5
+// us).  Above that the larger tiles' reuse wins.
+using USmall = DTile<32, 32, 16, 16, 3>;
 
 // Work list of a trailing update.  Column mode (the factor driver): the pairs
 // (r, c) of the columns c in [colStart, colEnd), c <= r < nb, column by column.
@@ -350,7 +358,8 @@ __device__ __forceinline__ void decode_pair(const UpdateArgs& a, int64_t pair, i
     *r = lo + (int)(pair - offset(lo));
 }
 
-__global__ void __launch_bounds__(UTile::kThreads, 2) update_dmma_kernel(UpdateArgs a) {
+template <int TM, int TN, int WM, int WN, int ST, int CTAS>
+__global__ void __launch_bounds__(DTile<TM, TN, WM, WN, ST>::kThreads, CTAS) update_dmma_kernel(UpdateArgs a) {
     extern __shared__ __align__(16) double smem[];
     const int tpb = a.tilesM * a.tilesN;
     const int64_t pair = blockIdx.x / tpb;
@@ -358,25 +367,26 @@ __global__ void __launch_bounds__(UTile::kThreads, 2) update_dmma_kernel(UpdateA
     int r, c;
     decode_pair(a, pair, &r, &c);
     const int ti = tile / a.tilesN, tj = tile % a.tilesN;
-    const int shift = tj * kUTN - ti * kUTM;  // tile column offset minus row offset inside the block
+    const int shift = tj * TN - ti * TM;  // tile column offset minus row offset inside the block
     const bool diag = r == c;
-    if (diag && shift > kUTM - 1) return;      // entirely above the diagonal
-    const bool lower = diag && shift + kUTN - 1 > 0;
+    if (diag && shift > TM - 1) return;      // entirely above the diagonal
+    const bool lower = diag && shift + TN - 1 > 0;
     const size_t bb = (size_t)a.bsz * a.bsz;
-    double* C = a.A + (size_t)block_id(r, c, a.nb) * bb + (size_t)ti * kUTM * a.bsz + (size_t)tj * kUTN;
-    const double* Ag = a.A + (size_t)(a.blockID + (r - a.blockRow)) * bb + (size_t)ti * kUTM * a.bsz;
-    const double* Bg = a.A + (size_t)(a.blockID + (c - a.blockRow)) * bb + (size_t)tj * kUTN * a.bsz;
-    dmma_tile_t<kUTM, kUTN, kUWM, kUWN, kUST, false>(C, a.bsz, Ag, a.bsz, Bg, a.bsz, a.bsz, lower, shift, smem);
+    double* C = a.A + (size_t)block_id(r, c, a.nb) * bb + (size_t)ti * TM * a.bsz + (size_t)tj * TN;
+    const double* Ag = a.A + (size_t)(a.blockID + (r - a.blockRow)) * bb + (size_t)ti * TM * a.bsz;
+    const double* Bg = a.A + (size_t)(a.blockID + (c - a.blockRow)) * bb + (size_t)tj * TN * a.bsz;
+    dmma_tile_t<TM, TN, WM, WN, ST, false>(C, a.bsz, Ag, a.bsz, Bg, a.bsz, a.bsz, lower, shift, smem);
 }
+constexpr auto update_large = update_dmma_kernel<kUTM, kUTN, kUWM, kUWN, kUST, 2>;
+constexpr auto update_small = update_dmma_kernel<32, 32, 16, 16, 3, 4>;
 
 // Panel TRSM as a tensor-core product: B <- B Y with Y = L_kk^-T (row major, upper
-// triangular), in place; one CTA per 64 rows of a panel block.
-template <int BSZ>
-struct TrsmTile {
-    using T = DTile<64, BSZ, 32, BSZ / 4, 3>;
-};
+// triangular), in place; one CTA per ROWS rows of a panel block: 64, or 32 where 64 leave
+// SMs without work.
+template <int BSZ, int ROWS>
+using TrsmTile = DTile<ROWS, BSZ, 32, ROWS * BSZ / 256, 3>;
 
-template <int BSZ>
+template <int BSZ, int ROWS>
 __global__ void __launch_bounds__(256, 1) trsm_dmma_kernel(double* A, int64_t firstBlock, const double* __restrict__ Y,
                                                            double* Lkk) {
     extern __shared__ __align__(16) double smem[];
@@ -390,11 +400,11 @@ __global__ void __launch_bounds__(256, 1) trsm_dmma_kernel(double* A, int64_t fi
                     make_double2(0.0, 0.0);
         }
     }
-    constexpr int kSlabs = BSZ / 64;
+    constexpr int kSlabs = BSZ / ROWS;
     const int64_t item = blockIdx.x / kSlabs;
     const int slab = blockIdx.x % kSlabs;
-    double* B = A + (size_t)(firstBlock + item) * BSZ * BSZ + (size_t)slab * 64 * BSZ;
-    dmma_tile_t<64, BSZ, 32, BSZ / 4, 3, true>(B, BSZ, B, BSZ, Y, BSZ, BSZ, false, 0, smem);
+    double* B = A + (size_t)(firstBlock + item) * BSZ * BSZ + (size_t)slab * ROWS * BSZ;
+    dmma_tile_t<ROWS, BSZ, 32, ROWS * BSZ / 256, 3, true>(B, BSZ, B, BSZ, Y, BSZ, BSZ, false, 0, smem);
 }
 
 // scalar fallback (any bsz): one thread per output element; SYRK follows
@@ -429,11 +439,16 @@ hs_status set_attrs() {
     int dev = 0;
     HS_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && attrs_done[dev]) return HS_OK;
-    HS_CUDA(cudaFuncSetAttribute(update_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, UTile::kSmem));
-    HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 TrsmTile<128>::T::kSmem));
-    HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 TrsmTile<256>::T::kSmem));
+    HS_CUDA(cudaFuncSetAttribute(update_large, cudaFuncAttributeMaxDynamicSharedMemorySize, UTile::kSmem));
+    HS_CUDA(cudaFuncSetAttribute(update_small, cudaFuncAttributeMaxDynamicSharedMemorySize, USmall::kSmem));
+    HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<128, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 TrsmTile<128, 64>::kSmem));
+    HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<256, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 TrsmTile<256, 64>::kSmem));
+    HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<128, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 TrsmTile<128, 32>::kSmem));
+    HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 TrsmTile<256, 32>::kSmem));
     HS_CUDA(cudaFuncSetAttribute(trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(256)));
     HS_CUDA(cudaFuncSetAttribute(potrf_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(128 * 129 * sizeof(double))));
@@ -501,11 +516,18 @@ hs_status launch_trsm_dmma(hs_ctx ctx, double* A, int64_t firstBlock, int blockC
     const double n = bsz;
     prof_begin(ctx, s, HS_KERNEL_TRSM);
     ctx->launches += 1;
-    const unsigned grid = (unsigned)((int64_t)blockCount * (bsz / 64));
-    if (bsz == 256)
-        trsm_dmma_kernel<256><<<grid, 256, TrsmTile<256>::T::kSmem, s>>>(A, firstBlock, Y, Lkk);
-    else
-        trsm_dmma_kernel<128><<<grid, 256, TrsmTile<128>::T::kSmem, s>>>(A, firstBlock, Y, Lkk);
+    const int64_t wide = (int64_t)blockCount * (bsz / 64);
+    if (wide <= ctx->num_sms) {
+        const unsigned grid = (unsigned)(2 * wide);
+        if (bsz == 256)
+            trsm_dmma_kernel<256, 32><<<grid, 256, TrsmTile<256, 32>::kSmem, s>>>(A, firstBlock, Y, Lkk);
+        else
+            trsm_dmma_kernel<128, 32><<<grid, 256, TrsmTile<128, 32>::kSmem, s>>>(A, firstBlock, Y, Lkk);
+    } else if (bsz == 256) {
+        trsm_dmma_kernel<256, 64><<<(unsigned)wide, 256, TrsmTile<256, 64>::kSmem, s>>>(A, firstBlock, Y, Lkk);
+    } else {
+        trsm_dmma_kernel<128, 64><<<(unsigned)wide, 256, TrsmTile<128, 64>::kSmem, s>>>(A, firstBlock, Y, Lkk);
+    }
     HS_CHECK_LAUNCH("trsm_dmma");
     // algorithmic work: the triangular solve's n^3 flops a block
     prof_end(ctx, s, HS_KERNEL_TRSM, blockCount * n * n * n, (2.0 * blockCount + 1.0) * n * n * 8.0);
@@ -546,12 +568,17 @@ hs_status run_update(hs_ctx ctx, UpdateArgs& a, double flops, double bytes, cuda
     const bool dmma = ctx->bsz % kUTM == 0;
     a.tilesM = dmma ? ctx->bsz / kUTM : 1;
     a.tilesN = dmma ? ctx->bsz / kUTN : 1;
+    const bool small = dmma && a.totalPairs * a.tilesM * a.tilesN <= ctx->num_sms;
+    if (small) a.tilesM = a.tilesN = ctx->bsz / 32;
     const int64_t grid = a.totalPairs * a.tilesM * a.tilesN;
     HS_REQUIRE(grid < (1LL << 31), "trailing update too large for one launch");
     prof_begin(ctx, s, HS_KERNEL_UPDATE);
     ctx->launches += 1;
     if (dmma) {
-        update_dmma_kernel<<<(unsigned)grid, UTile::kThreads, UTile::kSmem, s>>>(a);
+        if (small)
+            update_small<<<(unsigned)grid, USmall::kThreads, USmall::kSmem, s>>>(a);
+        else
+            update_large<<<(unsigned)grid, UTile::kThreads, UTile::kSmem, s>>>(a);
         HS_CHECK_LAUNCH("update_dmma");
     } else {
         const int64_t bb = (int64_t)ctx->bsz * ctx->bsz;

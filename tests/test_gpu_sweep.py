@@ -1,6 +1,7 @@
 """GPU suite: the single-launch triangular sweeps at the edges of their division of labour:
 the chain alone (1 to 3 block rows), one slice a CTA, several slices a CTA, padding in the
-last block; FP64 factors and the mixed form's FP32 factor."""
+last block; FP64 factors and the mixed form's FP32 factor.  (The sizes also cross the
+factor's switches between small and large update tiles and panel slabs.)"""
 import numpy as np
 import pytest
 import torch
@@ -21,7 +22,7 @@ def _problem(hs, ctx, N, bsz):
     return A, K, y
 
 
-SIZES = [(128, n) for n in (129, 256, 300, 640, 1000, 4777)] + [(256, n) for n in (257, 512, 700, 1300, 5000, 9001)]
+SIZES = [(128, n) for n in (129, 256, 300, 640, 1000, 4777, 10001)] + [(256, n) for n in (257, 512, 700, 1300, 5000, 9001)]
 
 
 @pytest.mark.parametrize("bsz,N", SIZES)
