@@ -7,8 +7,8 @@
 // src/utility/MatrixGenerator.cpp:134-155 with ARD lengthscales) is
 //   NLML = 1/2 y^T K^-1 y + sum_i log L_ii + N/2 log 2pi,   K = L L^T,
 // and its gradient 1/2 tr((K^-1 - alpha alpha^T) dK/dtheta), alpha = K^-1 y,
-// is formed from the reverse-mode Cholesky of sum_i log L_ii (k_adjoint.cu)
-// and the on-the-fly contraction of k_gp.cu.
+// is formed from the adjoint of sum_i log L_ii with respect to K (logdet_adjoint_impl) and
+// the on-the-fly contraction of k_gp.cu.
 #include <cmath>
 #include <string>
 #include <vector>
@@ -217,6 +217,65 @@ hs_status cholesky_adjoint_impl(hs_ctx ctx, const double* L, double* Abar, const
     return HS_OK;
 }
 
+hs_status logdet_adjoint_impl(hs_ctx ctx, double* L, double* Abar, const double* Y, const AdjointWork& w,
+                              cudaStream_t s) {
+    // A^-1 = Z block column by block column, k = nb-1 .. 0, with P the rows below block k and
+    // M_P = L_P L_kk^-1 (from L^T Z = L^-1 block by block):
+    //   Z_P = -Z_trailing M_P,   Z_kk = L_kk^-T L_kk^-1 - M_P^T Z_P
+    // The reverse sweep of cholesky_adjoint_impl gives the same from diag(1 / L_ii), in eight
+    // dependent launches a column; these are two, and the products with the diagonal
+    // blocks are one launch each for all columns (a whole gradient at N = 2000: 3.05 -> 1.91
+    // ms, at 16384: 170 -> 159 ms).
+    const int nb = ctx->nb, bsz = ctx->bsz;
+    const int64_t bb = (int64_t)bsz * bsz;
+    hs_status st = launch_scale_panels(ctx, L, Y, s);
+    if (st != HS_OK) return st;
+    ChainArgs g = chain_args(bsz);  // Y_k Y_k^T
+    g.items = nb;
+    g.chain = 1;
+    g.A0 = g.B0 = Y;
+    g.sAi = g.sBi = bb;
+    g.tb = 1;
+    g.C0 = w.T;
+    g.sCi = bb;
+    if ((st = launch_chain(ctx, g, nullptr, 0, s)) != HS_OK) return st;
+    for (int k = nb - 1; k >= 0; --k) {
+        const int m = nb - k - 1;
+        const int64_t dk = block_id(k, k, nb);
+        ChainArgs a = chain_args(bsz);
+        if (m > 0) {
+            a.mode = CHAIN_SYMM;
+            a.k = k;
+            a.nb = nb;
+            a.items = m;
+            a.chain = nb - k;
+            a.allow_split = 1;
+            a.alpha = -1.0;
+            a.L = L;
+            a.Abar = Abar;
+            if ((st = launch_chain(ctx, a, w.partial, w.partial_blocks, s)) != HS_OK) return st;
+            a = chain_args(bsz);
+            a.A0 = L + (dk + 1) * bb;  // M_P
+            a.B0 = Abar + (dk + 1) * bb;
+            a.sAq = a.sBq = bb;
+            a.ta = 1;
+            a.chain = m;
+            a.alpha = -1.0;
+            a.addend = w.T + (size_t)k * bb;
+        } else {
+            a.A0 = a.B0 = Y + (size_t)k * bb;
+            a.tb = 1;
+            a.chain = 1;
+        }
+        a.items = 1;
+        a.C0 = Abar + dk * bb;
+        a.epi = EPI_TRIL_HALF;
+        a.allow_split = 1;
+        if ((st = launch_chain(ctx, a, w.partial, w.partial_blocks, s)) != HS_OK) return st;
+    }
+    return HS_OK;
+}
+
 }  // namespace hs
 
 using namespace hs;
@@ -357,9 +416,9 @@ static hs_status gp_nlml_grad_impl(hs_ctx ctx, const double* X, const double* y,
     ctx->launches += 1;
     nlml_terms_kernel<<<1, 1024, 0, s>>>(y, alpha, L, bsz, nb, N, res);
     HS_CHECK_LAUNCH("nlml terms");
-    // reverse sweep of sum_i log L_ii, then the gradient contraction
-    if ((st = launch_logdet_adjoint_init(ctx, L, Abar, s)) != HS_OK) return st;
-    if ((st = cholesky_adjoint_impl(ctx, L, Abar, w, s)) != HS_OK) return st;
+    // the adjoint of sum_i log L_ii, then the gradient contraction
+    if ((st = launch_diag_inverses(ctx, L, w.Y, w.T, s)) != HS_OK) return st;
+    if ((st = logdet_adjoint_impl(ctx, L, Abar, w.Y, w, s)) != HS_OK) return st;
     HS_CUDA(cudaEventRecord(ev[2], s));
     HS_CUDA(cudaMemcpyAsync(inv_ell_d, inv_ell.data(), d * sizeof(double), cudaMemcpyHostToDevice, s));
     if ((st = launch_scale_columns(ctx, X, Xs, d, inv_ell_d, s)) != HS_OK) return st;

@@ -29,6 +29,7 @@ struct ChainArgs {
     int ta, tb;        // CHAIN_LIST: transposed operands
     double* C0;        // CHAIN_LIST: output of item = C0 + item*sCi
     int64_t sCi;
+    const double* addend = nullptr;  // EPI_TRIL_HALF: a block added to the product before the triangle is taken
     double* partial;   // set by launch_chain
 };
 
@@ -44,10 +45,8 @@ inline ChainArgs chain_args(int bsz) {
 
 // `partial` (nullable) holds `partial_blocks` bsz x bsz blocks for split chains
 hs_status launch_chain(hs_ctx ctx, ChainArgs a, double* partial, int64_t partial_blocks, cudaStream_t s);
-hs_status launch_logdet_adjoint_init(hs_ctx ctx, const double* L, double* Abar, cudaStream_t s);
 hs_status launch_pad_unit_diag(hs_ctx ctx, const double* D, double* Dp, int valid, cudaStream_t s);
 hs_status launch_zero_diag_upper(hs_ctx ctx, double* Abar, cudaStream_t s);
-hs_status launch_identity(hs_ctx ctx, double* Y, cudaStream_t s);
 hs_status launch_sym_tril_half(hs_ctx ctx, const double* G, double* M, cudaStream_t s);
 
 // workspace of the reverse sweep
@@ -66,6 +65,14 @@ void adjoint_bind(void* base, int nb, int bsz, AdjointWork* w);
 // Abar (packed lower blocks, holding Lbar on entry) <- adjoint of the lower
 // entries of A = L L^T; L is not modified
 hs_status cholesky_adjoint_impl(hs_ctx ctx, const double* L, double* Abar, const AdjointWork& w, cudaStream_t s);
+
+// Abar <- the adjoint of sum_i log L_ii with respect to the lower entries of A = L L^T:
+// A^-1 below the diagonal, half of it on the diagonal.  Y: L_kk^-T for every diagonal block.
+// L's off-diagonal blocks are overwritten.
+hs_status logdet_adjoint_impl(hs_ctx ctx, double* L, double* Abar, const double* Y, const AdjointWork& w,
+                              cudaStream_t s);
+// L_rk <- L_rk Y_k^T = L_rk L_kk^-1 for every off-diagonal block of the packed factor
+hs_status launch_scale_panels(hs_ctx ctx, double* L, const double* Y, cudaStream_t s);
 
 // gradient of the GP NLML: sum over stored lower elements of
 // (Abar_ij - c_ij alpha_i alpha_j) dK_ij/dtheta, c = 1/2 on the diagonal

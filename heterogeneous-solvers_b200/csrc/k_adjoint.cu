@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256, 2) chain_dmma_kernel(ChainArgs a) {
             const int r = ti * BM + wm * WM + mi * 8 + g;
             const int c = tj * BN + wn * WN + ni * 8 + 2 * t;
             double* p = C + (size_t)r * bsz + c;
-            const double v0 = alpha * acc[mi][ni][0], v1 = alpha * acc[mi][ni][1];
+            double v0 = alpha * acc[mi][ni][0], v1 = alpha * acc[mi][ni][1];
             if (epi == EPI_STORE) {
                 *reinterpret_cast<double2*>(p) = make_double2(v0, v1);
             } else if (epi == EPI_ADD) {
@@ -226,6 +226,11 @@ __global__ void __launch_bounds__(256, 2) chain_dmma_kernel(ChainArgs a) {
                 if (c <= r) p[0] += v0;
                 if (c + 1 <= r) p[1] += v1;
             } else {  // EPI_TRIL_HALF: lower triangle, diagonal halved, upper zero
+                if (a.addend) {
+                    const double2 o = *reinterpret_cast<const double2*>(a.addend + (size_t)r * bsz + c);
+                    v0 += o.x;
+                    v1 += o.y;
+                }
                 p[0] = c < r ? v0 : (c == r ? 0.5 * v0 : 0.0);
                 p[1] = c + 1 < r ? v1 : (c + 1 == r ? 0.5 * v1 : 0.0);
             }
@@ -248,28 +253,13 @@ __global__ void reduce_splits_kernel(const double* __restrict__ partial, int spl
         else if (a.epi == EPI_ADD_LOWER) {
             if (c <= r) C[e] += s;
         } else {
+            if (a.addend) s += a.addend[e];
             C[e] = c < r ? s : (c == r ? 0.5 * s : 0.0);
         }
     }
 }
 
 // ------------------------------------------------------------------ helpers
-// Abar = 0 except diag(Abar_kk) = 1 / L_ii for valid rows: the adjoint of
-// sum_i log L_ii with respect to L
-__global__ void zero_kernel(double* __restrict__ p, int64_t total) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x)
-        p[e] = 0.0;
-}
-__global__ void set_logdet_diag_kernel(const double* __restrict__ L, double* __restrict__ Abar, int bsz, int nb,
-                                       int64_t N) {
-    const int64_t bb = (int64_t)bsz * bsz;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        const int k = (int)(i / bsz), r = (int)(i % bsz);
-        const int64_t off = block_id(k, k, nb) * bb + (int64_t)r * bsz + r;
-        Abar[off] = 1.0 / L[off];
-    }
-}
-
 // Dp = D with unit diagonal on the rows >= valid (padding rows of the last
 // block): the padded factor is diag(L, I), so its diagonal blocks are invertible
 __global__ void pad_unit_diag_kernel(const double* __restrict__ D, double* __restrict__ Dp, int bsz, int valid) {
@@ -286,11 +276,6 @@ __global__ void zero_diag_upper_kernel(double* __restrict__ Abar, int bsz, int n
     double* D = Abar + block_id(blockIdx.y, blockIdx.y, nb) * bb;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < bsz * bsz; e += gridDim.x * blockDim.x)
         if (e % bsz > e / bsz) D[e] = 0.0;
-}
-
-__global__ void identity_kernel(double* __restrict__ Y, int bsz) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < bsz * bsz; e += gridDim.x * blockDim.x)
-        Y[e] = (e / bsz == e % bsz) ? 1.0 : 0.0;
 }
 
 // M = H + H^T with H = tril_h(G): M_ij = G_ij (i > j), G_ji (i < j), G_ii (i == j)
@@ -363,15 +348,6 @@ hs_status launch_chain(hs_ctx ctx, ChainArgs a, double* partial, int64_t partial
     return HS_OK;
 }
 
-hs_status launch_logdet_adjoint_init(hs_ctx ctx, const double* L, double* Abar, cudaStream_t s) {
-    const int64_t total = total_blocks(ctx->nb) * (int64_t)ctx->bsz * ctx->bsz;
-    ctx->launches += 2;
-    zero_kernel<<<4 * ctx->num_sms, 256, 0, s>>>(Abar, total);
-    set_logdet_diag_kernel<<<64, 256, 0, s>>>(L, Abar, ctx->bsz, ctx->nb, ctx->N);
-    HS_CHECK_LAUNCH("logdet adjoint init");
-    return HS_OK;
-}
-
 hs_status launch_pad_unit_diag(hs_ctx ctx, const double* D, double* Dp, int valid, cudaStream_t s) {
     ctx->launches += 1;
     pad_unit_diag_kernel<<<64, 256, 0, s>>>(D, Dp, ctx->bsz, valid);
@@ -383,13 +359,6 @@ hs_status launch_zero_diag_upper(hs_ctx ctx, double* Abar, cudaStream_t s) {
     ctx->launches += 1;
     zero_diag_upper_kernel<<<dim3(16, ctx->nb), 256, 0, s>>>(Abar, ctx->bsz, ctx->nb);
     HS_CHECK_LAUNCH("zero diag upper");
-    return HS_OK;
-}
-
-hs_status launch_identity(hs_ctx ctx, double* Y, cudaStream_t s) {
-    ctx->launches += 1;
-    identity_kernel<<<64, 256, 0, s>>>(Y, ctx->bsz);
-    HS_CHECK_LAUNCH("identity");
     return HS_OK;
 }
 

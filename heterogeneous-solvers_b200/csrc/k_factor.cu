@@ -14,6 +14,7 @@
 // result is C - sum_k a_ik b_jk accumulated in k order.  Other block sizes use
 // a scalar fallback with the reference's accumulation order.  The diagonal block
 // of bsz 128 and 256 is k_diag.cu's.
+#include "hs_gp.cuh"
 #include "hs_internal.cuh"
 #include "hs_mixed.cuh"
 
@@ -198,14 +199,16 @@ struct DTile {
     static_assert((TM * (BK / 2)) % 32 == 0, "A and B copies must not share a warp");
 };
 
-// PRODUCT = false: C (TM x TN, ldc) <- C - A (TM x K, lda) B (TN x K, ldb)^T,
+// PRODUCT = 0: C (TM x TN, ldc) <- C - A (TM x K, lda) B (TN x K, ldb)^T,
 //   accumulated from -C in k order; with `lower`, entry (r, c) is written only
 //   if c + shift <= r (a tile that crosses the diagonal of a diagonal block).
-// PRODUCT = true: C <- A B with B (K x TN, ldb) upper triangular (B[k][c] = 0 for
+// PRODUCT = 2: C <- A B^T with B (TN x K, ldb) upper triangular (B[c][k] = 0 for k < c):
+//   a warp skips the K slabs before its first column.  C may be A itself.
+// PRODUCT = 1: C <- A B with B (K x TN, ldb) upper triangular (B[k][c] = 0 for
 //   k > c): a warp skips the K slabs past its last column, and what B holds below its
 //   WN x WN diagonal blocks is not used.  C may be A itself: every load of A completes
 //   before the first store.
-template <int TM, int TN, int WM, int WN, int ST, bool PRODUCT>
+template <int TM, int TN, int WM, int WN, int ST, int PRODUCT>
 __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double* Ag, int64_t lda,
                                             const double* __restrict__ Bg, int64_t ldb, int K, bool lower, int shift,
                                             double* smem) {
@@ -214,7 +217,7 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
     double* Bs = smem + ST * TM * SPAD;  // [ST][TN][SPAD]
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    // PRODUCT: later columns have longer sums; warps w and w + 4 share a scheduler, so the
+    // PRODUCT: columns have sums of different lengths; warps w and w + 4 share a scheduler, so the
     // second four take the columns in reverse
     const int wm = warp / D::kWarpsN;
     const int wn = PRODUCT && warp >= 4 ? D::kWarpsN - 1 - warp % 4 % D::kWarpsN : warp % D::kWarpsN;
@@ -238,8 +241,9 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
         }
 
     const int ktiles = K / BK;
-    // PRODUCT: columns wn*WN .. wn*WN+WN-1 of B vanish past row wn*WN+WN-1
-    const int kt_warp = PRODUCT ? min(ktiles, (wn * WN + WN + BK - 1) / BK) : ktiles;
+    // PRODUCT 1: columns wn*WN .. wn*WN+WN-1 of B vanish past row wn*WN+WN-1; 2: before row wn*WN
+    const int kt_warp = PRODUCT == 1 ? min(ktiles, (wn * WN + WN + BK - 1) / BK) : ktiles;
+    const int kt_first = PRODUCT == 2 ? wn * WN / BK : 0;
     auto load_stage = [&](int stage, int kt) {
         const int kc = kt * BK;
 #pragma unroll
@@ -248,7 +252,7 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
             const int row = e >> 3, ch = e & 7;
             if (row < TM) {
                 cp_async16(As + (stage * TM + row) * SPAD + ch * 2, Ag + (size_t)row * lda + kc + ch * 2);
-            } else if (PRODUCT) {
+            } else if (PRODUCT == 1) {
                 const int eb = e - TM * (BK / 2), kr = eb / (TN / 2), cc = 2 * (eb % (TN / 2));
                 cp_async16(Bs + stage * D::kBStage + kr * D::kBRow + cc, Bg + (size_t)(kc + kr) * ldb + cc);
             } else {
@@ -270,17 +274,17 @@ __device__ __forceinline__ void dmma_tile_t(double* C, int64_t ldc, const double
             if (nk < ktiles) load_stage(nk % ST, nk);
             cp_async_commit();
         }
-        if (kt < kt_warp) {
+        if (kt >= kt_first && kt < kt_warp) {
             const double* as = As + (kt % ST) * TM * SPAD + (wm * WM + g) * SPAD + t;
             const double* bs = Bs + (kt % ST) * D::kBStage +
-                               (PRODUCT ? t * D::kBRow + wn * WN + g : (wn * WN + g) * SPAD + t);
+                               (PRODUCT == 1 ? t * D::kBRow + wn * WN + g : (wn * WN + g) * SPAD + t);
 #pragma unroll
             for (int kk = 0; kk < BK / 4; ++kk) {
                 double a[D::kMi], b[D::kNi];
 #pragma unroll
                 for (int mi = 0; mi < D::kMi; ++mi) a[mi] = as[mi * 8 * SPAD + kk * 4];
 #pragma unroll
-                for (int ni = 0; ni < D::kNi; ++ni) b[ni] = PRODUCT ? bs[kk * 4 * D::kBRow + ni * 8] : bs[ni * 8 * SPAD + kk * 4];
+                for (int ni = 0; ni < D::kNi; ++ni) b[ni] = PRODUCT == 1 ? bs[kk * 4 * D::kBRow + ni * 8] : bs[ni * 8 * SPAD + kk * 4];
 #pragma unroll
                 for (int mi = 0; mi < D::kMi; ++mi)
 #pragma unroll
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(DTile<TM, TN, WM, WN, ST>::kThreads, CTAS) upd
     double* C = a.A + (size_t)block_id(r, c, a.nb) * bb + (size_t)ti * TM * a.bsz + (size_t)tj * TN;
     const double* Ag = a.A + (size_t)(a.blockID + (r - a.blockRow)) * bb + (size_t)ti * TM * a.bsz;
     const double* Bg = a.A + (size_t)(a.blockID + (c - a.blockRow)) * bb + (size_t)tj * TN * a.bsz;
-    dmma_tile_t<TM, TN, WM, WN, ST, false>(C, a.bsz, Ag, a.bsz, Bg, a.bsz, a.bsz, lower, shift, smem);
+    dmma_tile_t<TM, TN, WM, WN, ST, 0>(C, a.bsz, Ag, a.bsz, Bg, a.bsz, a.bsz, lower, shift, smem);
 }
 constexpr auto update_large = update_dmma_kernel<kUTM, kUTN, kUWM, kUWN, kUST, 2>;
 constexpr auto update_small = update_dmma_kernel<32, 32, 16, 16, 3, 4>;
@@ -404,7 +408,20 @@ __global__ void __launch_bounds__(256, 1) trsm_dmma_kernel(double* A, int64_t fi
     const int64_t item = blockIdx.x / kSlabs;
     const int slab = blockIdx.x % kSlabs;
     double* B = A + (size_t)(firstBlock + item) * BSZ * BSZ + (size_t)slab * ROWS * BSZ;
-    dmma_tile_t<ROWS, BSZ, 32, ROWS * BSZ / 256, 3, true>(B, BSZ, B, BSZ, Y, BSZ, BSZ, false, 0, smem);
+    dmma_tile_t<ROWS, BSZ, 32, ROWS * BSZ / 256, 3, 1>(B, BSZ, B, BSZ, Y, BSZ, BSZ, false, 0, smem);
+}
+
+// L_rk <- L_rk Y_k^T for every off-diagonal block, one CTA per ROWS rows of a block
+template <int BSZ, int ROWS>
+__global__ void __launch_bounds__(256, 1) scale_panels_kernel(double* L, int nb, const double* __restrict__ Y) {
+    extern __shared__ __align__(16) double smem[];
+    constexpr int kSlabs = BSZ / ROWS;
+    const int64_t pair = blockIdx.x / kSlabs;  // (r, k), r > k: triangle of nb - 1 columns
+    int i, k;
+    block_coords(pair, nb - 1, &i, &k);
+    double* B = L + ((size_t)block_id(i + 1, k, nb) * BSZ + (size_t)(blockIdx.x % kSlabs) * ROWS) * BSZ;
+    dmma_tile_t<ROWS, BSZ, 32, ROWS * BSZ / 256, 3, 2>(B, BSZ, B, BSZ, Y + (size_t)k * BSZ * BSZ, BSZ, BSZ, false, 0,
+                                                       smem);
 }
 
 // scalar fallback (any bsz): one thread per output element; SYRK follows
@@ -449,6 +466,10 @@ hs_status set_attrs() {
                                  TrsmTile<128, 32>::kSmem));
     HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  TrsmTile<256, 32>::kSmem));
+    HS_CUDA(cudaFuncSetAttribute(scale_panels_kernel<128, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 TrsmTile<128, 64>::kSmem));
+    HS_CUDA(cudaFuncSetAttribute(scale_panels_kernel<256, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 TrsmTile<256, 64>::kSmem));
     HS_CUDA(cudaFuncSetAttribute(trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(256)));
     HS_CUDA(cudaFuncSetAttribute(potrf_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(128 * 129 * sizeof(double))));
@@ -531,6 +552,26 @@ hs_status launch_trsm_dmma(hs_ctx ctx, double* A, int64_t firstBlock, int blockC
     HS_CHECK_LAUNCH("trsm_dmma");
     // algorithmic work: the triangular solve's n^3 flops a block
     prof_end(ctx, s, HS_KERNEL_TRSM, blockCount * n * n * n, (2.0 * blockCount + 1.0) * n * n * 8.0);
+    return HS_OK;
+}
+
+hs_status launch_scale_panels(hs_ctx ctx, double* L, const double* Y, cudaStream_t s) {
+    const int nb = ctx->nb, bsz = ctx->bsz;
+    if (nb < 2) return HS_OK;
+    hs_status st = set_attrs();
+    if (st != HS_OK) return st;
+    HS_REQUIRE(bsz == 128 || bsz == 256, "the tensor-core panels need matrixBlockSize 128 or 256");
+    const int64_t blocks = total_blocks(nb - 1), grid = blocks * (bsz / 64);
+    HS_REQUIRE(grid < (1LL << 31), "too many blocks");
+    const double n = bsz;
+    prof_begin(ctx, s, HS_KERNEL_ADJOINT);
+    ctx->launches += 1;
+    if (bsz == 256)
+        scale_panels_kernel<256, 64><<<(unsigned)grid, 256, TrsmTile<256, 64>::kSmem, s>>>(L, nb, Y);
+    else
+        scale_panels_kernel<128, 64><<<(unsigned)grid, 256, TrsmTile<128, 64>::kSmem, s>>>(L, nb, Y);
+    HS_CHECK_LAUNCH("scale_panels");
+    prof_end(ctx, s, HS_KERNEL_ADJOINT, blocks * n * n * n, 2.0 * blocks * n * n * 8.0);
     return HS_OK;
 }
 

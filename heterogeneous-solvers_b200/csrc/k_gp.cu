@@ -36,28 +36,31 @@ __global__ void __launch_bounds__(kGradThreads) gp_grad_kernel(const double* __r
                                                                const double* __restrict__ Xs,
                                                                const double* __restrict__ alpha, int d, int ard,
                                                                double sf2, double sn2, int bsz, int nb, int64_t N,
-                                                               int64_t T, double* __restrict__ part) {
+                                                               int64_t T, int rows, double* __restrict__ part) {
     extern __shared__ double sm[];
-    double* xr = sm;                   // [bsz][d]  rows of the row block
-    double* xc = sm + (size_t)bsz * d; // [d][bsz]  rows of the column block, transposed
+    double* xr = sm;                    // [rows][d]  rows of the row block
+    double* xc = sm + (size_t)rows * d; // [d][bsz]  rows of the column block, transposed
     constexpr int NACC = DMAX + 2;
     double acc[NACC];
 #pragma unroll
     for (int q = 0; q < NACC; ++q) acc[q] = 0.0;
     const int64_t bb = (int64_t)bsz * bsz;
-    for (int64_t blk = blockIdx.x; blk < T; blk += gridDim.x) {
+    const int nsub = bsz / rows;  // slices of `rows` rows of a block
+    for (int64_t item = blockIdx.x; item < T * nsub; item += gridDim.x) {
+        const int64_t blk = item / nsub;
+        const int r0 = (int)(item % nsub) * rows;
         int bi, bj;
         block_coords(blk, nb, &bi, &bj);
-        const int64_t i0 = (int64_t)bi * bsz, j0 = (int64_t)bj * bsz;
+        const int64_t i0 = (int64_t)bi * bsz + r0, j0 = (int64_t)bj * bsz;
         __syncthreads();
+        for (int e = threadIdx.x; e < rows * d; e += blockDim.x) xr[e] = (i0 + e / d < N) ? Xs[i0 * d + e] : 0.0;
         for (int e = threadIdx.x; e < bsz * d; e += blockDim.x) {
             const int r = e / d, k = e % d;
-            xr[e] = (i0 + r < N) ? Xs[(i0 + r) * d + k] : 0.0;
             xc[(size_t)k * bsz + r] = (j0 + r < N) ? Xs[(j0 + r) * d + k] : 0.0;
         }
         __syncthreads();
-        const double* Ab = Abar + blk * bb;
-        for (int64_t e = threadIdx.x; e < bb; e += blockDim.x) {
+        const double* Ab = Abar + blk * bb + (int64_t)r0 * bsz;
+        for (int64_t e = threadIdx.x; e < (int64_t)rows * bsz; e += blockDim.x) {
             const int i = (int)(e / bsz), j = (int)(e % bsz);
             const int64_t gi = i0 + i, gj = j0 + j;
             if (gi >= N || gj >= N || gj > gi) continue;
@@ -105,11 +108,12 @@ __global__ void __launch_bounds__(kGradThreads) gp_grad_kernel(const double* __r
 template <int DMAX>
 __global__ void grad_final_kernel(const double* __restrict__ part, int parts, double* __restrict__ out) {
     constexpr int NACC = DMAX + 2;
-    const int q = threadIdx.x;
-    if (q >= NACC) return;
+    // one warp a component: lanes stride the parts, then a tree (a fixed order)
+    const int q = blockIdx.x, lane = threadIdx.x;
     double s = 0.0;
-    for (int p = 0; p < parts; ++p) s += part[(int64_t)p * NACC + q];
-    out[q] = s;
+    for (int p = lane; p < parts; p += 32) s += part[(int64_t)p * NACC + q];
+    s = warp_sum(s);
+    if (lane == 0) out[q] = s;
 }
 
 template <int DMAX>
@@ -122,9 +126,13 @@ hs_status grad_launch(hs_ctx ctx, const double* Abar, const double* Xs, const do
     const int64_t T = total_blocks(ctx->nb);
     prof_begin(ctx, s, HS_KERNEL_GRAD);
     ctx->launches += 2;
+    // whole blocks where there are several for every CTA, else slices of them (36 blocks of
+    // 256 on 296 CTAs: 279 -> 50 us with slices of 16 rows)
+    int rows = bsz;
+    while (rows % 2 == 0 && rows > 16 && T * (bsz / rows) < 4LL * parts) rows /= 2;
     gp_grad_kernel<DMAX><<<parts, kGradThreads, smem, s>>>(Abar, Xs, alpha, d, ard, sf2, sn2, bsz, ctx->nb, ctx->N,
-                                                            T, part);
-    grad_final_kernel<DMAX><<<1, 64, 0, s>>>(part, parts, out);
+                                                            T, rows, part);
+    grad_final_kernel<DMAX><<<DMAX + 2, 32, 0, s>>>(part, parts, out);
     HS_CHECK_LAUNCH("gp_grad");
     const double elems = (double)ctx->N * (ctx->N + 1) / 2.0;
     prof_end(ctx, s, HS_KERNEL_GRAD, elems * (4.0 * d + 12.0), (double)T * bsz * bsz * 8.0);
