@@ -397,6 +397,10 @@ hs_status hs_ctx_take_info(hs_ctx ctx, int64_t* info) {
     ctx->launches += 1;
     set_i64_kernel<<<1, 1, 0, ctx->stream>>>(ctx->d_info, INT64_MAX);
     HS_CHECK_LAUNCH("reset info");
+    if (v < 0) {  // the trailing update's mark
+        set_error("hs_ctx_take_info: a bounded wait of the factor's trailing update ran out");
+        return HS_ERR_TIMEOUT;
+    }
     if (info) *info = (v == INT64_MAX) ? -1 : (int64_t)v;
     return HS_OK;
 }

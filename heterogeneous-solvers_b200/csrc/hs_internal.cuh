@@ -167,6 +167,34 @@ __host__ __device__ __forceinline__ int tri_root(int64_t t) {
     return r;
 }
 
+__host__ __device__ __forceinline__ int64_t tri64(int64_t n) { return n * (n + 1) / 2; }
+// block rows a group of the grouped enumeration of a trailing triangle holds
+constexpr int kGroup = 16;
+// pair p of the grouped enumeration of the m x m lower triangle -> (r', c')
+__device__ __forceinline__ void grouped_pair(int64_t p, int m, int* rr, int* cc) {
+    int lo = 0, hi = (m + kGroup - 1) / kGroup;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tri64((int64_t)mid * kGroup) <= p) lo = mid; else hi = mid - 1;
+    }
+    const int r0 = lo * kGroup;
+    const int r1 = min(r0 + kGroup, m), h = r1 - r0;
+    int64_t l = p - tri64(r0);
+    if (l < (int64_t)r0 * h) {
+        *rr = r0 + (int)(l % h);
+        *cc = (int)(l / h);
+        return;
+    }
+    l -= (int64_t)r0 * h;
+    int j = 0;
+    while (l >= h - j) {
+        l -= h - j;
+        ++j;
+    }
+    *rr = r0 + j + (int)l;
+    *cc = r0 + j;
+}
+
 inline size_t block_elems(const hs_ctx ctx) { return (size_t)ctx->bsz * (size_t)ctx->bsz; }
 
 // ---------------------------------------------------------- kernel entry points
@@ -185,6 +213,12 @@ hs_status launch_update(hs_ctx ctx, double* A, int blockID, int blockRow, int sy
 // (SYRK on their diagonal blocks, GEMM below them)
 hs_status launch_update_cols(hs_ctx ctx, double* A, int blockID, int blockRow, int colStart, int colEnd,
                              cudaStream_t s);
+// the same for the columns [colStart, nb) or one column on the INT8 tensor cores
+// (k_split_update.cu): first the digits of panel k, then its update, on one stream.  ws:
+// split_update_bytes, 256-byte aligned; a wait that ran out: -1 in d_info
+size_t split_update_bytes(int nb, int bsz);
+hs_status launch_split_digits(hs_ctx ctx, const double* A, int k, void* ws, cudaStream_t s);
+hs_status launch_split_update(hs_ctx ctx, double* A, int k, int colStart, int colEnd, void* ws, cudaStream_t s);
 // one diagonal block of bsz 128 or 256 (k_diag.cu): L and its inverse in one launch
 struct DiagFactor {
     const double* in64 = nullptr;  // the block, or

@@ -11,7 +11,8 @@
 // runs on the FP64 tensor pipe (DMMA, mma.sync m8n8k4 f64): 128x64 output tiles,
 // two CTAs an SM, K streamed in 16-wide slabs through a 3-stage cp.async ring in
 // shared memory, accumulators held in registers and initialised with -C so the
-// result is C - sum_k a_ik b_jk accumulated in k order.  Other block sizes use
+// result is C - sum_k a_ik b_jk accumulated in k order (the factor's large updates are
+// k_split_update.cu's).  Other block sizes use
 // a scalar fallback with the reference's accumulation order.  The diagonal block
 // of bsz 128 and 256 is k_diag.cu's.
 #include "hs_gp.cuh"

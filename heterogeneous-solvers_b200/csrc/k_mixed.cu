@@ -311,7 +311,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // L2 traffic but adds shared-memory traffic on the port the tensor core reads
 // its operands through; measured slower.  Strips of 16 block rows were ~1.5 %
 // faster than 8 at N=131072, strips of 32 ~8 % slower.)
-constexpr int kGroup = 16;
 constexpr int kUpdThreads = 320;
 // K floats per stage: 32 (128-byte rows, 128-byte swizzle, 2 stages of 96 KB)
 // measured faster than 16 (64-byte swizzle, 4 stages of 48 KB); the kernel is
@@ -365,7 +364,6 @@ __device__ __forceinline__ uint64_t upd_desc(uint32_t addr) {
     return kUpdK == 32 ? umma_desc_sw128(addr) : umma_desc_sw64(addr);
 }
 
-__host__ __device__ __forceinline__ int64_t tri64(int64_t n) { return n * (n + 1) / 2; }
 
 // Tile hand-off inside a CTA of the persistent update.  The producer takes the
 // CTA's j-th tile (from the shared counter, or by stride) and publishes it in slot
@@ -413,31 +411,6 @@ __host__ __device__ __forceinline__ int64_t update_tiles(int part, int m, int nc
     else
         blocks = tri64(part == 2 ? m - 1 : m);
     return blocks * tiles_per_block;
-}
-
-// pair p of the grouped enumeration of the m x m lower triangle -> (r', c')
-__device__ __forceinline__ void grouped_pair(int64_t p, int m, int* rr, int* cc) {
-    int lo = 0, hi = (m + kGroup - 1) / kGroup;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (tri64((int64_t)mid * kGroup) <= p) lo = mid; else hi = mid - 1;
-    }
-    const int r0 = lo * kGroup;
-    const int r1 = min(r0 + kGroup, m), h = r1 - r0;
-    int64_t l = p - tri64(r0);
-    if (l < (int64_t)r0 * h) {
-        *rr = r0 + (int)(l % h);
-        *cc = (int)(l / h);
-        return;
-    }
-    l -= (int64_t)r0 * h;
-    int j = 0;
-    while (l >= h - j) {
-        l -= h - j;
-        ++j;
-    }
-    *rr = r0 + j + (int)l;
-    *cc = r0 + j;
 }
 
 // mU*: maps of the hi parts, mV*: of the lo parts (*128: 128-row boxes, *B: BSZ-row boxes)

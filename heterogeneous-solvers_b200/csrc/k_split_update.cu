@@ -1,0 +1,417 @@
+// k_split_update.cu — the FP64 trailing update on the tensor cores' INT8 path.
+//
+// The large trailing updates of the FP64 Cholesky (MatrixMatrixOperations.cpp:146-906) are
+// C <- C - P P^T with a panel P of one block column.  The FP64 tensor pipe bounds them at 64
+// multiply-adds a cycle and SM; the INT8 pipe does over a hundred times that.  Each row of the panel
+// is therefore scaled by a power of two to |t| <= 0.497 and written as seven balanced
+// base-256 digits, t = sum_i d_i 2^-8(i+1) with |error| <= 2^-57, and the product of two rows
+// is the sum over levels l = i + j of 2^-8l (digit plane i) x (digit plane j): exact INT32
+// sums in the tensor cores, levels 0..7 kept (34 plane products), carried into one 64-bit
+// integer, rounded to FP64 once and added to C.  (K. Ozaki, T. Ogita,
+// S. Oishi, S. M. Rump, "Error-free transformations of matrix multiplication by using fast
+// routines of matrix multiplication and its applications", 2012; H. Ootomo, K. Ozaki, R.
+// Yokota, "DGEMM on integer matrix multiplication unit", 2024.)
+//
+// Error of one update, in units of the rows' scales: the digits' 2^-57 a factor, levels
+// past 7 at most 2^-64 a product and the last unit 2^-57; then a rounding of the product and
+// one of C.  The FP64 pipe's chain rounds 64 times at 2^-53 |C|.  Measured, max |A - L L^T| /
+// sqrt(a_ii a_jj) of a factor at N = 4800 (Wishart): 7.6e-15 -> 2.4e-15.  Scale_i scale_j <= 16 max|P_i| max|P_j| <= 16 sqrt(A_ii A_jj), so the
+// factor keeps the backward error bound of the plain form, relative to sqrt(A_ii A_jj).
+#include "hs_internal.cuh"
+#include "stream_common.cuh"
+#include "tc_common.cuh"
+
+namespace hs {
+
+namespace {
+
+using namespace tc;
+
+constexpr int kPlanes = 7, kHighPlanes = 4;  // digits a value; those of levels 0..3
+constexpr int kKc = 64;                      // K bytes a stage (64-byte swizzle)
+constexpr int kPlane = 128 * kKc;            // one plane of 128 rows of a stage
+constexpr int kOperand = kPlanes * kPlane;
+constexpr int kStage = 2 * kOperand, kStages = 2;  // 112 KB each
+constexpr int kSmem = 512 + kStages * kStage + 256 * 8 + 104;  // + the tile's scales, barriers
+constexpr int kEpi = 16, kThreads = 64 + 32 * kEpi;  // copy warp, MMA warp, epilogue warps
+constexpr int kPerCta = 4;     // tiles a CTA
+constexpr int kMinExp = -900;  // rows whose largest entry lies below 2^-900 keep that scale
+
+// ------------------------------------------------------------------ digits
+// One warp a row of the panel: its scale and its seven planes, in the order the update reads them: for
+// each 128 rows and 64 columns the planes one after the other, each as 64-byte rows with the
+// 64-byte swizzle (16-byte unit u of row r at u ^ (r / 2 % 4)), so that an operand's stage is
+// one contiguous copy.  A row that holds an infinity or NaN gets the scale NaN (and zero
+// digits), so that what it updates becomes NaN.
+template <int BSZ>
+__global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ P, int64_t rows, int8_t* __restrict__ D,
+                                                     double* __restrict__ scale) {
+    constexpr int E = BSZ / 32;  // entries a lane
+    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    double v[E];
+    long long m = 0;
+#pragma unroll
+    for (int q = 0; q < E / 2; ++q) {
+        const double2 x = *reinterpret_cast<const double2*>(P + row * BSZ + lane * E + 2 * q);
+        v[2 * q] = x.x;
+        v[2 * q + 1] = x.y;
+    }
+#pragma unroll
+    for (int q = 0; q < E; ++q) m = max(m, __double_as_longlong(v[q]) & 0x7fffffffffffffffll);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const bool finite = m < 0x7ff0000000000000ll;
+    // m < 2^(E - 1022); |t| = |x| 2^-e <= 0.497 keeps every digit within [-128, 127]
+    int e = max((int)(m >> 52) - 1021 + (((m >> 44) & 0xff) >= 0xfd), kMinExp);
+    const double s = __longlong_as_double((long long)(56 - (finite ? e : 0) + 1023) << 52);
+    unsigned long long u[E];
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        // adding 128 to every digit makes the bytes of the sum the digits plus 128
+        const long long t = finite ? __double2ll_rn(v[q] * s) : 0;
+        u[q] = ((unsigned long long)(t + 0x0080808080808080ll)) ^ 0x0080808080808080ull;
+    }
+    const int r = (int)(row & 127), chunk = lane * E / kKc, byte = lane * E % kKc;
+    int8_t* out = D + ((row >> 7) * (BSZ / kKc) + chunk) * kOperand + r * kKc +
+                  (((byte >> 4) ^ (r >> 1 & 3)) << 4) + (byte & 15);
+#pragma unroll
+    for (int i = 0; i < kPlanes; ++i) {
+        const int sh = 8 * (kPlanes - 1 - i);
+        unsigned w[E / 4];
+#pragma unroll
+        for (int q = 0; q < E / 4; ++q)
+            w[q] = (unsigned)(u[4 * q] >> sh & 0xff) | (unsigned)(u[4 * q + 1] >> sh & 0xff) << 8 |
+                   (unsigned)(u[4 * q + 2] >> sh & 0xff) << 16 | (unsigned)(u[4 * q + 3] >> sh & 0xff) << 24;
+        int8_t* dst = out + i * kPlane;
+        if constexpr (E == 8)
+            *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+        else
+            *reinterpret_cast<unsigned*>(dst) = w[0];
+    }
+    // two rows' scales together turn units of 2^-56 into the product
+    if (lane == 0)
+        scale[row] = finite ? __longlong_as_double((long long)(e - 28 + 1023) << 52) : __longlong_as_double(~0ll);
+}
+
+// ------------------------------------------------------------------ update
+struct SplitArgs {
+    double* A;
+    const int8_t* digits;
+    const double* scale;  // of the panel's rows, from the block below the diagonal on
+    int k, nb, bsz;
+    int first_col, m;  // trailing block columns [first_col, first_col + m), one column if !triangle
+    int triangle;
+    int64_t items;     // 128 x 128 tiles
+    long long* info;
+};
+
+// kind::i8 instruction descriptor: D s32 (2 at bit 4), A and B signed (1 at bits 7 and 10),
+// both K-major, N >> 3 in [17, 23), M >> 4 in [24, 29)
+constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+
+__device__ __forceinline__ void umma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(kIdesc), "r"(accumulate)
+        : "memory");
+}
+
+// The products of levels LEVEL + 3 .. LEVEL of one stage, highest first, as straight-line code with
+// descriptors at constant distances (in a loop that formed each descriptor a product took 130
+// cycles to issue; the tensor core takes 64).  wait / done: the four accumulators'
+// barriers, or null.
+template <int LEVEL>
+__device__ __forceinline__ bool issue_levels(uint32_t taddr, uint64_t da, uint32_t accumulate, uint64_t* wait,
+                                             uint64_t* done, uint32_t parity, volatile int* fail) {
+    const uint64_t db = da + (kOperand >> 4);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        if (wait) {
+            if (!thread_wait(&wait[x], parity, fail)) return false;
+            tc_fence_after();
+        }
+        constexpr int kTop = kPlanes - 1;
+        const int level = LEVEL + 3 - x, first = level > kTop ? level - kTop : 0, last = level < kTop ? level : kTop;
+#pragma unroll
+        for (int i = first; i <= last; ++i)
+#pragma unroll
+            for (int ks = 0; ks < kKc / 32; ++ks)
+                umma_i8(taddr + x * 128, da + ((i * kPlane + ks * 32) >> 4),
+                        db + (((level - i) * kPlane + ks * 32) >> 4), i > first || ks > 0 ? 1u : accumulate);
+        if (done) umma_commit(&done[x]);
+    }
+    return true;
+}
+
+// top 2^32 + low, rounded to nearest; exact halves by the exponent's position (the conversion
+// instruction from 64 bits is slower)
+__device__ __forceinline__ double to_double(int top, unsigned low) {
+    const double hi = __hiloint2double(0x43300000, top ^ (int)0x80000000) - 4503601774854144.0;  // 2^52 + 2^31
+    const double lo = __hiloint2double(0x43300000, (int)low) - 4503599627370496.0;               // 2^52
+    return fma(hi, 4294967296.0, lo);
+}
+
+__device__ __forceinline__ void red_add(double* p, double v) {
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+
+// a tile: its entry (0, 0) in A, its rows' and columns' first rows in the panel, in 128s
+struct Tile {
+    int64_t c;
+    int rows, cols;
+    bool skip, lower;  // above the diagonal; crosses it
+};
+__device__ __forceinline__ Tile decode(const SplitArgs& a, int64_t item) {
+    const int side = a.bsz >> 7, lg = a.bsz == 256 ? 2 : 0;
+    const int64_t p = item >> lg;
+    const int e = (int)item & ((1 << lg) - 1), ti = e >> (lg >> 1), tj = e & (side - 1);
+    int rr = (int)p, cc = 0;
+    if (a.triangle) grouped_pair(p, a.m, &rr, &cc);
+    rr += a.first_col;
+    cc += a.first_col;
+    Tile t;
+    t.c = (block_id(rr, cc, a.nb) * a.bsz + ti * 128) * a.bsz + tj * 128;
+    t.rows = (rr - a.k - 1) * side + ti;
+    t.cols = (cc - a.k - 1) * side + tj;
+    t.skip = t.rows < t.cols;
+    t.lower = t.rows == t.cols;
+    return t;
+}
+
+// One CTA: kPerCta consecutive 128 x 128 tiles, two passes each: levels 7..4 (24 plane
+// products, all planes), then 3..0 (10 products of planes 0..3).  A pass's four levels are
+// four accumulators of 128 columns, the whole of TMEM; in a pass's last K chunk the levels
+// are finished one by one and in the next pass's first chunk begun one by one, so that the
+// epilogue warps drain a level while the others are being computed.  C gets one add an
+// entry, without a load (loads of C waited behind the copies' queue: 4 us more a tile).
+// N = 64 would read shared memory 1.5 times as fast as it delivers; 128 columns take all of
+// it, and copies and adds contend with the operands (measured without them: 15 us a tile).
+// A tile of a 256-wide panel takes an SM 21 us (45 us on the FP64 pipe); the update of
+// 62 block columns of 256 2.15 -> 1.10 ms.
+__global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) {
+    extern __shared__ uint8_t raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 511) & ~(uintptr_t)511);
+    double* scales = reinterpret_cast<double*>(smem + kStages * kStage);  // 128 rows, 128 columns
+    uint64_t* bars = reinterpret_cast<uint64_t*>(scales + 256);
+    uint64_t *full = bars, *empty = bars + kStages, *tfull = empty + kStages, *tempty = tfull + 4, *drained = tempty + 4;
+    uint32_t* slot = reinterpret_cast<uint32_t*>(drained + 1);
+    int* fail = reinterpret_cast<int*>(slot + 1);
+    __shared__ Tile tiles[kPerCta];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStages; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(&tfull[i], 1);
+            mbar_init(&tempty[i], kEpi);
+        }
+        mbar_init(drained, 1);
+        *fail = 0;
+        fence_barrier_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(slot, 512);
+        tmem_relinquish();
+    }
+    if (warp == 2 && lane < kPerCta && (int64_t)blockIdx.x * kPerCta + lane < a.items)
+        tiles[lane] = decode(a, (int64_t)blockIdx.x * kPerCta + lane);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t taddr = *slot;
+    const int count = (int)min((int64_t)kPerCta, a.items - (int64_t)blockIdx.x * kPerCta);
+    const int chunks = a.bsz / kKc;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t g = 0;
+            bool ok = true;
+            for (int it = 0; it < count && ok; ++it) {
+                const Tile t = tiles[it];
+                if (t.skip) continue;
+                const int8_t* dA = a.digits + (int64_t)t.rows * chunks * kOperand;
+                const int8_t* dB = a.digits + (int64_t)t.cols * chunks * kOperand;
+                for (int pass = 0; pass < 2 && ok; ++pass) {
+                    const uint32_t bytes = (pass ? kHighPlanes : kPlanes) * kPlane;
+                    for (int kc = 0; kc < chunks; ++kc, ++g) {
+                        const uint32_t s = g % kStages;
+                        if (g >= kStages && !thread_wait(&empty[s], (g / kStages - 1) & 1, fail)) {
+                            ok = false;
+                            break;
+                        }
+                        uint8_t* st = smem + s * kStage;
+                        mbar_arrive_expect_tx(&full[s], 2 * bytes);
+                        bulk_load(st, dA + kc * kOperand, bytes, &full[s]);
+                        bulk_load(st + kOperand, dB + kc * kOperand, bytes, &full[s]);
+                    }
+                }
+            }
+            // no load may still be writing into shared memory when the CTA leaves
+            for (uint32_t h = g > kStages ? g - kStages : 0; h < g; ++h) {
+                const long long t0 = clock64();
+                while (!mbar_test(&full[h % kStages], (h / kStages) & 1) && clock64() - t0 < kWaitClk) {}
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            uint32_t g = 0, u = 0;
+            bool ok = true;
+            for (int it = 0; it < count && ok; ++it) {
+                if (tiles[it].skip) continue;
+                for (int pass = 0; pass < 2 && ok; ++pass, ++u) {
+                    for (int kc = 0; kc < chunks; ++kc, ++g) {
+                        const uint32_t s = g % kStages;
+                        if (!(ok = thread_wait(&full[s], (g / kStages) & 1, fail))) break;
+                        tc_fence_after();
+                        const uint64_t da = umma_desc_sw64(smem_u32(smem + s * kStage));
+                        uint64_t* wait = kc == 0 && u > 0 ? tempty : nullptr;
+                        uint64_t* done = kc == chunks - 1 ? tfull : nullptr;
+                        ok = pass == 0 ? issue_levels<kHighPlanes>(taddr, da, kc > 0, wait, done, (u - 1) & 1, fail)
+                                       : issue_levels<0>(taddr, da, kc > 0, wait, done, (u - 1) & 1, fail);
+                        if (!ok) break;
+                        umma_commit(&empty[s]);
+                    }
+                }
+            }
+            // TMEM is released only after every MMA issued here has completed
+            umma_commit(drained);
+            const long long t0 = clock64();
+            while (!mbar_test(drained, 0) && clock64() - t0 < kWaitClk) {}
+        }
+    } else {
+        // warp: rows 32 q .. +31 and 32 columns of the tile.  TMEM is read in 16 x 32 pieces
+        // whose lane (g, t) holds rows g and g + 8, columns 8 j + 2 t and the next: an access to
+        // C takes 64 bytes of each of eight rows (a row a lane: 32 lines an access).
+        const int q = warp & 3, col0 = ((warp - 2) >> 2) * 32, gr = lane >> 2, t4 = lane & 3;
+        const uint32_t tcol = taddr + ((uint32_t)(q * 32) << 16) + col0;
+        uint32_t u = 0;
+        bool ok = true;
+        for (int it = 0; it < count; ++it) {  // also after a wait ran out: the barriers below
+            const Tile t = tiles[it];
+            if (t.skip) continue;
+            double* C = a.A + t.c + (int64_t)(32 * q) * a.bsz + col0;
+            const int e = threadIdx.x - 64;
+            const double sc = e < 256 ? a.scale[(int64_t)(e < 128 ? t.rows : t.cols) * 128 + (e & 127)] : 0.0;
+            asm volatile("bar.sync 1, 512;" ::: "memory");  // every warp has read the last tile's
+            if (e < 256) scales[e] = sc;
+            asm volatile("bar.sync 1, 512;" ::: "memory");
+            // The levels come lowest first and each is carried into the next, so that 32 bits do:
+            // top = the sum so far in the last level's unit, low = the bytes below it (the
+            // last one 2^-56; of levels 6 and 7 only the carry, rounded to nearest).
+            int top[2][16];  // [row half]
+            unsigned low[2][16];
+#pragma unroll
+            for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    if (ok) ok = warp_wait(&tfull[x], (u + pass) & 1, fail);
+                    if (!ok) continue;
+                    tc_fence_after();
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t v[16];
+                        tmem_ld_16x256b_x4(tcol + ((uint32_t)(16 * h) << 16) + x * 128, v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            int& w = top[h][e];
+                            const int p = (int)v[e], level = pass ? 3 - x : 7 - x;
+                            if (level == 4)
+                                low[h][e] = (unsigned)w << 24;
+                            else if (level < 4 && level > 0)
+                                low[h][e] = __funnelshift_r(low[h][e], w, 8);
+                            w = level == 7 ? p + (1 << 15) : level > 0 ? (w >> 8) + p : w + p * 256;
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty[x]);
+                }
+            }
+            if (!ok) continue;
+            u += 2;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int o = 0; o < 2; ++o) {  // rows g + 8 o of the half
+                    const int r = 16 * h + 8 * o + gr;
+                    double* p = C + (size_t)r * a.bsz + 2 * t4;
+                    const double sr = scales[32 * q + r];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int cc = 8 * j + 2 * t4;
+                        const double2 s2 = *reinterpret_cast<const double2*>(scales + 128 + col0 + cc);
+                        const int over = col0 + cc - 32 * q - r;  // > 0: above the diagonal, as it was
+                        if (!t.lower || over <= 0) red_add(p + 8 * j, -(to_double(top[h][4 * j + 2 * o], low[h][4 * j + 2 * o]) * sr) * s2.x);
+                        if (!t.lower || over < 0) red_add(p + 8 * j + 1, -(to_double(top[h][4 * j + 2 * o + 1], low[h][4 * j + 2 * o + 1]) * sr) * s2.y);
+                    }
+                }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && *fail) atomicMin(a.info, -1ll);
+    if (warp == 0) tmem_dealloc(taddr, 512);
+}
+
+}  // namespace
+
+size_t split_update_bytes(int nb, int bsz) {
+    const size_t rows = (size_t)(nb - 1) * bsz;
+    return rows * bsz * kPlanes + rows * sizeof(double);
+}
+
+hs_status launch_split_digits(hs_ctx ctx, const double* A, int k, void* ws, cudaStream_t s) {
+    const int nb = ctx->nb, bsz = ctx->bsz;
+    const int64_t cap = (int64_t)(nb - 1) * bsz, rows = (int64_t)(nb - 1 - k) * bsz;
+    int8_t* D = static_cast<int8_t*>(ws);
+    double* scale = reinterpret_cast<double*>(D + cap * bsz * kPlanes);
+    const double* P = A + (size_t)(block_id(k, k, nb) + 1) * bsz * bsz;
+    ctx->launches += 1;
+    if (bsz == 256)
+        digits_kernel<256><<<(unsigned)(rows / 8), 256, 0, s>>>(P, rows, D, scale);
+    else
+        digits_kernel<128><<<(unsigned)(rows / 8), 256, 0, s>>>(P, rows, D, scale);
+    HS_CHECK_LAUNCH("split_digits");
+    return HS_OK;
+}
+
+hs_status launch_split_update(hs_ctx ctx, double* A, int k, int colStart, int colEnd, void* ws, cudaStream_t s) {
+    const int nb = ctx->nb, bsz = ctx->bsz;
+    const int64_t cap = (int64_t)(nb - 1) * bsz;
+    int8_t* D = static_cast<int8_t*>(ws);
+    HS_CUDA(cudaFuncSetAttribute(split_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    SplitArgs a{};
+    a.A = A;
+    a.digits = D;
+    a.scale = reinterpret_cast<const double*>(D + cap * bsz * kPlanes);
+    a.k = k;
+    a.nb = nb;
+    a.bsz = bsz;
+    a.first_col = colStart;
+    a.m = nb - colStart;
+    a.triangle = colEnd - colStart > 1;
+    HS_REQUIRE(colEnd == nb || !a.triangle, "the trailing triangle or one column");
+    const int64_t blocks = a.triangle ? (int64_t)a.m * (a.m + 1) / 2 : a.m;
+    const int64_t per_block = (int64_t)(bsz / 128) * (bsz / 128);
+    a.items = blocks * per_block;
+    a.info = ctx->d_info;
+    const int64_t grid = (a.items + kPerCta - 1) / kPerCta;
+    HS_REQUIRE(grid < (1LL << 31), "trailing update too large for one launch");
+    const double n = bsz, cols = colEnd - colStart;
+    prof_begin(ctx, s, HS_KERNEL_UPDATE);
+    ctx->launches += 1;
+    split_update_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(a);
+    HS_CHECK_LAUNCH("split_update");
+    prof_end(ctx, s, HS_KERNEL_UPDATE, (blocks - cols) * 2.0 * n * n * n + cols * n * n * (n + 1.0),
+             (2.0 * blocks + a.m) * n * n * 8.0);
+    return HS_OK;
+}
+
+}  // namespace hs
