@@ -116,7 +116,7 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
     // twice a column.)
     const size_t bb = (size_t)bsz * bsz;
     // Large updates go to the INT8 tensor cores (if the digits' workspace can be had): from a
-    // tile an SM on for panels of 256 (a factor at N = 9973: 13.3 -> 9.3 ms), and eight for 128,
+    // tile an SM on for panels of 256 (a factor at N = 9973: 13.3 -> 8.8 ms), and eight for 128,
     // whose tiles do half the products for the same epilogue and find the chain longer.
     const size_t base = kSmallScratch + kDiagScratchBlocks * bb * sizeof(double);
     auto split_pays = [&](int64_t m) {

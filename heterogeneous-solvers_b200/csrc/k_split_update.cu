@@ -2,21 +2,22 @@
 //
 // The large trailing updates of the FP64 Cholesky (MatrixMatrixOperations.cpp:146-906) are
 // C <- C - P P^T with a panel P of one block column.  The FP64 tensor pipe bounds them at 64
-// multiply-adds a cycle and SM; the INT8 pipe does over a hundred times that.  Each row of the panel
-// is therefore scaled by a power of two to |t| <= 0.497 and written as seven balanced
+// multiply-adds a cycle and SM; the INT8 pipe does 8192.  Each row of the panel is therefore
+// scaled by a power of two to |t| <= 0.497 and written as seven balanced
 // base-256 digits, t = sum_i d_i 2^-8(i+1) with |error| <= 2^-57, and the product of two rows
 // is the sum over levels l = i + j of 2^-8l (digit plane i) x (digit plane j): exact INT32
 // sums in the tensor cores, levels 0..7 kept (34 plane products), carried into one 64-bit
-// integer, rounded to FP64 once and added to C.  (K. Ozaki, T. Ogita,
-// S. Oishi, S. M. Rump, "Error-free transformations of matrix multiplication by using fast
-// routines of matrix multiplication and its applications", 2012; H. Ootomo, K. Ozaki, R.
-// Yokota, "DGEMM on integer matrix multiplication unit", 2024.)
+// integer, rounded to FP64 once and added to C.  (K. Ozaki, T. Ogita, S. Oishi, S. M. Rump,
+// "Error-free transformations of matrix multiplication by using fast routines of matrix
+// multiplication and its applications", 2012; H. Ootomo, K. Ozaki, R. Yokota, "DGEMM on
+// integer matrix multiplication unit", 2024.)
 //
 // Error of one update, in units of the rows' scales: the digits' 2^-57 a factor, levels
 // past 7 at most 2^-64 a product and the last unit 2^-57; then a rounding of the product and
 // one of C.  The FP64 pipe's chain rounds 64 times at 2^-53 |C|.  Measured, max |A - L L^T| /
-// sqrt(a_ii a_jj) of a factor at N = 4800 (Wishart): 7.6e-15 -> 2.4e-15.  Scale_i scale_j <= 16 max|P_i| max|P_j| <= 16 sqrt(A_ii A_jj), so the
-// factor keeps the backward error bound of the plain form, relative to sqrt(A_ii A_jj).
+// sqrt(a_ii a_jj) of a factor at N = 4800 (Wishart): 7.6e-15 -> 2.4e-15.  Scale_i scale_j <=
+// 16 max|P_i| max|P_j| <= 16 sqrt(A_ii A_jj), so the factor keeps the plain form's backward
+// error bound relative to sqrt(A_ii A_jj).
 #include "hs_internal.cuh"
 #include "stream_common.cuh"
 #include "tc_common.cuh"
@@ -33,7 +34,7 @@ constexpr int kPlane = 128 * kKc;            // one plane of 128 rows of a stage
 constexpr int kOperand = kPlanes * kPlane;
 constexpr int kStage = 2 * kOperand, kStages = 2;  // 112 KB each
 constexpr int kSmem = 512 + kStages * kStage + 256 * 8 + 104;  // + the tile's scales, barriers
-constexpr int kEpi = 16, kThreads = 64 + 32 * kEpi;  // copy warp, MMA warp, epilogue warps
+constexpr int kEpi = 8, kThreads = 64 + 32 * kEpi;  // copy warp, MMA warp, epilogue warps
 constexpr int kPerCta = 4;     // tiles a CTA
 constexpr int kMinExp = -900;  // rows whose largest entry lies below 2^-900 keep that scale
 
@@ -96,6 +97,29 @@ __global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ 
 }
 
 // ------------------------------------------------------------------ update
+// Bounded waits that suspend the thread between tries: warps that poll take the shared-memory
+// port from the tensor core's operands.
+__device__ __forceinline__ bool suspended_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait(bar, parity)) {
+        if (*fail || clock64() - t0 > kWaitClk) {
+            *fail = 1;
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ bool suspended_wait_warp(uint64_t* bar, uint32_t parity, volatile int* fail) {
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        if (__any_sync(0xffffffffu, *fail || clock64() - t0 > kWaitClk)) {
+            *fail = 1;
+            return false;
+        }
+    }
+    return true;
+}
+
 struct SplitArgs {
     double* A;
     const int8_t* digits;
@@ -111,38 +135,44 @@ struct SplitArgs {
 // both K-major, N >> 3 in [17, 23), M >> 4 in [24, 29)
 constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
-__device__ __forceinline__ void umma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
+// the descriptors' low words; the rest is the same for every plane
+__device__ __forceinline__ void umma_i8(uint32_t d, uint32_t a, uint32_t b, uint32_t high, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(kIdesc), "r"(accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}\n" ::"r"(d),
+        "r"(a), "r"(b), "r"(high), "r"(kIdesc), "r"(accumulate)
         : "memory");
 }
 
-// The products of levels LEVEL + 3 .. LEVEL of one stage, highest first, as straight-line code with
-// descriptors at constant distances (in a loop that formed each descriptor a product took 130
-// cycles to issue; the tensor core takes 64).  wait / done: the four accumulators'
-// barriers, or null.
+// The products of levels LEVEL + 3 .. LEVEL of one stage, highest first, as straight-line code
+// with descriptors at constant distances, issued by one lane of a warp that walks the loop
+// together (a product takes the tensor core 35 ns; issued by a lone thread 53 ns, and
+// with descriptors formed in a loop 68 ns).  wait / done: the four accumulators' barriers, or
+// null.
 template <int LEVEL>
-__device__ __forceinline__ bool issue_levels(uint32_t taddr, uint64_t da, uint32_t accumulate, uint64_t* wait,
-                                             uint64_t* done, uint32_t parity, volatile int* fail) {
-    const uint64_t db = da + (kOperand >> 4);
+__device__ __forceinline__ bool issue_levels(uint32_t taddr, uint64_t desc, uint32_t accumulate, uint64_t* wait,
+                                             uint64_t* done, uint32_t parity, bool leader, volatile int* fail) {
+    const uint32_t da = (uint32_t)desc, db = da + (kOperand >> 4), high = (uint32_t)(desc >> 32);
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
         if (wait) {
-            if (!thread_wait(&wait[x], parity, fail)) return false;
+            if (!suspended_wait_warp(&wait[x], parity, fail)) return false;
             tc_fence_after();
         }
-        constexpr int kTop = kPlanes - 1;
-        const int level = LEVEL + 3 - x, first = level > kTop ? level - kTop : 0, last = level < kTop ? level : kTop;
+        if (leader) {
+            constexpr int kTop = kPlanes - 1;
+            const int level = LEVEL + 3 - x, first = level > kTop ? level - kTop : 0, last = level < kTop ? level : kTop;
 #pragma unroll
-        for (int i = first; i <= last; ++i)
+            for (int i = first; i <= last; ++i)
 #pragma unroll
-            for (int ks = 0; ks < kKc / 32; ++ks)
-                umma_i8(taddr + x * 128, da + ((i * kPlane + ks * 32) >> 4),
-                        db + (((level - i) * kPlane + ks * 32) >> 4), i > first || ks > 0 ? 1u : accumulate);
-        if (done) umma_commit(&done[x]);
+                for (int ks = 0; ks < kKc / 32; ++ks)
+                    umma_i8(taddr + x * 128, da + ((i * kPlane + ks * 32) >> 4),
+                            db + (((level - i) * kPlane + ks * 32) >> 4), high, i > first || ks > 0 ? 1u : accumulate);
+            if (done) umma_commit(&done[x]);
+        }
+        __syncwarp();
     }
     return true;
 }
@@ -156,7 +186,30 @@ __device__ __forceinline__ double to_double(int top, unsigned low) {
 }
 
 __device__ __forceinline__ void red_add(double* p, double v) {
-    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(p), "d"(v));
+}
+
+// C += the warp's 32 x 32 part; LOWER: entries with column <= row + diag only (what lies above
+// the diagonal stays as it was)
+template <bool LOWER>
+__device__ __forceinline__ void add_tile(double* C, int ldc, const double* row_scale, const double* col_scale,
+                                         const int (&top)[4][16], const unsigned (&low)[4][16], int gr, int t4, int diag) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+            const int r = 16 * (h >> 1) + 8 * o + gr;
+            double* p = C + (size_t)r * ldc + 2 * t4;
+            const double sr = -row_scale[r];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int z = 0; z < 2; ++z) {
+                    const int e = 4 * j + 2 * o + z, c = 32 * (h & 1) + 8 * j + z;
+                    const double v = to_double(top[h][e], low[h][e]) * sr * col_scale[c + 2 * t4];
+                    if (!LOWER || c + 2 * t4 <= r + diag) red_add(p + c, v);
+                }
+        }
 }
 
 // a tile: its entry (0, 0) in A, its rows' and columns' first rows in the panel, in 128s
@@ -187,11 +240,13 @@ __device__ __forceinline__ Tile decode(const SplitArgs& a, int64_t item) {
 // four accumulators of 128 columns, the whole of TMEM; in a pass's last K chunk the levels
 // are finished one by one and in the next pass's first chunk begun one by one, so that the
 // epilogue warps drain a level while the others are being computed.  C gets one add an
-// entry, without a load (loads of C waited behind the copies' queue: 4 us more a tile).
-// N = 64 would read shared memory 1.5 times as fast as it delivers; 128 columns take all of
-// it, and copies and adds contend with the operands (measured without them: 15 us a tile).
-// A tile of a 256-wide panel takes an SM 21 us (45 us on the FP64 pipe); the update of
-// 62 block columns of 256 2.15 -> 1.10 ms.
+// entry, without a load: a load waits behind the copies' queue (a tile took 24 to 38 us that
+// way), and the adds run at the L2's rate for FP64 (12 us a tile, beside the products).
+// N = 64 would read shared memory 1.5 times as fast as it delivers.  Pairs of SMs
+// (cta_group::2) and stages of half the depth were slower: their smaller copies take
+// longer than the products (11 and 10 us a tile against 7.5).
+// A tile of a 256-wide panel takes an SM 19.4 us (45 us on the FP64 pipe; 12 without the
+// adds); the update of 62 block columns of 256 2.15 -> 1.01 ms.
 __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) {
     extern __shared__ uint8_t raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 511) & ~(uintptr_t)511);
@@ -241,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
                     const uint32_t bytes = (pass ? kHighPlanes : kPlanes) * kPlane;
                     for (int kc = 0; kc < chunks; ++kc, ++g) {
                         const uint32_t s = g % kStages;
-                        if (g >= kStages && !thread_wait(&empty[s], (g / kStages - 1) & 1, fail)) {
+                        if (g >= kStages && !suspended_wait(&empty[s], (g / kStages - 1) & 1, fail)) {
                             ok = false;
                             break;
                         }
@@ -259,36 +314,37 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t g = 0, u = 0;
-            bool ok = true;
-            for (int it = 0; it < count && ok; ++it) {
-                if (tiles[it].skip) continue;
-                for (int pass = 0; pass < 2 && ok; ++pass, ++u) {
-                    for (int kc = 0; kc < chunks; ++kc, ++g) {
-                        const uint32_t s = g % kStages;
-                        if (!(ok = thread_wait(&full[s], (g / kStages) & 1, fail))) break;
-                        tc_fence_after();
-                        const uint64_t da = umma_desc_sw64(smem_u32(smem + s * kStage));
-                        uint64_t* wait = kc == 0 && u > 0 ? tempty : nullptr;
-                        uint64_t* done = kc == chunks - 1 ? tfull : nullptr;
-                        ok = pass == 0 ? issue_levels<kHighPlanes>(taddr, da, kc > 0, wait, done, (u - 1) & 1, fail)
-                                       : issue_levels<0>(taddr, da, kc > 0, wait, done, (u - 1) & 1, fail);
-                        if (!ok) break;
-                        umma_commit(&empty[s]);
-                    }
+        const bool leader = elect_one();  // the whole warp walks the loop, so that descriptors stay in uniform registers
+        uint32_t g = 0, u = 0;
+        bool ok = true;
+        for (int it = 0; it < count && ok; ++it) {
+            if (tiles[it].skip) continue;
+            for (int pass = 0; pass < 2 && ok; ++pass, ++u) {
+                for (int kc = 0; kc < chunks; ++kc, ++g) {
+                    const uint32_t s = g % kStages;
+                    if (!(ok = suspended_wait_warp(&full[s], (g / kStages) & 1, fail))) break;
+                    tc_fence_after();
+                    const uint64_t da = umma_desc_sw64(smem_u32(smem + s * kStage));
+                    uint64_t* wait = kc == 0 && u > 0 ? tempty : nullptr;
+                    uint64_t* done = kc == chunks - 1 ? tfull : nullptr;
+                    ok = pass == 0 ? issue_levels<kHighPlanes>(taddr, da, kc > 0, wait, done, (u - 1) & 1, leader, fail)
+                                   : issue_levels<0>(taddr, da, kc > 0, wait, done, (u - 1) & 1, leader, fail);
+                    if (!ok) break;
+                    if (leader) umma_commit(&empty[s]);
+                    __syncwarp();
                 }
             }
-            // TMEM is released only after every MMA issued here has completed
-            umma_commit(drained);
-            const long long t0 = clock64();
-            while (!mbar_test(drained, 0) && clock64() - t0 < kWaitClk) {}
         }
+        // TMEM is released only after every MMA issued here has completed
+        if (leader) umma_commit(drained);
+        __syncwarp();
+        const long long t0 = clock64();
+        while (!mbar_try_wait(drained, 0) && clock64() - t0 < kWaitClk) {}
     } else {
         // warp: rows 32 q .. +31 and 32 columns of the tile.  TMEM is read in 16 x 32 pieces
         // whose lane (g, t) holds rows g and g + 8, columns 8 j + 2 t and the next: an access to
         // C takes 64 bytes of each of eight rows (a row a lane: 32 lines an access).
-        const int q = warp & 3, col0 = ((warp - 2) >> 2) * 32, gr = lane >> 2, t4 = lane & 3;
+        const int q = warp & 3, col0 = ((warp - 2) >> 2) * 64, gr = lane >> 2, t4 = lane & 3;
         const uint32_t tcol = taddr + ((uint32_t)(q * 32) << 16) + col0;
         uint32_t u = 0;
         bool ok = true;
@@ -298,25 +354,25 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
             double* C = a.A + t.c + (int64_t)(32 * q) * a.bsz + col0;
             const int e = threadIdx.x - 64;
             const double sc = e < 256 ? a.scale[(int64_t)(e < 128 ? t.rows : t.cols) * 128 + (e & 127)] : 0.0;
-            asm volatile("bar.sync 1, 512;" ::: "memory");  // every warp has read the last tile's
+            asm volatile("bar.sync 1, 256;" ::: "memory");  // every warp has read the last tile's
             if (e < 256) scales[e] = sc;
-            asm volatile("bar.sync 1, 512;" ::: "memory");
+            asm volatile("bar.sync 1, 256;" ::: "memory");
             // The levels come lowest first and each is carried into the next, so that 32 bits do:
             // top = the sum so far in the last level's unit, low = the bytes below it (the
             // last one 2^-56; of levels 6 and 7 only the carry, rounded to nearest).
-            int top[2][16];  // [row half]
-            unsigned low[2][16];
+            int top[4][16];  // [row half, column half]
+            unsigned low[4][16];
 #pragma unroll
             for (int pass = 0; pass < 2; ++pass) {
 #pragma unroll
                 for (int x = 0; x < 4; ++x) {
-                    if (ok) ok = warp_wait(&tfull[x], (u + pass) & 1, fail);
+                    if (ok) ok = suspended_wait_warp(&tfull[x], (u + pass) & 1, fail);
                     if (!ok) continue;
                     tc_fence_after();
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
+                    for (int h = 0; h < 4; ++h) {
                         uint32_t v[16];
-                        tmem_ld_16x256b_x4(tcol + ((uint32_t)(16 * h) << 16) + x * 128, v);
+                        tmem_ld_16x256b_x4(tcol + ((uint32_t)(16 * (h >> 1)) << 16) + x * 128 + (h & 1) * 32, v);
                         tmem_ld_wait();
 #pragma unroll
                         for (int e = 0; e < 16; ++e) {
@@ -336,22 +392,10 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
             }
             if (!ok) continue;
             u += 2;
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int o = 0; o < 2; ++o) {  // rows g + 8 o of the half
-                    const int r = 16 * h + 8 * o + gr;
-                    double* p = C + (size_t)r * a.bsz + 2 * t4;
-                    const double sr = scales[32 * q + r];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int cc = 8 * j + 2 * t4;
-                        const double2 s2 = *reinterpret_cast<const double2*>(scales + 128 + col0 + cc);
-                        const int over = col0 + cc - 32 * q - r;  // > 0: above the diagonal, as it was
-                        if (!t.lower || over <= 0) red_add(p + 8 * j, -(to_double(top[h][4 * j + 2 * o], low[h][4 * j + 2 * o]) * sr) * s2.x);
-                        if (!t.lower || over < 0) red_add(p + 8 * j + 1, -(to_double(top[h][4 * j + 2 * o + 1], low[h][4 * j + 2 * o + 1]) * sr) * s2.y);
-                    }
-                }
+            if (t.lower)
+                add_tile<true>(C, a.bsz, scales + 32 * q, scales + 128 + col0, top, low, gr, t4, 32 * q - col0);
+            else
+                add_tile<false>(C, a.bsz, scales + 32 * q, scales + 128 + col0, top, low, gr, t4, 0);
         }
     }
     tc_fence_before();
