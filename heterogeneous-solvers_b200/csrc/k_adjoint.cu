@@ -24,21 +24,31 @@
 namespace hs {
 namespace {
 
-// 128 x 64 output tiles, 8 warps of 32 x 32, 3-stage ring: 128 registers and 90 KB of
-// shared memory, two CTAs an SM (one CTA's prologue / epilogue beside the other's MMAs)
-constexpr int BM = 128, BN = 64, BK = 16, STAGES = 3;
-constexpr int WM = 32, WN = 32, kWarpsN = BN / WN;
+// Output tiles of BM x BN by warps of WM x WN, 3-stage ring.
+// Large: 128 x 64, 8 warps of 32 x 32: 128 registers and 90 KB of shared memory, two CTAs an
+// SM (one CTA's prologue / epilogue beside the other's MMAs).
+// Small: 32 x 32, 4 warps of 16 x 16, 30 KB: for products with too few large tiles for the SMs.
+constexpr int BK = 16, STAGES = 3;
 constexpr int SPAD = 20;        // row pitch (doubles) of K-contiguous operand rows
-// M- / N-contiguous rows are read by lane (g, t) at row 4 kk + t, column 8 i + g: a pitch
-// of 4 (mod 16) doubles puts the 16 lanes of each half-warp's 8-byte loads on 16
-// different 8-byte bank pairs (a pitch of 8 mod 16 would put t and t + 2 on the same pair)
-constexpr int LDTA = BM + 4;    // row pitch (doubles) of M-contiguous A rows
-constexpr int LDTB = BN + 4;    // row pitch (doubles) of N-contiguous B rows
-constexpr int kStageA = BM * SPAD;  // >= BK * LDTA
-constexpr int kStageB = BN * SPAD;  // >= BK * LDTB
-constexpr int kStage = kStageA + kStageB;
-constexpr int kChainSmem = STAGES * kStage * (int)sizeof(double);  // 90 KB
-static_assert(BK * LDTA <= kStageA && BK * LDTB <= kStageB, "stage layout");
+template <int BM_, int BN_, int WM_, int WN_>
+struct ChainTile {
+    static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_;
+    static constexpr int kWarpsN = BN / WN, kThreads = 32 * (BM / WM) * kWarpsN;
+    static constexpr int kMi = WM / 8, kNi = WN / 8;
+    // M- / N-contiguous rows are read by lane (g, t) at row 4 kk + t, column 8 i + g: a pitch
+    // of 4 (mod 16) doubles puts the 16 lanes of each half-warp's 8-byte loads on 16
+    // different 8-byte bank pairs (a pitch of 8 mod 16 would put t and t + 2 on the same pair)
+    static constexpr int LDTA = BM + 4;    // row pitch (doubles) of M-contiguous A rows
+    static constexpr int LDTB = BN + 4;    // row pitch (doubles) of N-contiguous B rows
+    static constexpr int kStageA = BM * SPAD;  // >= BK * LDTA
+    static constexpr int kStageB = BN * SPAD;  // >= BK * LDTB
+    static constexpr int kStage = kStageA + kStageB;
+    static constexpr int kSmem = STAGES * kStage * (int)sizeof(double);
+    static_assert(BK * LDTA <= kStageA && BK * LDTB <= kStageB, "stage layout");
+    static_assert(BM * 8 % kThreads == 0 && BN * 8 % kThreads == 0, "16-byte copies a stage");
+};
+using ChainLarge = ChainTile<128, 64, 32, 32>;
+using ChainSmall = ChainTile<32, 32, 16, 16>;
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -84,33 +94,38 @@ __device__ __forceinline__ Elem chain_elem(const ChainArgs& a, int item, int64_t
     return e;
 }
 
-// One K slab of the warp's 32 x 32 tile, for one operand orientation (TA: A staged
+// One K slab of the warp's tile, for one operand orientation (TA: A staged
 // M-contiguous, TB: B staged K-contiguous), as straight-line code per orientation
-template <bool TA, bool TB>
-__device__ __forceinline__ void slab_mma(double (&acc)[4][4][2], const double* __restrict__ As,
+template <typename T, bool TA, bool TB>
+__device__ __forceinline__ void slab_mma(double (&acc)[T::kMi][T::kNi][2], const double* __restrict__ As,
                                          const double* __restrict__ Bs, int wm, int wn, int g, int t) {
 #pragma unroll
     for (int kk = 0; kk < BK / 4; ++kk) {
-        double av[4], bv[4];
+        double av[T::kMi], bv[T::kNi];
 #pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
-            av[mi] = TA ? As[(kk * 4 + t) * LDTA + wm * WM + mi * 8 + g] : As[(wm * WM + mi * 8 + g) * SPAD + kk * 4 + t];
+        for (int mi = 0; mi < T::kMi; ++mi)
+            av[mi] = TA ? As[(kk * 4 + t) * T::LDTA + wm * T::WM + mi * 8 + g]
+                        : As[(wm * T::WM + mi * 8 + g) * SPAD + kk * 4 + t];
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-            bv[ni] = TB ? Bs[(wn * WN + ni * 8 + g) * SPAD + kk * 4 + t] : Bs[(kk * 4 + t) * LDTB + wn * WN + ni * 8 + g];
+        for (int ni = 0; ni < T::kNi; ++ni)
+            bv[ni] = TB ? Bs[(wn * T::WN + ni * 8 + g) * SPAD + kk * 4 + t]
+                        : Bs[(kk * 4 + t) * T::LDTB + wn * T::WN + ni * 8 + g];
 #pragma unroll
-        for (int mi = 0; mi < 4; ++mi)
+        for (int mi = 0; mi < T::kMi; ++mi)
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni) dmma884(acc[mi][ni], av[mi], bv[ni]);
+            for (int ni = 0; ni < T::kNi; ++ni) dmma884(acc[mi][ni], av[mi], bv[ni]);
     }
 }
 
-// One CTA = one 128 x 64 tile of one output block, accumulating the chain
-// elements [q0, q1) of its item; 8 warps of 32 x 32, K streamed in 16-wide
+// One CTA = one tile of one output block, accumulating the chain
+// elements [q0, q1) of its item; K streamed in 16-wide
 // slabs through a 3-stage cp.async ring.  Operands that enter transposed are
 // staged with the M (or N) index contiguous, the others with K contiguous.
-__global__ void __launch_bounds__(256, 2) chain_dmma_kernel(ChainArgs a) {
+template <typename T, int CTAS>
+__global__ void __launch_bounds__(T::kThreads, CTAS) chain_dmma_kernel(ChainArgs a) {
     extern __shared__ __align__(16) double smem[];
+    constexpr int BM = T::BM, BN = T::BN, WM = T::WM, WN = T::WN, LDTA = T::LDTA, LDTB = T::LDTB;
+    constexpr int kStage = T::kStage, kStageA = T::kStageA, NT = T::kThreads;
     const int tpm = a.bsz / BM, tpn = a.bsz / BN;
     const int64_t idx = blockIdx.x;
     const int split = (int)(idx % a.splits);
@@ -126,14 +141,14 @@ __global__ void __launch_bounds__(256, 2) chain_dmma_kernel(ChainArgs a) {
     const int bsz = a.bsz;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = warp / kWarpsN, wn = warp % kWarpsN;
+    const int wm = warp / T::kWarpsN, wn = warp % T::kWarpsN;
     const int g = lane >> 2, t = lane & 3;
 
-    double acc[4][4][2];
+    double acc[T::kMi][T::kNi][2];
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
+    for (int mi = 0; mi < T::kMi; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+        for (int ni = 0; ni < T::kNi; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
 
     auto load_stage = [&](int stage, int kt) {
         const Elem e = chain_elem(a, item, q0 + (kt >> lg));
@@ -141,23 +156,23 @@ __global__ void __launch_bounds__(256, 2) chain_dmma_kernel(ChainArgs a) {
         double* As = smem + stage * kStage;
         double* Bs = As + kStageA;
 #pragma unroll
-        for (int qq = 0; qq < 4; ++qq) {  // A: 1024 16-byte copies
-            const int x = tid + 256 * qq;
-            if (!e.ta) {  // A_op[m][k] = A[ti*128+m][kc+k]: rows m, K contiguous
+        for (int qq = 0; qq < BM * 8 / NT; ++qq) {  // A: 16-byte copies
+            const int x = tid + NT * qq;
+            if (!e.ta) {  // A_op[m][k] = A[ti*BM+m][kc+k]: rows m, K contiguous
                 const int row = x >> 3, ch = x & 7;
                 cp_async16(As + row * SPAD + ch * 2, e.A + (size_t)(ti * BM + row) * bsz + kc + ch * 2);
-            } else {      // A_op[m][k] = A[kc+k][ti*128+m]: rows k, M contiguous
-                const int row = x >> 6, ch = x & 63;
+            } else {      // A_op[m][k] = A[kc+k][ti*BM+m]: rows k, M contiguous
+                const int row = x / (BM / 2), ch = x % (BM / 2);
                 cp_async16(As + row * LDTA + ch * 2, e.A + (size_t)(kc + row) * bsz + ti * BM + ch * 2);
             }
         }
 #pragma unroll
-        for (int qq = 0; qq < 2; ++qq) {  // B: 512 16-byte copies
-            const int x = tid + 256 * qq;
-            if (!e.tb) {  // B_op[k][n] = B[kc+k][tj*64+n]: rows k, N contiguous
-                const int row = x >> 5, ch = x & 31;
+        for (int qq = 0; qq < BN * 8 / NT; ++qq) {  // B: 16-byte copies
+            const int x = tid + NT * qq;
+            if (!e.tb) {  // B_op[k][n] = B[kc+k][tj*BN+n]: rows k, N contiguous
+                const int row = x / (BN / 2), ch = x % (BN / 2);
                 cp_async16(Bs + row * LDTB + ch * 2, e.B + (size_t)(kc + row) * bsz + tj * BN + ch * 2);
-            } else {      // B_op[k][n] = B[tj*64+n][kc+k]: rows n, K contiguous
+            } else {      // B_op[k][n] = B[tj*BN+n][kc+k]: rows n, K contiguous
                 const int row = x >> 3, ch = x & 7;
                 cp_async16(Bs + row * SPAD + ch * 2, e.B + (size_t)(tj * BN + row) * bsz + kc + ch * 2);
             }
@@ -184,13 +199,13 @@ __global__ void __launch_bounds__(256, 2) chain_dmma_kernel(ChainArgs a) {
         const double* As = smem + st * kStage;
         const double* Bs = As + kStageA;
         if (!eta && !etb)
-            slab_mma<false, false>(acc, As, Bs, wm, wn, g, t);
+            slab_mma<T, false, false>(acc, As, Bs, wm, wn, g, t);
         else if (eta && !etb)
-            slab_mma<true, false>(acc, As, Bs, wm, wn, g, t);
+            slab_mma<T, true, false>(acc, As, Bs, wm, wn, g, t);
         else if (!eta)
-            slab_mma<false, true>(acc, As, Bs, wm, wn, g, t);
+            slab_mma<T, false, true>(acc, As, Bs, wm, wn, g, t);
         else
-            slab_mma<true, true>(acc, As, Bs, wm, wn, g, t);
+            slab_mma<T, true, true>(acc, As, Bs, wm, wn, g, t);
     }
     cp_async_wait<0>();
 
@@ -208,9 +223,9 @@ __global__ void __launch_bounds__(256, 2) chain_dmma_kernel(ChainArgs a) {
     }
     const double alpha = a.alpha;
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
+    for (int mi = 0; mi < T::kMi; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
+        for (int ni = 0; ni < T::kNi; ++ni) {
             const int r = ti * BM + wm * WM + mi * 8 + g;
             const int c = tj * BN + wn * WN + ni * 8 + 2 * t;
             double* p = C + (size_t)r * bsz + c;
@@ -290,7 +305,7 @@ __global__ void sym_tril_half_kernel(const double* __restrict__ G, double* __res
 // minimises the time model waves(base s) x ceil(chain / s) chain steps, plus the
 // fixed-order reduction of the s partial blocks of each item (~0.1 chain step a
 // partial tile a CTA slot), so that the last wave is not left mostly empty.
-int pick_splits(int64_t base_ctas, int64_t chain, int items, int64_t partial_blocks, int sms) {
+int pick_splits(int64_t base_ctas, int64_t chain, int items, int64_t partial_blocks, int sms, double* cost_out) {
     int64_t best = 1;
     double best_cost = 1e300;
     const int64_t smax = chain < 64 ? chain : 64;
@@ -304,8 +319,15 @@ int pick_splits(int64_t base_ctas, int64_t chain, int items, int64_t partial_blo
             best = s;
         }
     }
+    *cost_out = best_cost;
     return (int)best;
 }
+
+// N = 2000 (blocks of 256): 1.91 -> 1.69 ms a gradient, 4000: 5.1 -> 4.75; small tiles alone
+// 149 ms at 16384 against 136
+constexpr double kSmallStep = 0.35;
+constexpr auto chain_large = chain_dmma_kernel<ChainLarge, 2>;
+constexpr auto chain_small = chain_dmma_kernel<ChainSmall, 4>;
 
 bool g_chain_attr[64] = {};
 
@@ -313,7 +335,7 @@ hs_status chain_attrs() {
     int dev = 0;
     HS_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && g_chain_attr[dev]) return HS_OK;
-    HS_CUDA(cudaFuncSetAttribute(chain_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmem));
+    HS_CUDA(cudaFuncSetAttribute(chain_large, cudaFuncAttributeMaxDynamicSharedMemorySize, ChainLarge::kSmem));
     if (dev >= 0 && dev < 64) g_chain_attr[dev] = true;
     return HS_OK;
 }
@@ -326,15 +348,32 @@ hs_status launch_chain(hs_ctx ctx, ChainArgs a, double* partial, int64_t partial
     HS_REQUIRE(a.bsz == 128 || a.bsz == 256, "the tensor-core adjoint supports matrixBlockSize 128 or 256");
     if (a.items <= 0 || a.chain <= 0) return HS_OK;
     HS_REQUIRE(a.chain * (a.bsz / BK) < (1LL << 31), "product chain too long");
-    const int64_t base = (int64_t)a.items * (a.bsz / BM) * (a.bsz / BN);
-    a.splits = (partial && a.allow_split) ? pick_splits(base, a.chain, a.items, partial_blocks, 2 * ctx->num_sms) : 1;
+    using CL = ChainLarge;
+    using CS = ChainSmall;
+    // Both tiles' times by the model of pick_splits, in large steps: four small tiles an SM
+    // take kSmallStep of what two large ones do.
+    const bool split = partial && a.allow_split;
+    int64_t base = (int64_t)a.items * (a.bsz / CL::BM) * (a.bsz / CL::BN);
+    const int64_t base_small = (int64_t)a.items * (a.bsz / CS::BM) * (a.bsz / CS::BN);
+    double cost, cost_small;
+    const int64_t room = split ? partial_blocks : 0;
+    a.splits = pick_splits(base, a.chain, a.items, room, 2 * ctx->num_sms, &cost);
+    const int splits_small = pick_splits(base_small, a.chain, a.items, room, 4 * ctx->num_sms, &cost_small);
+    const bool small = kSmallStep * cost_small < cost;
+    if (small) {
+        a.splits = splits_small;
+        base = base_small;
+    }
     a.partial = partial;
     const int64_t grid = base * a.splits;
     HS_REQUIRE(grid < (1LL << 31), "too many tiles");
     const double n3 = (double)a.bsz * a.bsz * a.bsz;
     prof_begin(ctx, s, HS_KERNEL_ADJOINT);
     ctx->launches += 1;
-    chain_dmma_kernel<<<(unsigned)grid, 256, kChainSmem, s>>>(a);
+    if (small)
+        chain_small<<<(unsigned)grid, CS::kThreads, CS::kSmem, s>>>(a);
+    else
+        chain_large<<<(unsigned)grid, CL::kThreads, CL::kSmem, s>>>(a);
     HS_CHECK_LAUNCH("chain_dmma_kernel");
     prof_end(ctx, s, HS_KERNEL_ADJOINT, 2.0 * n3 * (double)a.chain * a.items,
              8.0 * (double)a.bsz * a.bsz * (2.0 * a.chain * a.items + 2.0 * a.items));

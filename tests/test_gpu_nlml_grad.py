@@ -5,6 +5,7 @@ from pathlib import Path
 
 import numpy as np
 import pytest
+import torch
 
 sys.path.insert(0, str(Path(__file__).resolve().parents[1] / "oracle"))
 import gp_dense as g  # noqa: E402
@@ -30,3 +31,26 @@ def test_gradient_at_block_edges(hs, ctx, N, bsz, d, ard):
     tol = 64 * 2.0 ** -52 * (1.3 * N / sn2 + 1)
     assert abs(nlml - nlml_ref) <= tol * (abs(nlml_ref) + N)
     assert np.max(np.abs(grad - grad_ref)) <= tol * (np.max(np.abs(grad_ref)) + N / 2)
+
+
+def test_gradient_with_large_tiles(hs, ctx):
+    """Enough block rows that the products take large tiles and whole waves; the reference is
+    the dense inverse in FP64 on the device, with the bound of the test above."""
+    N, bsz, d, sf2, sn2 = 10100, 256, 3, 1.3, 2e-2
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N)
+    X = torch.rand((N, d), dtype=torch.float64, device="cuda", generator=g)
+    y = torch.sin(X.sum(1)) + 0.1 * torch.randn(N, dtype=torch.float64, device="cuda", generator=g)
+    ell = torch.tensor([0.6, 0.9, 1.4], dtype=torch.float64, device="cuda")
+    theta = np.log(np.array([0.6, 0.9, 1.4, sf2, sn2]))
+    ctx.set_problem(N, bsz)
+    _, grad, _ = hs.gp_nlml_grad(ctx, X, y, theta)
+    D = [((X[:, k, None] - X[None, :, k]) / ell[k]).square() for k in range(d)]
+    Kf = sf2 * torch.exp(-0.5 * sum(D))
+    L = torch.linalg.cholesky(Kf + sn2 * torch.eye(N, dtype=torch.float64, device="cuda"))
+    alpha = torch.cholesky_solve(y[:, None], L)
+    W = torch.cholesky_inverse(L) - alpha @ alpha.T
+    ref = [0.5 * (W * Kf * Dk).sum().item() for Dk in D]
+    ref += [0.5 * (W * Kf).sum().item(), 0.5 * sn2 * W.diagonal().sum().item()]
+    tol = 64 * 2.0 ** -52 * (sf2 * N / sn2 + 1)
+    assert np.max(np.abs(grad - ref)) <= tol * (np.max(np.abs(ref)) + N / 2)
