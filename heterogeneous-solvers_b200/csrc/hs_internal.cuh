@@ -213,12 +213,11 @@ hs_status launch_update(hs_ctx ctx, double* A, int blockID, int blockRow, int sy
 // (SYRK on their diagonal blocks, GEMM below them)
 hs_status launch_update_cols(hs_ctx ctx, double* A, int blockID, int blockRow, int colStart, int colEnd,
                              cudaStream_t s);
-// the same for the columns [colStart, nb) or one column on the INT8 tensor cores
-// (k_split_update.cu): first the digits of panel k, then its update, on one stream.  ws:
-// split_update_bytes, 256-byte aligned; a wait that ran out: -1 in d_info
-size_t split_update_bytes(int nb, int bsz);
-hs_status launch_split_digits(hs_ctx ctx, const double* A, int k, void* ws, cudaStream_t s);
-hs_status launch_split_update(hs_ctx ctx, double* A, int k, int colStart, int colEnd, void* ws, cudaStream_t s);
+// the update of the columns [colStart, nb) by the panels k .. k + panels - 1 (one or two,
+// colStart past them) on the INT8 tensor cores (k_split_update.cu).  ws: split_update_bytes,
+// 256-byte aligned; a wait that ran out: -1 in d_info
+size_t split_update_bytes(int nb, int bsz, int panels);
+hs_status launch_split_update(hs_ctx ctx, double* A, int k, int panels, int colStart, void* ws, cudaStream_t s);
 // one diagonal block of bsz 128 or 256 (k_diag.cu): L and its inverse in one launch
 struct DiagFactor {
     const double* in64 = nullptr;  // the block, or

@@ -115,20 +115,22 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
     // lookahead.  (With the column update on the caller's stream, the chain crossed streams
     // twice a column.)
     const size_t bb = (size_t)bsz * bsz;
-    // Large updates go to the INT8 tensor cores (if the digits' workspace can be had): from a
-    // tile an SM on for panels of 256 (a factor at N = 9973: 13.3 -> 8.8 ms), and eight for 128,
-    // whose tiles do half the products for the same epilogue and find the chain longer.
+    // Large updates go to the INT8 tensor cores (if the digits' workspace can be had).  Panels
+    // of 256 one by one from a tile an SM on (a factor at N = 9973: 13.3 -> 8.6 ms).  Two panels
+    // at once halve the adds to C for more work on the chain: from two tiles an SM for
+    // panels of 128 (N = 9300: 9.9 -> 7.5 ms; one by one these gain nothing below eight), from eight
+    // for 256 (N = 32768: 221 -> 189 ms; at N = 6000 3.30 ms and 3.84 with pairs from one on).
     const size_t base = kSmallScratch + kDiagScratchBlocks * bb * sizeof(double);
-    auto split_pays = [&](int64_t m) {
-        return m * (m + 1) / 2 * (bsz / 128) * (bsz / 128) >= (bsz == 256 ? 1 : 8) * ctx->num_sms;
-    };
-    bool split = split_pays(nb - 2);
+    auto tiles = [&](int64_t m) { return m > 0 ? m * (m + 1) / 2 * (bsz / 128) * (bsz / 128) : 0; };
+    auto split_pays = [&](int64_t m) { return bsz == 256 && tiles(m) >= ctx->num_sms; };
+    auto pairs_pay = [&](int64_t m) { return tiles(m) >= (bsz == 256 ? 8 : 2) * ctx->num_sms; };
+    int split = pairs_pay(nb - 4) ? 2 : split_pays(nb - 2) ? 1 : 0;  // panels the workspace holds
     hs_status st = HS_OK;
-    if (split && ensure_scratch(ctx, base + split_update_bytes(nb, bsz)) != HS_OK) {
+    for (; split > 0; --split) {
+        if (ensure_scratch(ctx, base + split_update_bytes(nb, bsz, split)) == HS_OK) break;
         cudaGetLastError();
-        split = false;
     }
-    if (!split) st = ensure_scratch(ctx, base);
+    if (split == 0) st = ensure_scratch(ctx, base);
     if (st != HS_OK) return st;
     char* digits = static_cast<char*>(ctx->scratch) + base;
     auto diag = [&](int k, cudaStream_t q) -> hs_status {
@@ -148,7 +150,23 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
     HS_CUDA(cudaEventRecord(ctx->ev_a, s));
     HS_CUDA(cudaStreamWaitEvent(c, ctx->ev_a, 0));
     if ((st = diag(0, c)) != HS_OK) return st;
-    for (int k = 0; k + 1 < nb; ++k) {
+    int k = 0;
+    for (; split == 2 && pairs_pay(nb - k - 4); k += 2) {
+        // panels k and k + 1: the chain brings columns k + 1 .. k + 3 up to date, the update of
+        // columns k + 4 on runs beside it
+        const int first = diag_id(k), second = diag_id(k + 1);
+        if ((st = launch_update_cols(ctx, A, first, k, k + 1, k + 2, c)) != HS_OK) return st;
+        if ((st = diag(k + 1, c)) != HS_OK) return st;
+        HS_CUDA(cudaEventRecord(ctx->ev_a, c));
+        HS_CUDA(cudaStreamWaitEvent(s, ctx->ev_a, 0));
+        if (k > 0) HS_CUDA(cudaStreamWaitEvent(c, ctx->ev_b, 0));  // columns k + 2 and k + 3 have panels 0 .. k - 1
+        if ((st = launch_split_update(ctx, A, k, 2, k + 4, digits, s)) != HS_OK) return st;
+        HS_CUDA(cudaEventRecord(ctx->ev_b, s));
+        if ((st = launch_update_cols(ctx, A, first, k, k + 2, k + 4, c)) != HS_OK) return st;
+        if ((st = launch_update_cols(ctx, A, second, k + 1, k + 2, k + 4, c)) != HS_OK) return st;
+        if ((st = diag(k + 2, c)) != HS_OK) return st;
+    }
+    for (; k + 1 < nb; ++k) {
         const int blockID = diag_id(k);
         const int64_t m = nb - k - 2;  // block columns of the rest of panel k's update
         // A diagonal block's CTAs need whole SMs, and beside an update that fills the chip
@@ -170,9 +188,8 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
             HS_CUDA(cudaStreamWaitEvent(s, ctx->ev_a, 0));
         }
         if (m > 0) {
-            if (split && split_pays(m)) {
-                if ((st = launch_split_digits(ctx, A, k, digits, s)) != HS_OK) return st;
-                st = launch_split_update(ctx, A, k, k + 2, nb, digits, s);
+            if (split > 0 && split_pays(m)) {
+                st = launch_split_update(ctx, A, k, 1, k + 2, digits, s);
             } else {
                 st = launch_update_cols(ctx, A, blockID, k, k + 2, nb, s);
             }

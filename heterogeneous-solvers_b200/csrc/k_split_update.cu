@@ -1,7 +1,7 @@
 // k_split_update.cu — the FP64 trailing update on the tensor cores' INT8 path.
 //
 // The large trailing updates of the FP64 Cholesky (MatrixMatrixOperations.cpp:146-906) are
-// C <- C - P P^T with a panel P of one block column.  The FP64 tensor pipe bounds them at 64
+// C <- C - P P^T with a panel P of one block column, or of two at once.  The FP64 tensor pipe bounds them at 64
 // multiply-adds a cycle and SM; the INT8 pipe does 8192.  Each row of the panel is therefore
 // scaled by a power of two to |t| <= 0.497 and written as seven balanced
 // base-256 digits, t = sum_i d_i 2^-8(i+1) with |error| <= 2^-57, and the product of two rows
@@ -44,18 +44,20 @@ constexpr int kMinExp = -900;  // rows whose largest entry lies below 2^-900 kee
 // 64-byte swizzle (16-byte unit u of row r at u ^ (r / 2 % 4)), so that an operand's stage is
 // one contiguous copy.  A row that holds an infinity or NaN gets the scale NaN (and zero
 // digits), so that what it updates becomes NaN.
-template <int BSZ>
-__global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ P, int64_t rows, int8_t* __restrict__ D,
-                                                     double* __restrict__ scale) {
-    constexpr int E = BSZ / 32;  // entries a lane
+// K entries a row: of one panel (P1 unused) or half of them of each of two.
+template <int K>
+__global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ P0, const double* __restrict__ P1, int bsz,
+                                                     int64_t rows, int8_t* __restrict__ D, double* __restrict__ scale) {
+    constexpr int E = K / 32;  // entries a lane
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
+    const double* src = (lane * E < bsz ? P0 : P1) + row * bsz + lane * E % bsz;
     double v[E];
     long long m = 0;
 #pragma unroll
     for (int q = 0; q < E / 2; ++q) {
-        const double2 x = *reinterpret_cast<const double2*>(P + row * BSZ + lane * E + 2 * q);
+        const double2 x = *reinterpret_cast<const double2*>(src + 2 * q);
         v[2 * q] = x.x;
         v[2 * q + 1] = x.y;
     }
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ 
         u[q] = ((unsigned long long)(t + 0x0080808080808080ll)) ^ 0x0080808080808080ull;
     }
     const int r = (int)(row & 127), chunk = lane * E / kKc, byte = lane * E % kKc;
-    int8_t* out = D + ((row >> 7) * (BSZ / kKc) + chunk) * kOperand + r * kKc +
+    int8_t* out = D + ((row >> 7) * (K / kKc) + chunk) * kOperand + r * kKc +
                   (((byte >> 4) ^ (r >> 1 & 3)) << 4) + (byte & 15);
 #pragma unroll
     for (int i = 0; i < kPlanes; ++i) {
@@ -86,10 +88,10 @@ __global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ 
             w[q] = (unsigned)(u[4 * q] >> sh & 0xff) | (unsigned)(u[4 * q + 1] >> sh & 0xff) << 8 |
                    (unsigned)(u[4 * q + 2] >> sh & 0xff) << 16 | (unsigned)(u[4 * q + 3] >> sh & 0xff) << 24;
         int8_t* dst = out + i * kPlane;
-        if constexpr (E == 8)
-            *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+        if constexpr (E == 16)
+            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
         else
-            *reinterpret_cast<unsigned*>(dst) = w[0];
+            *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
     }
     // two rows' scales together turn units of 2^-56 into the product
     if (lane == 0)
@@ -123,10 +125,10 @@ __device__ __forceinline__ bool suspended_wait_warp(uint64_t* bar, uint32_t pari
 struct SplitArgs {
     double* A;
     const int8_t* digits;
-    const double* scale;  // of the panel's rows, from the block below the diagonal on
-    int k, nb, bsz;
-    int first_col, m;  // trailing block columns [first_col, first_col + m), one column if !triangle
-    int triangle;
+    const double* scale;  // of the panels' rows, from block row row0 on
+    int row0, depth;      // depth: columns of the panels, 256 or 512
+    int nb, bsz;
+    int first_col, m;  // the trailing triangle of m block columns
     int64_t items;     // 128 x 128 tiles
     long long* info;
 };
@@ -222,14 +224,14 @@ __device__ __forceinline__ Tile decode(const SplitArgs& a, int64_t item) {
     const int side = a.bsz >> 7, lg = a.bsz == 256 ? 2 : 0;
     const int64_t p = item >> lg;
     const int e = (int)item & ((1 << lg) - 1), ti = e >> (lg >> 1), tj = e & (side - 1);
-    int rr = (int)p, cc = 0;
-    if (a.triangle) grouped_pair(p, a.m, &rr, &cc);
+    int rr, cc;
+    grouped_pair(p, a.m, &rr, &cc);
     rr += a.first_col;
     cc += a.first_col;
     Tile t;
     t.c = (block_id(rr, cc, a.nb) * a.bsz + ti * 128) * a.bsz + tj * 128;
-    t.rows = (rr - a.k - 1) * side + ti;
-    t.cols = (cc - a.k - 1) * side + tj;
+    t.rows = (rr - a.row0) * side + ti;
+    t.cols = (cc - a.row0) * side + tj;
     t.skip = t.rows < t.cols;
     t.lower = t.rows == t.cols;
     return t;
@@ -246,7 +248,9 @@ __device__ __forceinline__ Tile decode(const SplitArgs& a, int64_t item) {
 // (cta_group::2) and stages of half the depth were slower: their smaller copies take
 // longer than the products (11 and 10 us a tile against 7.5).
 // A tile of a 256-wide panel takes an SM 19.4 us (45 us on the FP64 pipe; 12 without the
-// adds); the update of 62 block columns of 256 2.15 -> 1.01 ms.
+// adds); the update of 62 block columns of 256 2.15 -> 1.01 ms.  Two panels at once do twice
+// the products for the same adds: the top level's sums then just fit (512 x 127^2 x 256
+// < 2^31).
 __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) {
     extern __shared__ uint8_t raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 511) & ~(uintptr_t)511);
@@ -281,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
     tc_fence_after();
     const uint32_t taddr = *slot;
     const int count = (int)min((int64_t)kPerCta, a.items - (int64_t)blockIdx.x * kPerCta);
-    const int chunks = a.bsz / kKc;
+    const int chunks = a.depth / kKc;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -406,55 +410,48 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
 
 }  // namespace
 
-size_t split_update_bytes(int nb, int bsz) {
-    const size_t rows = (size_t)(nb - 1) * bsz;
-    return rows * bsz * kPlanes + rows * sizeof(double);
+size_t split_update_bytes(int nb, int bsz, int panels) {
+    const size_t rows = (size_t)(nb - panels) * bsz;
+    return rows * panels * bsz * kPlanes + rows * sizeof(double);
 }
 
-hs_status launch_split_digits(hs_ctx ctx, const double* A, int k, void* ws, cudaStream_t s) {
+hs_status launch_split_update(hs_ctx ctx, double* A, int k, int panels, int colStart, void* ws, cudaStream_t s) {
     const int nb = ctx->nb, bsz = ctx->bsz;
-    const int64_t cap = (int64_t)(nb - 1) * bsz, rows = (int64_t)(nb - 1 - k) * bsz;
-    int8_t* D = static_cast<int8_t*>(ws);
-    double* scale = reinterpret_cast<double*>(D + cap * bsz * kPlanes);
-    const double* P = A + (size_t)(block_id(k, k, nb) + 1) * bsz * bsz;
-    ctx->launches += 1;
-    if (bsz == 256)
-        digits_kernel<256><<<(unsigned)(rows / 8), 256, 0, s>>>(P, rows, D, scale);
-    else
-        digits_kernel<128><<<(unsigned)(rows / 8), 256, 0, s>>>(P, rows, D, scale);
-    HS_CHECK_LAUNCH("split_digits");
-    return HS_OK;
-}
-
-hs_status launch_split_update(hs_ctx ctx, double* A, int k, int colStart, int colEnd, void* ws, cudaStream_t s) {
-    const int nb = ctx->nb, bsz = ctx->bsz;
-    const int64_t cap = (int64_t)(nb - 1) * bsz;
-    int8_t* D = static_cast<int8_t*>(ws);
-    HS_CUDA(cudaFuncSetAttribute(split_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    const size_t bb = (size_t)bsz * bsz;
     SplitArgs a{};
+    a.row0 = k + panels;
+    a.depth = panels * bsz;
+    HS_REQUIRE(a.depth == 256 || a.depth == 512, "one or two panels of 256, or two of 128");
+    const int64_t rows = (int64_t)(nb - a.row0) * bsz;
+    int8_t* D = static_cast<int8_t*>(ws);
+    double* scale = reinterpret_cast<double*>(D + rows * a.depth * kPlanes);
+    const double* P0 = A + (size_t)block_id(a.row0, k, nb) * bb;
+    const double* P1 = panels == 2 ? A + (size_t)block_id(a.row0, k + 1, nb) * bb : P0;
+    HS_CUDA(cudaFuncSetAttribute(split_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    prof_begin(ctx, s, HS_KERNEL_UPDATE);
+    ctx->launches += 2;
+    if (a.depth == 512)
+        digits_kernel<512><<<(unsigned)(rows / 8), 256, 0, s>>>(P0, P1, bsz, rows, D, scale);
+    else
+        digits_kernel<256><<<(unsigned)(rows / 8), 256, 0, s>>>(P0, P1, bsz, rows, D, scale);
+    HS_CHECK_LAUNCH("split_digits");
     a.A = A;
     a.digits = D;
-    a.scale = reinterpret_cast<const double*>(D + cap * bsz * kPlanes);
-    a.k = k;
+    a.scale = scale;
     a.nb = nb;
     a.bsz = bsz;
     a.first_col = colStart;
     a.m = nb - colStart;
-    a.triangle = colEnd - colStart > 1;
-    HS_REQUIRE(colEnd == nb || !a.triangle, "the trailing triangle or one column");
-    const int64_t blocks = a.triangle ? (int64_t)a.m * (a.m + 1) / 2 : a.m;
-    const int64_t per_block = (int64_t)(bsz / 128) * (bsz / 128);
-    a.items = blocks * per_block;
     a.info = ctx->d_info;
+    const int64_t blocks = (int64_t)a.m * (a.m + 1) / 2;
+    a.items = blocks * (bsz / 128) * (bsz / 128);
     const int64_t grid = (a.items + kPerCta - 1) / kPerCta;
     HS_REQUIRE(grid < (1LL << 31), "trailing update too large for one launch");
-    const double n = bsz, cols = colEnd - colStart;
-    prof_begin(ctx, s, HS_KERNEL_UPDATE);
-    ctx->launches += 1;
     split_update_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(a);
     HS_CHECK_LAUNCH("split_update");
-    prof_end(ctx, s, HS_KERNEL_UPDATE, (blocks - cols) * 2.0 * n * n * n + cols * n * n * (n + 1.0),
-             (2.0 * blocks + a.m) * n * n * 8.0);
+    const double n = bsz, m = a.m;
+    prof_end(ctx, s, HS_KERNEL_UPDATE, panels * ((blocks - m) * 2.0 * n * n * n + m * n * n * (n + 1.0)),
+             (2.0 * blocks + panels * m) * n * n * 8.0);
     return HS_OK;
 }
 
