@@ -66,11 +66,15 @@ void adjoint_bind(void* base, int nb, int bsz, AdjointWork* w);
 // entries of A = L L^T; L is not modified
 hs_status cholesky_adjoint_impl(hs_ctx ctx, const double* L, double* Abar, const AdjointWork& w, cudaStream_t s);
 
-// Abar <- the adjoint of sum_i log L_ii with respect to the lower entries of A = L L^T:
-// A^-1 below the diagonal, half of it on the diagonal.  Y: L_kk^-T for every diagonal block.
-// L's off-diagonal blocks are overwritten.
-hs_status logdet_adjoint_impl(hs_ctx ctx, double* L, double* Abar, const double* Y, const AdjointWork& w,
+// The adjoint of sum_i log L_ii with respect to the lower entries of A = L L^T: A^-1 below the
+// diagonal, half of it on the diagonal, in *out (L or Abar; both are overwritten).  Y: L_kk^-T
+// for every diagonal block.
+hs_status logdet_adjoint_impl(hs_ctx ctx, double* L, double* Abar, const double* Y, const AdjointWork& w, double** out,
                               cudaStream_t s);
+// S <- the identity, lower blocks row by row
+hs_status launch_identity_by_rows(hs_ctx ctx, double* S, cudaStream_t s);
+// the diagonal entries of a packed lower matrix halved
+hs_status launch_halve_diagonal(hs_ctx ctx, double* A, cudaStream_t s);
 // L_rk <- L_rk Y_k^T = L_rk L_kk^-1 for every off-diagonal block of the packed factor
 hs_status launch_scale_panels(hs_ctx ctx, double* L, const double* Y, cudaStream_t s);
 

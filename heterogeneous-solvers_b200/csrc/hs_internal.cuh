@@ -218,6 +218,11 @@ hs_status launch_update_cols(hs_ctx ctx, double* A, int blockID, int blockRow, i
 // 256-byte aligned; a wait that ran out: -1 in d_info
 size_t split_update_bytes(int nb, int bsz, int panels);
 hs_status launch_split_update(hs_ctx ctx, double* A, int k, int panels, int colStart, void* ws, cudaStream_t s);
+// block row k of the inverse by W = L^-1, A^-1 = W^T W (blocks of 256).  W: row k of W, k + 1
+// blocks; S (blocks of the lower triangle, row by row) -= column k of L times it for the rows
+// below; column k of L is then cleared and L's first k + 1 block columns += W_k^T W_k
+size_t split_inverse_bytes(int nb);
+hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* W, double* S, void* ws, cudaStream_t s);
 // one diagonal block of bsz 128 or 256 (k_diag.cu): L and its inverse in one launch
 struct DiagFactor {
     const double* in64 = nullptr;  // the block, or

@@ -301,6 +301,20 @@ __global__ void sym_tril_half_kernel(const double* __restrict__ G, double* __res
     }
 }
 
+__global__ void unit_diag_by_rows_kernel(double* __restrict__ S, int bsz, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t b = i / bsz, r = i % bsz;
+    S[((tri64(b) + b) * bsz + r) * bsz + r] = 1.0;
+}
+
+__global__ void halve_diagonal_kernel(double* __restrict__ A, int bsz, int nb, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int64_t b = i / bsz, r = i % bsz;
+    A[(block_id(b, b, nb) * bsz + r) * bsz + r] *= 0.5;
+}
+
 // Split count of a chain over `base_ctas` output tiles (`sms` = CTAs resident at once): the s that
 // minimises the time model waves(base s) x ceil(chain / s) chain steps, plus the
 // fixed-order reduction of the s partial blocks of each item (~0.1 chain step a
@@ -405,6 +419,23 @@ hs_status launch_sym_tril_half(hs_ctx ctx, const double* G, double* M, cudaStrea
     ctx->launches += 1;
     sym_tril_half_kernel<<<64, 256, 0, s>>>(G, M, ctx->bsz);
     HS_CHECK_LAUNCH("sym tril half");
+    return HS_OK;
+}
+
+hs_status launch_identity_by_rows(hs_ctx ctx, double* S, cudaStream_t s) {
+    const int64_t n = (int64_t)ctx->nb * ctx->bsz;
+    HS_CUDA(cudaMemsetAsync(S, 0, (size_t)total_blocks(ctx->nb) * ctx->bsz * ctx->bsz * sizeof(double), s));
+    ctx->launches += 1;
+    unit_diag_by_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(S, ctx->bsz, n);
+    HS_CHECK_LAUNCH("unit diagonal");
+    return HS_OK;
+}
+
+hs_status launch_halve_diagonal(hs_ctx ctx, double* A, cudaStream_t s) {
+    const int64_t n = (int64_t)ctx->nb * ctx->bsz;
+    ctx->launches += 1;
+    halve_diagonal_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(A, ctx->bsz, ctx->nb, n);
+    HS_CHECK_LAUNCH("halve diagonal");
     return HS_OK;
 }
 

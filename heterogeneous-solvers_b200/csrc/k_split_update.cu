@@ -39,28 +39,15 @@ constexpr int kPerCta = 4;     // tiles a CTA
 constexpr int kMinExp = -900;  // rows whose largest entry lies below 2^-900 keep that scale
 
 // ------------------------------------------------------------------ digits
-// One warp a row of the panel: its scale and its seven planes, in the order the update reads them: for
-// each 128 rows and 64 columns the planes one after the other, each as 64-byte rows with the
-// 64-byte swizzle (16-byte unit u of row r at u ^ (r / 2 % 4)), so that an operand's stage is
-// one contiguous copy.  A row that holds an infinity or NaN gets the scale NaN (and zero
-// digits), so that what it updates becomes NaN.
-// K entries a row: of one panel (P1 unused) or half of them of each of two.
-template <int K>
-__global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ P0, const double* __restrict__ P1, int bsz,
-                                                     int64_t rows, int8_t* __restrict__ D, double* __restrict__ scale) {
-    constexpr int E = K / 32;  // entries a lane
-    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const double* src = (lane * E < bsz ? P0 : P1) + row * bsz + lane * E % bsz;
-    double v[E];
+// One row's scale and seven planes, by a warp whose lane holds entries E lane .. of the K = 32 E,
+// in the order the update reads them: for each 128 rows and 64 columns the planes one after
+// the other, each as 64-byte rows with the 64-byte swizzle (16-byte unit u of row r at
+// u ^ (r / 2 % 4)), so that an operand's stage is one contiguous copy.  A row that holds an
+// infinity or NaN gets the scale NaN (and zero digits), so that what it updates becomes NaN.
+template <int E>
+__device__ __forceinline__ void split_row(const double (&v)[E], int64_t row, int lane, int8_t* D, double* scale) {
+    constexpr int K = 32 * E;
     long long m = 0;
-#pragma unroll
-    for (int q = 0; q < E / 2; ++q) {
-        const double2 x = *reinterpret_cast<const double2*>(src + 2 * q);
-        v[2 * q] = x.x;
-        v[2 * q + 1] = x.y;
-    }
 #pragma unroll
     for (int q = 0; q < E; ++q) m = max(m, __double_as_longlong(v[q]) & 0x7fffffffffffffffll);
 #pragma unroll
@@ -98,6 +85,43 @@ __global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ 
         scale[row] = finite ? __longlong_as_double((long long)(e - 28 + 1023) << 52) : __longlong_as_double(~0ll);
 }
 
+// The rows of a panel; K entries a row: of one panel (P1 unused) or half of them of each of two.
+template <int K>
+__global__ void __launch_bounds__(256) digits_kernel(const double* __restrict__ P0, const double* __restrict__ P1, int bsz,
+                                                     int64_t rows, int8_t* __restrict__ D, double* __restrict__ scale) {
+    constexpr int E = K / 32;  // entries a lane
+    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    const double* src = (lane * E < bsz ? P0 : P1) + row * bsz + lane * E % bsz;
+    double v[E];
+#pragma unroll
+    for (int q = 0; q < E / 2; ++q) {
+        const double2 x = *reinterpret_cast<const double2*>(src + 2 * q);
+        v[2 * q] = x.x;
+        v[2 * q + 1] = x.y;
+    }
+    split_row<E>(v, row, lane, D, scale);
+}
+
+// The columns of consecutive blocks of 256, 16 of them a CTA
+__global__ void __launch_bounds__(256) digits_transposed_kernel(const double* __restrict__ P, int8_t* __restrict__ D,
+                                                                double* __restrict__ scale) {
+    __shared__ double t[256][17];
+    const double* src = P + (size_t)blockIdx.y * 65536 + blockIdx.x * 16;
+    for (int e = threadIdx.x; e < 256 * 16; e += 256) t[e >> 4][e & 15] = src[(size_t)(e >> 4) * 256 + (e & 15)];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int z = 0; z < 2; ++z) {
+        const int c = 2 * (threadIdx.x >> 5) + z;
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = t[8 * lane + q][c];
+        split_row<8>(v, (int64_t)blockIdx.y * 256 + blockIdx.x * 16 + c, lane, D, scale);
+    }
+}
+
 // ------------------------------------------------------------------ update
 // Bounded waits that suspend the thread between tries: warps that poll take the shared-memory
 // port from the tensor core's operands.
@@ -122,13 +146,19 @@ __device__ __forceinline__ bool suspended_wait_warp(uint64_t* bar, uint32_t pari
     return true;
 }
 
+// C += sign A B^T over a part of the blocks of C
 struct SplitArgs {
-    double* A;
-    const int8_t* digits;
-    const double* scale;  // of the panels' rows, from block row row0 on
-    int row0, depth;      // depth: columns of the panels, 256 or 512
+    double* C;
+    const int8_t *digA, *digB;
+    const double *scaleA, *scaleB;
+    double sign;
+    int depth;         // columns of A and B: 256 or 512
     int nb, bsz;
-    int first_col, m;  // the trailing triangle of m block columns
+    int by_rows;       // C: blocks of a lower triangle stored row by row (else column by column)
+    int rows;          // 0: a lower triangle of `cols` block columns; else a rectangle of rows x cols
+    int cols;
+    int r0, c0;        // its first block row and column in C
+    int offset;        // the same in A's and B's digits (in blocks)
     int64_t items;     // 128 x 128 tiles
     long long* info;
 };
@@ -202,7 +232,7 @@ __device__ __forceinline__ void add_tile(double* C, int ldc, const double* row_s
         for (int o = 0; o < 2; ++o) {
             const int r = 16 * (h >> 1) + 8 * o + gr;
             double* p = C + (size_t)r * ldc + 2 * t4;
-            const double sr = -row_scale[r];
+            const double sr = row_scale[r];
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -214,7 +244,7 @@ __device__ __forceinline__ void add_tile(double* C, int ldc, const double* row_s
         }
 }
 
-// a tile: its entry (0, 0) in A, its rows' and columns' first rows in the panel, in 128s
+// a tile: its entry (0, 0) in C, its first rows in A and B, in 128s
 struct Tile {
     int64_t c;
     int rows, cols;
@@ -225,15 +255,19 @@ __device__ __forceinline__ Tile decode(const SplitArgs& a, int64_t item) {
     const int64_t p = item >> lg;
     const int e = (int)item & ((1 << lg) - 1), ti = e >> (lg >> 1), tj = e & (side - 1);
     int rr, cc;
-    grouped_pair(p, a.m, &rr, &cc);
-    rr += a.first_col;
-    cc += a.first_col;
+    if (a.rows > 0) {
+        rr = (int)(p % a.rows);
+        cc = (int)(p / a.rows);
+    } else {
+        grouped_pair(p, a.cols, &rr, &cc);
+    }
+    const int64_t r = a.r0 + rr, c = a.c0 + cc;
     Tile t;
-    t.c = (block_id(rr, cc, a.nb) * a.bsz + ti * 128) * a.bsz + tj * 128;
-    t.rows = (rr - a.row0) * side + ti;
-    t.cols = (cc - a.row0) * side + tj;
-    t.skip = t.rows < t.cols;
-    t.lower = t.rows == t.cols;
+    t.c = ((a.by_rows ? tri64(r) + c : block_id(r, c, a.nb)) * a.bsz + ti * 128) * a.bsz + tj * 128;
+    t.rows = (a.offset + rr) * side + ti;
+    t.cols = (a.offset + cc) * side + tj;
+    t.skip = a.rows == 0 && t.rows < t.cols;
+    t.lower = a.rows == 0 && t.rows == t.cols;
     return t;
 }
 
@@ -294,8 +328,8 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
             for (int it = 0; it < count && ok; ++it) {
                 const Tile t = tiles[it];
                 if (t.skip) continue;
-                const int8_t* dA = a.digits + (int64_t)t.rows * chunks * kOperand;
-                const int8_t* dB = a.digits + (int64_t)t.cols * chunks * kOperand;
+                const int8_t* dA = a.digA + (int64_t)t.rows * chunks * kOperand;
+                const int8_t* dB = a.digB + (int64_t)t.cols * chunks * kOperand;
                 for (int pass = 0; pass < 2 && ok; ++pass) {
                     const uint32_t bytes = (pass ? kHighPlanes : kPlanes) * kPlane;
                     for (int kc = 0; kc < chunks; ++kc, ++g) {
@@ -355,9 +389,9 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
         for (int it = 0; it < count; ++it) {  // also after a wait ran out: the barriers below
             const Tile t = tiles[it];
             if (t.skip) continue;
-            double* C = a.A + t.c + (int64_t)(32 * q) * a.bsz + col0;
+            double* C = a.C + t.c + (int64_t)(32 * q) * a.bsz + col0;
             const int e = threadIdx.x - 64;
-            const double sc = e < 256 ? a.scale[(int64_t)(e < 128 ? t.rows : t.cols) * 128 + (e & 127)] : 0.0;
+            const double sc = e < 128 ? a.sign * a.scaleA[(int64_t)t.rows * 128 + e] : a.scaleB[(int64_t)t.cols * 128 + e - 128];
             asm volatile("bar.sync 1, 256;" ::: "memory");  // every warp has read the last tile's
             if (e < 256) scales[e] = sc;
             asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -408,50 +442,108 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
     if (warp == 0) tmem_dealloc(taddr, 512);
 }
 
-}  // namespace
 
-size_t split_update_bytes(int nb, int bsz, int panels) {
-    const size_t rows = (size_t)(nb - panels) * bsz;
-    return rows * panels * bsz * kPlanes + rows * sizeof(double);
+size_t digits_bytes(int64_t rows, int depth) { return (size_t)rows * (depth * kPlanes + sizeof(double)); }
+
+hs_status launch_products(hs_ctx ctx, SplitArgs& a, cudaStream_t s) {
+    const int64_t blocks = a.rows > 0 ? (int64_t)a.rows * a.cols : tri64(a.cols);
+    a.nb = ctx->nb;
+    a.bsz = ctx->bsz;
+    a.items = blocks * (a.bsz / 128) * (a.bsz / 128);
+    a.info = ctx->d_info;
+    const int64_t grid = (a.items + kPerCta - 1) / kPerCta;
+    HS_REQUIRE(grid < (1LL << 31), "too many tiles for one launch");
+    HS_CUDA(cudaFuncSetAttribute(split_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    ctx->launches += 1;
+    split_update_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(a);
+    HS_CHECK_LAUNCH("split_update");
+    return HS_OK;
 }
 
+}  // namespace
+
+size_t split_update_bytes(int nb, int bsz, int panels) { return digits_bytes((int64_t)(nb - panels) * bsz, panels * bsz); }
+
 hs_status launch_split_update(hs_ctx ctx, double* A, int k, int panels, int colStart, void* ws, cudaStream_t s) {
-    const int nb = ctx->nb, bsz = ctx->bsz;
+    const int nb = ctx->nb, bsz = ctx->bsz, row0 = k + panels;
     const size_t bb = (size_t)bsz * bsz;
+    const int64_t rows = (int64_t)(nb - row0) * bsz;
     SplitArgs a{};
-    a.row0 = k + panels;
     a.depth = panels * bsz;
     HS_REQUIRE(a.depth == 256 || a.depth == 512, "one or two panels of 256, or two of 128");
-    const int64_t rows = (int64_t)(nb - a.row0) * bsz;
     int8_t* D = static_cast<int8_t*>(ws);
     double* scale = reinterpret_cast<double*>(D + rows * a.depth * kPlanes);
-    const double* P0 = A + (size_t)block_id(a.row0, k, nb) * bb;
-    const double* P1 = panels == 2 ? A + (size_t)block_id(a.row0, k + 1, nb) * bb : P0;
-    HS_CUDA(cudaFuncSetAttribute(split_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    const double* P0 = A + (size_t)block_id(row0, k, nb) * bb;
+    const double* P1 = panels == 2 ? A + (size_t)block_id(row0, k + 1, nb) * bb : P0;
     prof_begin(ctx, s, HS_KERNEL_UPDATE);
-    ctx->launches += 2;
+    ctx->launches += 1;
     if (a.depth == 512)
         digits_kernel<512><<<(unsigned)(rows / 8), 256, 0, s>>>(P0, P1, bsz, rows, D, scale);
     else
         digits_kernel<256><<<(unsigned)(rows / 8), 256, 0, s>>>(P0, P1, bsz, rows, D, scale);
     HS_CHECK_LAUNCH("split_digits");
-    a.A = A;
-    a.digits = D;
-    a.scale = scale;
-    a.nb = nb;
-    a.bsz = bsz;
-    a.first_col = colStart;
-    a.m = nb - colStart;
-    a.info = ctx->d_info;
-    const int64_t blocks = (int64_t)a.m * (a.m + 1) / 2;
-    a.items = blocks * (bsz / 128) * (bsz / 128);
-    const int64_t grid = (a.items + kPerCta - 1) / kPerCta;
-    HS_REQUIRE(grid < (1LL << 31), "trailing update too large for one launch");
-    split_update_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(a);
-    HS_CHECK_LAUNCH("split_update");
-    const double n = bsz, m = a.m;
+    a.C = A;
+    a.digA = a.digB = D;
+    a.scaleA = a.scaleB = scale;
+    a.sign = -1.0;
+    a.cols = nb - colStart;
+    a.r0 = a.c0 = colStart;
+    a.offset = colStart - row0;
+    hs_status st = launch_products(ctx, a, s);
+    if (st != HS_OK) return st;
+    const double n = bsz, m = a.cols, blocks = m * (m + 1) / 2;
     prof_end(ctx, s, HS_KERNEL_UPDATE, panels * ((blocks - m) * 2.0 * n * n * n + m * n * n * (n + 1.0)),
              (2.0 * blocks + panels * m) * n * n * 8.0);
+    return HS_OK;
+}
+
+size_t split_inverse_bytes(int nb) { return 2 * digits_bytes((int64_t)nb * 256, 256); }
+
+hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* W, double* S, void* ws, cudaStream_t s) {
+    const int nb = ctx->nb;
+    const size_t bb = 65536;
+    HS_REQUIRE(ctx->bsz == 256, "blocks of 256");
+    const int64_t cap = (int64_t)nb * 256;
+    int8_t *DW = static_cast<int8_t*>(ws), *DL = DW + cap * 256 * kPlanes;
+    double *scaleW = reinterpret_cast<double*>(DL + cap * 256 * kPlanes), *scaleL = scaleW + cap;
+    prof_begin(ctx, s, HS_KERNEL_ADJOINT);
+    ctx->launches += 1;
+    digits_transposed_kernel<<<dim3(16, k + 1), 256, 0, s>>>(W, DW, scaleW);
+    HS_CHECK_LAUNCH("digits_transposed");
+    SplitArgs a{};
+    a.depth = 256;
+    a.digB = DW;
+    a.scaleB = scaleW;
+    hs_status st;
+    const int below = nb - k - 1;
+    if (below > 0) {
+        const int64_t rows = (int64_t)below * 256;
+        ctx->launches += 1;
+        digits_kernel<256><<<(unsigned)(rows / 8), 256, 0, s>>>(L + (size_t)block_id(k + 1, k, nb) * bb, nullptr, 256, rows, DL,
+                                                                scaleL);
+        HS_CHECK_LAUNCH("split_digits");
+        a.C = S;
+        a.by_rows = 1;
+        a.digA = DL;
+        a.scaleA = scaleL;
+        a.sign = -1.0;
+        a.rows = below;
+        a.cols = k + 1;
+        a.r0 = k + 1;
+        if ((st = launch_products(ctx, a, s)) != HS_OK) return st;
+    }
+    HS_CUDA(cudaMemsetAsync(L + (size_t)block_id(k, k, nb) * bb, 0, (size_t)(nb - k) * bb * sizeof(double), s));
+    a.C = L;
+    a.by_rows = 0;
+    a.digA = DW;
+    a.scaleA = scaleW;
+    a.sign = 1.0;
+    a.rows = 0;
+    a.cols = k + 1;
+    a.r0 = 0;
+    if ((st = launch_products(ctx, a, s)) != HS_OK) return st;
+    const double blocks = (double)below * (k + 1) + 0.5 * (k + 1) * (k + 2), n = 256;
+    prof_end(ctx, s, HS_KERNEL_ADJOINT, 2.0 * blocks * n * n * n, 2.0 * blocks * n * n * 8.0);
     return HS_OK;
 }
 

@@ -33,10 +33,11 @@ def test_gradient_at_block_edges(hs, ctx, N, bsz, d, ard):
     assert np.max(np.abs(grad - grad_ref)) <= tol * (np.max(np.abs(grad_ref)) + N / 2)
 
 
-def test_gradient_with_large_tiles(hs, ctx):
-    """Enough block rows that the products take large tiles and whole waves; the reference is
-    the dense inverse in FP64 on the device, with the bound of the test above."""
-    N, bsz, d, sf2, sn2 = 10100, 256, 3, 1.3, 2e-2
+@pytest.mark.parametrize("N", [4864, 4865, 10100])
+def test_gradient_of_many_blocks(hs, ctx, N):
+    """Either side of the rule that takes the inverse to the INT8 tensor cores, and large tiles;
+    the reference is the dense inverse in FP64 on the device, with the bound of the test above."""
+    bsz, d, sf2, sn2 = 256, 3, 1.3, 2e-2
     g = torch.Generator(device="cuda")
     g.manual_seed(N)
     X = torch.rand((N, d), dtype=torch.float64, device="cuda", generator=g)
@@ -54,3 +55,18 @@ def test_gradient_with_large_tiles(hs, ctx):
     ref += [0.5 * (W * Kf).sum().item(), 0.5 * sn2 * W.diagonal().sum().item()]
     tol = 64 * 2.0 ** -52 * (sf2 * N / sn2 + 1)
     assert np.max(np.abs(grad - ref)) <= tol * (np.max(np.abs(ref)) + N / 2)
+
+
+def test_gradient_of_many_small_blocks(hs, ctx):
+    """Blocks of 128 stay with the recurrence; enough of them for its large tiles."""
+    N, d = 5000, 2
+    rng = np.random.default_rng(N)
+    X = rng.random((N, d))
+    y = np.sin(X.sum(1)) + 0.1 * rng.standard_normal(N)
+    theta = np.log([0.7, 1.1, 1.3, 2e-2])
+    grads = []
+    for bsz in (128, 256):
+        ctx.set_problem(N, bsz)
+        grads.append(hs.gp_nlml_grad(ctx, X, y, theta)[1])
+    tol = 64 * 2.0 ** -52 * (1.3 * N / 2e-2 + 1)
+    assert np.max(np.abs(grads[0] - grads[1])) <= tol * (np.max(np.abs(grads[0])) + N / 2)
