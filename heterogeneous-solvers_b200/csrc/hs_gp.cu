@@ -217,9 +217,9 @@ hs_status cholesky_adjoint_impl(hs_ctx ctx, const double* L, double* Abar, const
     return HS_OK;
 }
 
-// From 20 block rows the digits pay (a gradient at N = 4000 4.76 ms by the recurrence and 5.09
-// by these, 6000: 11.3 and 9.7, 16384: 133 and 88).
-constexpr int kSplitInverseBlocks = 20;
+// From 13 block rows the digits pay: a gradient at N = 3000 2.94 ms by the recurrence and 2.95
+// by these, 3500: 3.76 and 3.49, 6000: 11.3 and 8.2, 16384: 133 and 88.6.
+constexpr int kSplitInverseBlocks = 13;
 
 hs_status logdet_adjoint_impl(hs_ctx ctx, double* L, double* Abar, const double* Y, const AdjointWork& w, double** out,
                               cudaStream_t s) {
@@ -237,11 +237,21 @@ hs_status logdet_adjoint_impl(hs_ctx ctx, double* L, double* Abar, const double*
         // A^-1 = W^T W with W = L^-1, both by updates of rank 256 on the INT8 tensor cores: block
         // row k of W is L_kk^-1 (I - sum_c<k L_kc W_c), its term is taken from the rows
         // below and its product with itself added to A^-1, in place of L's first k + 1
-        // block columns, which are no longer needed.  S holds the rows' sums.
+        // block columns, which are no longer needed.  S holds the rows' sums.  The products with
+        // itself run on the side stream, beside the next rows (92 -> 88.6 ms at N = 16384).
         const size_t bytes = kSmallScratch + split_inverse_bytes(nb);
         if (ensure_scratch(ctx, bytes) == HS_OK) {
             double* S = Abar;
             char* digits = static_cast<char*>(ctx->scratch) + kSmallScratch;
+            cudaStream_t side = ctx->side ? ctx->side : s;
+            struct Events {
+                cudaEvent_t e[2] = {};
+                ~Events() {
+                    for (auto& v : e)
+                        if (v) cudaEventDestroy(v);
+                }
+            } done;
+            for (auto& v : done.e) HS_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
             if ((st = launch_identity_by_rows(ctx, S, s)) != HS_OK) return st;
             for (int k = 0; k < nb; ++k) {
                 ChainArgs a = chain_args(bsz);  // row k of W = L_kk^-1 (row k of S)
@@ -254,8 +264,9 @@ hs_status logdet_adjoint_impl(hs_ctx ctx, double* L, double* Abar, const double*
                 a.C0 = w.T;
                 a.sCi = bb;
                 if ((st = launch_chain(ctx, a, nullptr, 0, s)) != HS_OK) return st;
-                if ((st = launch_split_inverse_step(ctx, L, k, w.T, S, digits, s)) != HS_OK) return st;
+                if ((st = launch_split_inverse_step(ctx, L, k, w.T, S, digits, s, side, done.e)) != HS_OK) return st;
             }
+            HS_CUDA(cudaStreamWaitEvent(s, done.e[(nb - 1) & 1], 0));
             *out = L;
             return launch_halve_diagonal(ctx, L, s);
         }

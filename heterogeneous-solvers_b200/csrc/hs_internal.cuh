@@ -220,9 +220,12 @@ size_t split_update_bytes(int nb, int bsz, int panels);
 hs_status launch_split_update(hs_ctx ctx, double* A, int k, int panels, int colStart, void* ws, cudaStream_t s);
 // block row k of the inverse by W = L^-1, A^-1 = W^T W (blocks of 256).  W: row k of W, k + 1
 // blocks; S (blocks of the lower triangle, row by row) -= column k of L times it for the rows
-// below; column k of L is then cleared and L's first k + 1 block columns += W_k^T W_k
+// below; column k of L is then cleared and, on `side`, L's first k + 1 block columns +=
+// W_k^T W_k (done[k & 1] is recorded there)
 size_t split_inverse_bytes(int nb);
-hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* W, double* S, void* ws, cudaStream_t s);
+hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* W, double* S, void* ws,
+                                    cudaStream_t s, cudaStream_t side,
+                                    cudaEvent_t (&done)[2]);
 // one diagonal block of bsz 128 or 256 (k_diag.cu): L and its inverse in one launch
 struct DiagFactor {
     const double* in64 = nullptr;  // the block, or

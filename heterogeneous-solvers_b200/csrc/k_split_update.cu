@@ -497,15 +497,20 @@ hs_status launch_split_update(hs_ctx ctx, double* A, int k, int panels, int colS
     return HS_OK;
 }
 
-size_t split_inverse_bytes(int nb) { return 2 * digits_bytes((int64_t)nb * 256, 256); }
+size_t split_inverse_bytes(int nb) { return 3 * digits_bytes((int64_t)nb * 256, 256); }
 
-hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* W, double* S, void* ws, cudaStream_t s) {
+hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* W, double* S, void* ws,
+                                    cudaStream_t s, cudaStream_t side,
+                                    cudaEvent_t (&done)[2]) {
     const int nb = ctx->nb;
     const size_t bb = 65536;
     HS_REQUIRE(ctx->bsz == 256, "blocks of 256");
     const int64_t cap = (int64_t)nb * 256;
-    int8_t *DW = static_cast<int8_t*>(ws), *DL = DW + cap * 256 * kPlanes;
-    double *scaleW = reinterpret_cast<double*>(DL + cap * 256 * kPlanes), *scaleL = scaleW + cap;
+    const size_t one = digits_bytes(cap, 256);
+    int8_t *DW = static_cast<int8_t*>(ws) + (k & 1) * one, *DL = static_cast<int8_t*>(ws) + 2 * one;
+    double* scaleW = reinterpret_cast<double*>(DW + cap * 256 * kPlanes);
+    double* scaleL = reinterpret_cast<double*>(DL + cap * 256 * kPlanes);
+    if (k >= 2) HS_CUDA(cudaStreamWaitEvent(s, done[k & 1], 0));  // step k - 2's product with itself
     prof_begin(ctx, s, HS_KERNEL_ADJOINT);
     ctx->launches += 1;
     digits_transposed_kernel<<<dim3(16, k + 1), 256, 0, s>>>(W, DW, scaleW);
@@ -530,9 +535,11 @@ hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* 
         a.rows = below;
         a.cols = k + 1;
         a.r0 = k + 1;
-        if ((st = launch_products(ctx, a, s)) != HS_OK) return st;
     }
-    HS_CUDA(cudaMemsetAsync(L + (size_t)block_id(k, k, nb) * bb, 0, (size_t)(nb - k) * bb * sizeof(double), s));
+    HS_CUDA(cudaEventRecord(ctx->ev_a, s));
+    HS_CUDA(cudaStreamWaitEvent(side, ctx->ev_a, 0));
+    if (below > 0 && (st = launch_products(ctx, a, s)) != HS_OK) return st;
+    HS_CUDA(cudaMemsetAsync(L + (size_t)block_id(k, k, nb) * bb, 0, (size_t)(nb - k) * bb * sizeof(double), side));
     a.C = L;
     a.by_rows = 0;
     a.digA = DW;
@@ -541,7 +548,8 @@ hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* 
     a.rows = 0;
     a.cols = k + 1;
     a.r0 = 0;
-    if ((st = launch_products(ctx, a, s)) != HS_OK) return st;
+    if ((st = launch_products(ctx, a, side)) != HS_OK) return st;
+    HS_CUDA(cudaEventRecord(done[k & 1], side));
     const double blocks = (double)below * (k + 1) + 0.5 * (k + 1) * (k + 2), n = 256;
     prof_end(ctx, s, HS_KERNEL_ADJOINT, 2.0 * blocks * n * n * n, 2.0 * blocks * n * n * 8.0);
     return HS_OK;

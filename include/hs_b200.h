@@ -148,6 +148,7 @@ hs_status hs_ctx_set_mixed_lookahead(hs_ctx ctx, int side_sms, int min_rows);
 hs_status hs_potrf_block(hs_ctx ctx, double* A, int blockID, int blockRow);
 /* Read (and reset) the context's pivot record: *info = -1 when every POTRF since
  * the last call saw positive pivots, else the smallest failing global row.
+ * HS_ERR_TIMEOUT when a bounded wait of the factor's updates ran out.
  * Synchronises the stream. */
 hs_status hs_ctx_take_info(hs_ctx ctx, int64_t* info);
 /* Self-test of the failure path of every device-side wait in the library (no

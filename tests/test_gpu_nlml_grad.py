@@ -33,7 +33,7 @@ def test_gradient_at_block_edges(hs, ctx, N, bsz, d, ard):
     assert np.max(np.abs(grad - grad_ref)) <= tol * (np.max(np.abs(grad_ref)) + N / 2)
 
 
-@pytest.mark.parametrize("N", [4864, 4865, 10100])
+@pytest.mark.parametrize("N", [3072, 3073, 4865, 10100])
 def test_gradient_of_many_blocks(hs, ctx, N):
     """Either side of the rule that takes the inverse to the INT8 tensor cores, and large tiles;
     the reference is the dense inverse in FP64 on the device, with the bound of the test above."""
