@@ -1,14 +1,15 @@
 // k_split_update.cu — the FP64 trailing update on the tensor cores' INT8 path.
 //
 // The large trailing updates of the FP64 Cholesky (MatrixMatrixOperations.cpp:146-906) are
-// C <- C - P P^T with a panel P of one block column, or of two at once.  The FP64 tensor pipe bounds them at 64
-// multiply-adds a cycle and SM; the INT8 pipe does 8192.  Each row of the panel is therefore
-// scaled by a power of two to |t| <= 0.497 and written as seven balanced
-// base-256 digits, t = sum_i d_i 2^-8(i+1) with |error| <= 2^-57, and the product of two rows
-// is the sum over levels l = i + j of 2^-8l (digit plane i) x (digit plane j): exact INT32
-// sums in the tensor cores, levels 0..7 kept (34 plane products), carried into one 64-bit
-// integer, rounded to FP64 once and added to C.  (K. Ozaki, T. Ogita, S. Oishi, S. M. Rump,
-// "Error-free transformations of matrix multiplication by using fast routines of matrix
+// C <- C - P P^T with a panel P of one block column, or of two at once; the inverse of the
+// likelihood's gradient is built from updates C <- C +- P Q^T of the same form.  The FP64
+// tensor pipe bounds them at 64 multiply-adds a cycle and SM; the INT8 pipe does 8192.  Each
+// row of a panel is therefore scaled by a power of two to |t| <= 0.497 and written as seven
+// balanced base-256 digits, t = sum_i d_i 2^-8(i+1) with |error| <= 2^-57, and the product of
+// two rows is the sum over levels l = i + j of 2^-8l (digit plane i) x (digit plane j): exact
+// INT32 sums in the tensor cores, levels 0..7 kept (34 plane products), carried into one
+// 64-bit integer, rounded to FP64 once and added to C.  (K. Ozaki, T. Ogita, S. Oishi, S. M.
+// Rump, "Error-free transformations of matrix multiplication by using fast routines of matrix
 // multiplication and its applications", 2012; H. Ootomo, K. Ozaki, R. Yokota, "DGEMM on
 // integer matrix multiplication unit", 2024.)
 //
@@ -33,7 +34,7 @@ constexpr int kKc = 64;                      // K bytes a stage (64-byte swizzle
 constexpr int kPlane = 128 * kKc;            // one plane of 128 rows of a stage
 constexpr int kOperand = kPlanes * kPlane;
 constexpr int kStage = 2 * kOperand, kStages = 2;  // 112 KB each
-constexpr int kSmem = 512 + kStages * kStage + 256 * 8 + 104;  // + the tile's scales, barriers
+constexpr int kSmem = 512 + kStages * kStage + 256 * 8 + 112;  // + the tile's scales, barriers
 constexpr int kEpi = 8, kThreads = 64 + 32 * kEpi;  // copy warp, MMA warp, epilogue warps
 constexpr int kPerCta = 4;     // tiles a CTA
 constexpr int kMinExp = -900;  // rows whose largest entry lies below 2^-900 keep that scale
@@ -391,7 +392,8 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
             if (t.skip) continue;
             double* C = a.C + t.c + (int64_t)(32 * q) * a.bsz + col0;
             const int e = threadIdx.x - 64;
-            const double sc = e < 128 ? a.sign * a.scaleA[(int64_t)t.rows * 128 + e] : a.scaleB[(int64_t)t.cols * 128 + e - 128];
+            const double sc = e < 128 ? a.sign * a.scaleA[(int64_t)t.rows * 128 + e]
+                                      : a.scaleB[(int64_t)t.cols * 128 + e - 128];
             asm volatile("bar.sync 1, 256;" ::: "memory");  // every warp has read the last tile's
             if (e < 256) scales[e] = sc;
             asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -524,8 +526,8 @@ hs_status launch_split_inverse_step(hs_ctx ctx, double* L, int k, const double* 
     if (below > 0) {
         const int64_t rows = (int64_t)below * 256;
         ctx->launches += 1;
-        digits_kernel<256><<<(unsigned)(rows / 8), 256, 0, s>>>(L + (size_t)block_id(k + 1, k, nb) * bb, nullptr, 256, rows, DL,
-                                                                scaleL);
+        const double* P = L + (size_t)block_id(k + 1, k, nb) * bb;
+        digits_kernel<256><<<(unsigned)(rows / 8), 256, 0, s>>>(P, nullptr, 256, rows, DL, scaleL);
         HS_CHECK_LAUNCH("split_digits");
         a.C = S;
         a.by_rows = 1;
