@@ -91,8 +91,9 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
     double* red = ring + kWarps * kStages * kUnit;  // [warp][BSZ]
     __shared__ uint64_t s_full[kWarps][kStages];
     __shared__ double s_rows[kWarps][2][RW], s_part[kWarps], s_sum;
-    __shared__ int s_fail, s_good;
-    volatile int* fail = &s_fail;
+    __shared__ Waits s_waits;
+    __shared__ int s_good;
+    volatile Waits* waits = &s_waits;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int P = gridDim.x, c = blockIdx.x, nb = a.nb;
@@ -118,7 +119,10 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
         for (int k = 0; k < kStages; ++k) mbar_init(&full[k], 1);
         fence_barrier_init();
     }
-    if (tid == 0) s_fail = 0;
+    if (tid == 0) {
+        s_waits.fail = 0;
+        s_waits.limit = kWaitClk;
+    }
     __syncthreads();
     uint32_t issued = 0, taken = 0;
     // the unit of the next copy: the warp's units round and round
@@ -164,19 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
                 atomicAdd(a.count, 1ull);
             }
             __syncwarp();
-            bool good = true;
-            const long long t0 = clock64();
-            const unsigned long long want = st.sums * (unsigned long long)P;
-            for (;;) {
-                unsigned long long have = 0;
-                if (lane == 0)
-                    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(have) : "l"(a.count) : "memory");
-                if (__shfl_sync(0xffffffffu, have, 0) >= want) break;
-                if (__any_sync(0xffffffffu, *fail || clock64() - t0 > kWaitClk)) {
-                    good = false;
-                    break;
-                }
-            }
+            warp_count(a.count, st.sums * (unsigned long long)P, lane, waits);
             double y[kMaxCtas / 32];
 #pragma unroll
             for (int k = 0; k < kMaxCtas / 32; ++k) y[k] = lane + 32 * k < P ? __ldcg(part + lane + 32 * k) : 0.0;
@@ -185,9 +177,8 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
             for (int k = 0; k < kMaxCtas / 32; ++k) t += y[k];
             for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
             if (lane == 0) {
-                if (!good) *fail = 1;
                 s_sum = t;
-                s_good = *fail == 0;  // one answer for all warps
+                s_good = waits->fail == 0;  // one answer for all warps
                 if (!s_good) atomicExch(a.err, 1);
             }
         }
@@ -197,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
     };
 
     // phase A: partial sums of A v; v = r + beta d (type 0) or x (type 1).  Returns this
-    // thread's part of v . A v.  A wait that runs out leaves *fail set and the pass goes on
+    // thread's part of v . A v.  A wait that runs out leaves its mark and the pass goes on
     // to its end (later waits return at once); the next grid_sum ends the launch.
     auto matvec = [&](int type, double beta, const double* dold) -> double {
         auto val = [&](int64_t e) -> double {
@@ -221,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
             }
             for (; u < uhi; u += kWarps, ++k) {
                 const uint32_t m = resident ? (uint32_t)k : taken;
-                if (!resident || taken < (uint32_t)own) warp_wait(&full[m % kStages], (m / kStages) & 1, fail);
+                if (!resident || taken < (uint32_t)own) warp_wait(&full[m % kStages], (m / kStages) & 1, waits);
                 ++taken;
                 double* vr = s_rows[warp][k & 1];
                 if (lane < RW) vr[lane] = rv;
@@ -391,9 +382,9 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
     }
     // no copy may still be writing when the CTA leaves
     for (uint32_t h = issued > (uint32_t)kStages ? issued - kStages : 0; h < issued; ++h)
-        warp_wait(&full[h % kStages], (h / kStages) & 1, fail);
+        warp_wait(&full[h % kStages], (h / kStages) & 1, waits);
     __syncthreads();
-    if (tid == 0 && s_fail) atomicExch(a.err, 1);
+    if (tid == 0 && s_waits.fail) atomicExch(a.err, 1);
 }
 
 template <int BSZ>

@@ -1,0 +1,108 @@
+// k_selftest.cu — self-test of the bounded device-side waits: every wait that the library's
+// kernels use, on something that never happens, with a short limit.  No reference counterpart.
+#include <climits>
+#include <string>
+
+#include "hs_internal.cuh"
+#include "stream_common.cuh"
+
+namespace hs {
+namespace {
+
+// one warp a wait
+enum { kThread, kWarp, kSuspended, kSuspendedWarp, kCount, kPairs, kTimer, kWaitKinds };
+const char* const kNames[kWaitKinds] = {"thread_wait", "warp_wait",  "suspended_wait", "suspended_wait_warp",
+                                        "warp_count",  "warp_pairs", "mbar_wait_for"};
+
+struct SelftestArgs {
+    long long limit;                  // SM cycles
+    unsigned long long limit_ns;
+    const unsigned long long* count;  // zero
+    const ulonglong2* pairs;          // 32, zero
+    int* err;
+    int* ran_out;                     // [wait]: 1 if it ran out, and the next one returned at once
+    long long* info;                  // the trailing update's mark
+};
+
+__global__ void __launch_bounds__(32) wait_selftest_kernel(SelftestArgs a) {
+    __shared__ uint64_t bar;
+    __shared__ Waits s_waits;
+    volatile Waits* waits = &s_waits;
+    const int lane = threadIdx.x, kind = blockIdx.x;
+    if (lane == 0) {
+        mbar_init(&bar, 1);  // nothing arrives
+        fence_barrier_init();
+        s_waits.fail = 0;
+        s_waits.limit = a.limit;
+    }
+    __syncwarp();
+    auto wait = [&]() -> bool {
+        double v[1];
+        switch (kind) {
+            case kThread: return lane != 0 || thread_wait(&bar, 0, waits);
+            case kWarp: return warp_wait(&bar, 0, waits);
+            case kSuspended: return lane != 0 || suspended_wait(&bar, 0, waits);
+            case kSuspendedWarp: return suspended_wait_warp(&bar, 0, waits);
+            case kCount: return warp_count(a.count, 1, lane, waits);
+            case kPairs: return warp_pairs(a.pairs, 1, lane, waits, a.err, v);
+            default: return lane != 0 || mbar_wait_for(&bar, 0, a.limit_ns);
+        }
+    };
+    bool out = !wait();
+    __syncwarp();
+    if (kind != kTimer) {
+        const long long t0 = clock64();
+        out = out && !wait() && clock64() - t0 < a.limit / 2 && waits->fail == 1;
+        if (lane == 0 && out && (kind == kSuspended || kind == kSuspendedWarp)) atomicMin(a.info, -1ll);
+    }
+    if (lane == 0) a.ran_out[kind] = out;
+}
+
+}  // namespace
+
+hs_status launch_bounded_wait_selftest(hs_ctx ctx, int64_t timeout_ns) {
+    hs_status st = ensure_scratch(ctx, kSmallScratch);
+    if (st != HS_OK) return st;
+    cudaStream_t s = ctx->stream;
+    char* base = static_cast<char*>(ctx->scratch);
+    SelftestArgs a{};
+    a.limit = 2 * timeout_ns;  // the SM clock stays below 2 GHz
+    a.limit_ns = (unsigned long long)timeout_ns;
+    a.ran_out = reinterpret_cast<int*>(base);
+    a.count = reinterpret_cast<unsigned long long*>(base + 256);
+    a.err = reinterpret_cast<int*>(base + 512);
+    a.pairs = reinterpret_cast<ulonglong2*>(base + 1024);
+    a.info = ctx->d_info;
+    // the pivot record is lent to the test
+    long long record = 0;
+    HS_CUDA(cudaMemcpyAsync(&record, ctx->d_info, sizeof(record), cudaMemcpyDeviceToHost, s));
+    HS_CUDA(cudaMemsetAsync(base, 0, 2048, s));
+    HS_CUDA(cudaStreamSynchronize(s));
+    set_i64_dev(ctx->d_info, INT64_MAX, s);
+    ctx->launches += 2;
+    wait_selftest_kernel<<<kWaitKinds, 32, 0, s>>>(a);
+    HS_CHECK_LAUNCH("wait_selftest");
+    int out[kWaitKinds];
+    HS_CUDA(cudaMemcpyAsync(out, a.ran_out, sizeof(out), cudaMemcpyDeviceToHost, s));
+    HS_CUDA(cudaStreamSynchronize(s));
+    const hs_status mark = hs_ctx_take_info(ctx, nullptr);
+    set_i64_dev(ctx->d_info, record, s);
+    HS_CHECK_LAUNCH("restore info");
+    std::string names, wrong;
+    for (int i = 0; i < kWaitKinds; ++i) {
+        std::string& list = out[i] ? names : wrong;
+        list += (list.empty() ? "" : ", ") + std::string(kNames[i]);
+    }
+    if (!wrong.empty()) {
+        set_error("hs_selftest_bounded_wait: these waits did not run out: " + wrong);
+        return HS_OK;
+    }
+    if (mark != HS_ERR_TIMEOUT) {
+        set_error("hs_selftest_bounded_wait: the trailing update's mark was not reported");
+        return HS_ERR_CUDA;
+    }
+    set_error("hs_selftest_bounded_wait: every bounded wait ran out, as expected here: " + names);
+    return HS_ERR_TIMEOUT;
+}
+
+}  // namespace hs

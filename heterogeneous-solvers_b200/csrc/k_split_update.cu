@@ -124,29 +124,6 @@ __global__ void __launch_bounds__(256) digits_transposed_kernel(const double* __
 }
 
 // ------------------------------------------------------------------ update
-// Bounded waits that suspend the thread between tries: warps that poll take the shared-memory
-// port from the tensor core's operands.
-__device__ __forceinline__ bool suspended_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (*fail || clock64() - t0 > kWaitClk) {
-            *fail = 1;
-            return false;
-        }
-    }
-    return true;
-}
-__device__ __forceinline__ bool suspended_wait_warp(uint64_t* bar, uint32_t parity, volatile int* fail) {
-    const long long t0 = clock64();
-    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
-        if (__any_sync(0xffffffffu, *fail || clock64() - t0 > kWaitClk)) {
-            *fail = 1;
-            return false;
-        }
-    }
-    return true;
-}
-
 // C += sign A B^T over a part of the blocks of C
 struct SplitArgs {
     double* C;
@@ -186,12 +163,12 @@ __device__ __forceinline__ void umma_i8(uint32_t d, uint32_t a, uint32_t b, uint
 // null.
 template <int LEVEL>
 __device__ __forceinline__ bool issue_levels(uint32_t taddr, uint64_t desc, uint32_t accumulate, uint64_t* wait,
-                                             uint64_t* done, uint32_t parity, bool leader, volatile int* fail) {
+                                             uint64_t* done, uint32_t parity, bool leader, volatile Waits* waits) {
     const uint32_t da = (uint32_t)desc, db = da + (kOperand >> 4), high = (uint32_t)(desc >> 32);
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
         if (wait) {
-            if (!suspended_wait_warp(&wait[x], parity, fail)) return false;
+            if (!suspended_wait_warp(&wait[x], parity, waits)) return false;
             tc_fence_after();
         }
         if (leader) {
@@ -293,8 +270,9 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
     uint64_t* bars = reinterpret_cast<uint64_t*>(scales + 256);
     uint64_t *full = bars, *empty = bars + kStages, *tfull = empty + kStages, *tempty = tfull + 4, *drained = tempty + 4;
     uint32_t* slot = reinterpret_cast<uint32_t*>(drained + 1);
-    int* fail = reinterpret_cast<int*>(slot + 1);
     __shared__ Tile tiles[kPerCta];
+    __shared__ Waits s_waits;
+    volatile Waits* waits = &s_waits;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
@@ -306,7 +284,8 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
             mbar_init(&tempty[i], kEpi);
         }
         mbar_init(drained, 1);
-        *fail = 0;
+        s_waits.fail = 0;
+        s_waits.limit = kWaitClk;
         fence_barrier_init();
     }
     if (warp == 0) {
@@ -335,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
                     const uint32_t bytes = (pass ? kHighPlanes : kPlanes) * kPlane;
                     for (int kc = 0; kc < chunks; ++kc, ++g) {
                         const uint32_t s = g % kStages;
-                        if (g >= kStages && !suspended_wait(&empty[s], (g / kStages - 1) & 1, fail)) {
+                        if (g >= kStages && !suspended_wait(&empty[s], (g / kStages - 1) & 1, waits)) {
                             ok = false;
                             break;
                         }
@@ -361,13 +340,13 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
             for (int pass = 0; pass < 2 && ok; ++pass, ++u) {
                 for (int kc = 0; kc < chunks; ++kc, ++g) {
                     const uint32_t s = g % kStages;
-                    if (!(ok = suspended_wait_warp(&full[s], (g / kStages) & 1, fail))) break;
+                    if (!(ok = suspended_wait_warp(&full[s], (g / kStages) & 1, waits))) break;
                     tc_fence_after();
                     const uint64_t da = umma_desc_sw64(smem_u32(smem + s * kStage));
                     uint64_t* wait = kc == 0 && u > 0 ? tempty : nullptr;
                     uint64_t* done = kc == chunks - 1 ? tfull : nullptr;
-                    ok = pass == 0 ? issue_levels<kHighPlanes>(taddr, da, kc > 0, wait, done, (u - 1) & 1, leader, fail)
-                                   : issue_levels<0>(taddr, da, kc > 0, wait, done, (u - 1) & 1, leader, fail);
+                    ok = pass == 0 ? issue_levels<kHighPlanes>(taddr, da, kc > 0, wait, done, (u - 1) & 1, leader, waits)
+                                   : issue_levels<0>(taddr, da, kc > 0, wait, done, (u - 1) & 1, leader, waits);
                     if (!ok) break;
                     if (leader) umma_commit(&empty[s]);
                     __syncwarp();
@@ -406,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
             for (int pass = 0; pass < 2; ++pass) {
 #pragma unroll
                 for (int x = 0; x < 4; ++x) {
-                    if (ok) ok = suspended_wait_warp(&tfull[x], (u + pass) & 1, fail);
+                    if (ok) ok = suspended_wait_warp(&tfull[x], (u + pass) & 1, waits);
                     if (!ok) continue;
                     tc_fence_after();
 #pragma unroll
@@ -440,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
     }
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *fail) atomicMin(a.info, -1ll);
+    if (threadIdx.x == 0 && s_waits.fail) atomicMin(a.info, -1ll);
     if (warp == 0) tmem_dealloc(taddr, 512);
 }
 

@@ -21,7 +21,7 @@
 // Every sum has a fixed order (columns in order, lanes in a tree), so results are bitwise
 // reproducible.  x and r travel between chain and bulk through global memory as 16-byte
 // pairs (value, the sweep's epoch), stored and read whole: no fence, and a reader's poll
-// already has the value.  Every wait is bounded (2 s): on expiry *err = 2 and the sweep
+// already has the value.  Every wait is bounded (kWaitClk): on expiry *err = 2 and the sweep
 // winds down.
 //
 // Measured a sweep (the kernel before: one CTA a row, chain through global flags): FP64
@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t* rrdy = rbar + 1;    // chain: [2] rslot filled
     uint64_t* rfree = rrdy + 2;   // chain: [2] rslot read
     double* acc = rslot + 64 + 64;  // bulk: running right-hand sides, [slice][32]
-    __shared__ int s_fail;
-    volatile int* fail = &s_fail;
+    __shared__ Waits s_waits;
+    volatile Waits* waits = &s_waits;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned rank = cluster_rank();
@@ -142,7 +142,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_init(&rfree[i], 8);
         }
         fence_barrier_init();
-        s_fail = 0;
+        s_waits.fail = 0;
+        s_waits.limit = kWaitClk;
         if (chain) {
             mbar_arrive_expect_tx(&xbar[0], BSZ * 8);
             mbar_arrive_expect_tx(rbar, BSZ * 8);
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t n = 0;
             bool ok = true;
             auto put = [&](int t, int s, int q) {
-                if (n >= (uint32_t)S) ok = thread_wait(&empty[n % S], (n / S - 1) & 1, fail);
+                if (n >= (uint32_t)S) ok = thread_wait(&empty[n % S], (n / S - 1) & 1, waits);
                 if (ok) {
                     copy(n, t, s, q);
                     ++n;
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             // no copy may still be writing when the CTA leaves
             for (uint32_t h = n > (uint32_t)S ? n - S : 0; h < n; ++h)
-                thread_wait(&full[h % S], (h / S) & 1, fail);
+                thread_wait(&full[h % S], (h / S) & 1, waits);
         }
         __syncwarp();
     } else if (warp == 9) {
@@ -214,8 +215,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int last = (c + (own - 1) * P) / R;
             for (int s = 0; s <= last; ++s) {
                 double v[BSZ / 32];
-                if (s >= 3 && !warp_wait(&xfree[s % 3], (s / 3 - 1) & 1, fail)) break;
-                if (!warp_pairs(a.x + (size_t)s * BSZ, a.epoch, lane, fail, a.err, v)) break;
+                if (s >= 3 && !warp_wait(&xfree[s % 3], (s / 3 - 1) & 1, waits)) break;
+                if (!warp_pairs(a.x + (size_t)s * BSZ, a.epoch, lane, waits, a.err, v)) break;
 #pragma unroll
                 for (int q = 0; q < BSZ / 32; ++q) xs[(s % 3) * BSZ + lane + 32 * q] = v[q];
                 __syncwarp();
@@ -227,10 +228,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         // the first band + 1 steps
         if (chain) {
             for (int t = 0; t < nb; ++t) {
-                if (t >= 2 && !warp_wait(&rfree[t & 1], (t / 2 - 1) & 1, fail)) break;
+                if (t >= 2 && !warp_wait(&rfree[t & 1], (t / 2 - 1) & 1, waits)) break;
                 double v[1];
                 if (t > band) {
-                    if (!warp_pairs(a.r + (size_t)t * BSZ + 32 * rank, a.epoch, lane, fail, a.err, v)) break;
+                    if (!warp_pairs(a.r + (size_t)t * BSZ + 32 * rank, a.epoch, lane, waits, a.err, v)) break;
                 } else {
                     v[0] = a.in[(size_t)row_of(t) * BSZ + 32 * rank + lane];
                 }
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         T v[BSZ / 8];
         auto take = [&](auto slice) {  // the next tile into registers, its stage free again
-            ok = ok && warp_wait(&full[n % S], (n / S) & 1, fail);
+            ok = ok && warp_wait(&full[n % S], (n / S) & 1, waits);
             if (ok) decltype(slice)::load(ring + (size_t)(n % S) * C::kTile, warp, lane, v);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[n % S]);
@@ -265,19 +266,19 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int s = t > band ? t - band : 0; s < t && ok; ++s) {
                 take(Off{});
                 // x of the last step is the one still under way; those before it are known
-                if (s == t - 1) ok = ok && warp_wait(xbar, s & 1, fail);
+                if (s == t - 1) ok = ok && warp_wait(xbar, s & 1, waits);
                 if (!ok) break;
                 if (s == t - 1 && tid == 0) mbar_arrive_expect_tx(xbar, BSZ * 8);  // the next phase
                 Off::apply(v, xs + (s % (band + 1)) * BSZ, lane, s4);
             }
-            ok = ok && warp_wait(&rrdy[t & 1], (t / 2) & 1, fail);
+            ok = ok && warp_wait(&rrdy[t & 1], (t / 2) & 1, waits);
             if (!ok) break;
             const double r = rslot[(t & 1) * 32 + o] - Off::total(s4, lane);
             __syncwarp();
             if (lane == 0) mbar_arrive(&rfree[t & 1]);
             if (dst < R) st_async(r_rv, r, r_rbar);
             take(Diag{});
-            ok = ok && warp_wait(rbar, t & 1, fail);
+            ok = ok && warp_wait(rbar, t & 1, waits);
             if (!ok) break;
             if (tid == 0 && t + 1 < nb) mbar_arrive_expect_tx(rbar, BSZ * 8);
             double d4[4] = {0.0, 0.0, 0.0, 0.0};
@@ -290,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
         // every exchange has landed before this CTA leaves (bounded)
-        if (ok) warp_wait(xbar, (nb - 1) & 1, fail);
+        if (ok) warp_wait(xbar, (nb - 1) & 1, waits);
     } else if (own > 0) {
         // ---- bulk, 8 warps
         const int o = 4 * warp + (lane >> 3);
@@ -303,12 +304,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (; e < own && ok; ++e, ++n) {
                 const int g = c + e * P, t = band + 1 + g / R;
                 T v[BSZ / 8];
-                ok = warp_wait(&full[n % S], (n / S) & 1, fail);
+                ok = warp_wait(&full[n % S], (n / S) & 1, waits);
                 if (!ok) break;
                 Off::load(ring + (size_t)(n % S) * C::kTile, warp, lane, v);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[n % S]);
-                if (!have && !(ok = warp_wait(&xbar[s % 3], (s / 3) & 1, fail))) break;
+                if (!have && !(ok = warp_wait(&xbar[s % 3], (s / 3) & 1, waits))) break;
                 have = true;
                 double s4[4] = {0.0, 0.0, 0.0, 0.0};
                 Off::apply(v, xs + (s % 3) * BSZ, lane, s4);
@@ -322,13 +323,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             }
             if (!ok) break;
-            if (!have && !(ok = warp_wait(&xbar[s % 3], (s / 3) & 1, fail))) break;
+            if (!have && !(ok = warp_wait(&xbar[s % 3], (s / 3) & 1, waits))) break;
             __syncwarp();
             if (lane == 0) mbar_arrive(&xfree[s % 3]);
         }
     }
     __syncthreads();
-    if (tid == 0 && s_fail) atomicExch(a.err, 2);
+    if (tid == 0 && s_waits.fail) atomicExch(a.err, 2);
     cluster_sync_all();  // no CTA leaves while a peer may still write into its memory
 }
 

@@ -11,7 +11,14 @@ namespace {
 
 using namespace tc;
 
-constexpr long long kWaitClk = 4000000000ll;  // 2 s at 2 GHz, in SM cycles
+constexpr long long kWaitClk = 4000000000ll;  // limit of a wait in SM cycles: 2 s at 2 GHz
+
+// what the waits of a CTA share: a wait that runs out sets `fail`, and every later one returns
+// at once
+struct __align__(8) Waits {
+    int fail;
+    long long limit;  // SM cycles
+};
 
 // a value and its epoch, stored and read whole (16 bytes)
 __device__ __forceinline__ void pair_store(ulonglong2* p, double v, unsigned long long epoch) {
@@ -48,14 +55,18 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
+__device__ __forceinline__ bool out_of_time(const volatile Waits* w, long long t0) {
+    return w->fail || clock64() - t0 > w->limit;
+}
+
 // a bounded wait by one thread.  The limit counts SM cycles: reading the global nanosecond
 // timer holds up the whole SM for longer than most waits here take.
-__device__ __forceinline__ bool thread_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
+__device__ __forceinline__ bool thread_wait(uint64_t* bar, uint32_t parity, volatile Waits* w) {
     if (mbar_test(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_test(bar, parity)) {
-        if (*fail || clock64() - t0 > kWaitClk) {
-            *fail = 1;
+        if (out_of_time(w, t0)) {
+            w->fail = 1;
             return false;
         }
     }
@@ -63,23 +74,61 @@ __device__ __forceinline__ bool thread_wait(uint64_t* bar, uint32_t parity, vola
 }
 // the same for a whole warp, all lanes together: a wait by one lane leaves the warp split
 // afterwards (its code then ran six times slower until the next row)
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile Waits* w) {
     if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
     const long long t0 = clock64();
     while (!__all_sync(0xffffffffu, mbar_test(bar, parity))) {
-        if (__any_sync(0xffffffffu, *fail || clock64() - t0 > kWaitClk)) {
-            *fail = 1;
+        if (__any_sync(0xffffffffu, out_of_time(w, t0))) {
+            w->fail = 1;
+            return false;
+        }
+    }
+    return true;
+}
+// Both with the thread suspended between tries: for kernels whose tensor core reads operands
+// through the shared-memory port that polling warps would take.
+__device__ __forceinline__ bool suspended_wait(uint64_t* bar, uint32_t parity, volatile Waits* w) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait(bar, parity)) {
+        if (out_of_time(w, t0)) {
+            w->fail = 1;
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ bool suspended_wait_warp(uint64_t* bar, uint32_t parity, volatile Waits* w) {
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        if (__any_sync(0xffffffffu, out_of_time(w, t0))) {
+            w->fail = 1;
             return false;
         }
     }
     return true;
 }
 
+// a warp's bounded wait for a counter in global memory to reach `want`; what was written
+// before it was counted up is then visible to lane 0
+__device__ __forceinline__ bool warp_count(const unsigned long long* count, unsigned long long want, int lane,
+                                           volatile Waits* w) {
+    const long long t0 = clock64();
+    for (;;) {
+        unsigned long long have = 0;
+        if (lane == 0) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(have) : "l"(count) : "memory");
+        if (__shfl_sync(0xffffffffu, have, 0) >= want) return true;
+        if (__any_sync(0xffffffffu, out_of_time(w, t0))) {
+            w->fail = 1;
+            return false;
+        }
+    }
+}
+
 // lane l's pairs p[l + 32 q], q < M, once they carry the epoch; bounded as above.  While
 // they do not, only the last of each 32 is polled, and not at full rate: over a hundred CTAs
 // wait for the same vector, and polling all of it slowed the chain sixfold.
 template <int M>
-__device__ __forceinline__ bool warp_pairs(const ulonglong2* p, unsigned long long epoch, int lane, volatile int* fail,
+__device__ __forceinline__ bool warp_pairs(const ulonglong2* p, unsigned long long epoch, int lane, volatile Waits* w,
                                            int* err, double (&v)[M]) {
     const long long t0 = clock64();
     for (int n = 0;; ++n) {
@@ -90,9 +139,9 @@ __device__ __forceinline__ bool warp_pairs(const ulonglong2* p, unsigned long lo
             for (int q = 0; q < M; ++q) done &= pair_load(p + lane + 32 * q, epoch, &v[q]);
             if (__all_sync(0xffffffffu, done)) return true;
         }
-        if ((n & 63) == 63 && __any_sync(0xffffffffu, *fail || clock64() - t0 > kWaitClk ||
-                                                          *reinterpret_cast<volatile int*>(err) != 0)) {
-            *fail = 1;
+        if ((n & 63) == 63 &&
+            __any_sync(0xffffffffu, out_of_time(w, t0) || *reinterpret_cast<volatile int*>(err) != 0)) {
+            w->fail = 1;
             return false;
         }
         __nanosleep(40);

@@ -152,10 +152,14 @@ hs_status hs_potrf_block(hs_ctx ctx, double* A, int blockID, int blockRow);
  * Synchronises the stream. */
 hs_status hs_ctx_take_info(hs_ctx ctx, int64_t* info);
 /* Self-test of the failure path of every device-side wait in the library (no
- * reference counterpart): one device thread waits on a flag that nothing sets, with
- * the bounded wait the sweeps and tensor-core kernels use, for timeout_ns
- * (1e6 .. 2e9).  Returns HS_ERR_TIMEOUT when the wait ran out (the expected
- * outcome; the context stays usable), HS_OK if the flag was seen set. */
+ * reference counterpart): one warp for each kind of wait that the sweeps, CG and the
+ * tensor-core kernels use waits for something that never happens, with a limit of
+ * timeout_ns (1e6 .. 2e9; waits counted in SM cycles take 2 cycles a nanosecond, so up
+ * to 2 GHz / clock times as long; in the solvers' kernels the limit is 4e9 cycles).
+ * Returns HS_ERR_TIMEOUT when all of them ran out, every later wait then returned at
+ * once and the trailing update's mark came back from hs_ctx_take_info (the expected
+ * outcome; the context and its pivot record stay as they were); HS_OK if a wait came
+ * back as if it had been served. */
 hs_status hs_selftest_bounded_wait(hs_ctx ctx, int64_t timeout_ns);
 
 /* MatrixMatrixOperations::triangularSolve{,_optimizedGPU,_optimizedCPU}

@@ -1,0 +1,23 @@
+"""GPU: the self-test of the bounded waits reaches every kind of wait that the kernels use, and
+gives the context's pivot record back."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def test_every_kind_of_wait_runs_out(hs, ctx):
+    lib = hs._lib.load()
+    ctx.set_problem(128, 128)
+    A = torch.eye(128, dtype=torch.float64, device="cuda:0").reshape(-1)
+    A[5 * 129] = -1.0
+    ctx.take_info()
+    hs.MatrixOperations.cholesky(ctx, A, 0, 0)
+    st = lib.hs_selftest_bounded_wait(ctx.handle, 20_000_000)
+    text = lib.hs_last_error().decode()
+    assert hs._lib.STATUS_NAMES[st] == "HS_ERR_TIMEOUT", text
+    for kind in ("thread_wait", "warp_wait", "suspended_wait", "suspended_wait_warp", "warp_count", "warp_pairs",
+                 "mbar_wait_for"):
+        assert kind in text
+    assert ctx.take_info() == 5
+    assert ctx.take_info() == -1
