@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
     extern __shared__ uint8_t cg_smem[];
     double* ring = reinterpret_cast<double*>(cg_smem + ((1024u - (smem_u32(cg_smem) & 1023u)) & 1023u));
     double* red = ring + kWarps * kStages * kUnit;  // [warp][BSZ]
-    __shared__ uint64_t s_full[kWarps][kStages];
+    __shared__ uint64_t s_full[kWarps][kStages], s_read[kWarps][kStages];
     __shared__ double s_rows[kWarps][2][RW], s_part[kWarps], s_sum;
     __shared__ Waits s_waits;
     __shared__ int s_good;
@@ -113,10 +113,13 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
     }
     const bool resident = own <= kStages;  // they all stay: read once
     double* stage = ring + (size_t)warp * kStages * kUnit;
-    uint64_t* full = s_full[warp];
+    uint64_t *full = s_full[warp], *read = s_read[warp];
 
     if (lane == 0) {
-        for (int k = 0; k < kStages; ++k) mbar_init(&full[k], 1);
+        for (int k = 0; k < kStages; ++k) {
+            mbar_init(&full[k], 1);
+            mbar_init(&read[k], 1);
+        }
         fence_barrier_init();
     }
     if (tid == 0) {
@@ -226,6 +229,10 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
                     v[e + 1] = t.y;
                 }
                 __syncwarp();
+                // The stage is refilled through an mbarrier that this warp itself completes: an
+                // arrival follows the reads before it.  (Ordered by __syncwarp alone, the
+                // copy's write overtook reads still queued, once in some 10^8 units.)
+                if (lane == 0) mbar_arrive(&read[m % kStages]);
                 // v[r NC + e]: row r, the lane's column e
                 const unsigned off = u - u0;
                 const bool diag = off < UB;
@@ -239,6 +246,8 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
 #pragma unroll
                     for (int e = 0; e < NC; ++e) ca[e] = fma(v[r * NC + e], d, ca[e]);
                 }
+                // only what has been read may be overwritten
+                if (!resident && warp_wait(&read[m % kStages], (m / kStages) & 1, waits)) copy();
                 // row totals: row lane / (32 / RW)
                 const bool b4 = lane & 16, b3 = lane & 8;
                 double t;
@@ -253,10 +262,6 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
                 t += __shfl_xor_sync(0xffffffffu, t, 4);
                 t += __shfl_xor_sync(0xffffffffu, t, 2);
                 t += __shfl_xor_sync(0xffffffffu, t, 1);
-                // every lane's part has gone into the totals, so the unit has been read: only
-                // now may the copy engine overwrite it (after a mere __syncwarp its write
-                // overtook reads still queued, once in some 10^8 units)
-                if (!resident) copy();
                 if (lane % (32 / RW) == 0) {
                     const int r = lane / (32 / RW), i = j + (int)(off / UB);
                     __stcg(a.prow + ((size_t)i * (i + 1) / 2 + j) * BSZ + (off % UB) * RW + r, t);
