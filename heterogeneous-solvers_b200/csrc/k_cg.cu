@@ -153,6 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
 
     CgState st = *a.state;
     bool ok = true;
+    bool sound = true;  // no wait for a unit of this warp has run out: its copies go on
     const double* db[2] = {a.d, a.d + n};
 
     // sum over all CTAs of v (fixed order), a grid-wide barrier on the way
@@ -192,7 +193,8 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
 
     // phase A: partial sums of A v; v = r + beta d (type 0) or x (type 1).  Returns this
     // thread's part of v . A v.  A wait that runs out leaves its mark and the pass goes on
-    // to its end (later waits return at once); the next grid_sum ends the launch.
+    // to its end without further copies (later waits return at once); the next grid_sum ends
+    // the launch.
     auto matvec = [&](int type, double beta, const double* dold) -> double {
         auto val = [&](int64_t e) -> double {
             return type == 0 ? fma(beta, __ldcg(dold + e), __ldcg(a.r + e)) : __ldcg(a.x + e);
@@ -215,7 +217,8 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
             }
             for (; u < uhi; u += kWarps, ++k) {
                 const uint32_t m = resident ? (uint32_t)k : taken;
-                if (!resident || taken < (uint32_t)own) warp_wait(&full[m % kStages], (m / kStages) & 1, waits);
+                if (!resident || taken < (uint32_t)own)
+                    sound = sound && warp_wait(&full[m % kStages], (m / kStages) & 1, waits);
                 ++taken;
                 double* vr = s_rows[warp][k & 1];
                 if (lane < RW) vr[lane] = rv;
@@ -247,7 +250,8 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
                     for (int e = 0; e < NC; ++e) ca[e] = fma(v[r * NC + e], d, ca[e]);
                 }
                 // only what has been read may be overwritten
-                if (!resident && warp_wait(&read[m % kStages], (m / kStages) & 1, waits)) copy();
+                sound = sound && (resident || warp_wait(&read[m % kStages], (m / kStages) & 1, waits));
+                if (!resident && sound) copy();
                 // row totals: row lane / (32 / RW)
                 const bool b4 = lane & 16, b3 = lane & 8;
                 double t;
@@ -387,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
     }
     // no copy may still be writing when the CTA leaves
     for (uint32_t h = issued > (uint32_t)kStages ? issued - kStages : 0; h < issued; ++h)
-        warp_wait(&full[h % kStages], (h / kStages) & 1, waits);
+        landed(&full[h % kStages], (h / kStages) & 1, waits);
     __syncthreads();
     if (tid == 0 && s_waits.fail) atomicExch(a.err, 1);
 }

@@ -1,5 +1,6 @@
 // k_selftest.cu — self-test of the bounded device-side waits: every wait that the library's
-// kernels use, on something that never happens, with a short limit.  No reference counterpart.
+// kernels use, on something that never happens, with a short limit; and the wait for copies in
+// flight before a CTA leaves, after another wait has run out.  No reference counterpart.
 #include <climits>
 #include <string>
 
@@ -10,27 +11,31 @@ namespace hs {
 namespace {
 
 // one warp a wait
-enum { kThread, kWarp, kSuspended, kSuspendedWarp, kCount, kPairs, kTimer, kWaitKinds };
+enum { kThread, kWarp, kSuspended, kSuspendedWarp, kCount, kPairs, kTimer, kLanded, kWaitKinds };
 const char* const kNames[kWaitKinds] = {"thread_wait", "warp_wait",  "suspended_wait", "suspended_wait_warp",
-                                        "warp_count",  "warp_pairs", "mbar_wait_for"};
+                                        "warp_count",  "warp_pairs", "mbar_wait_for",  "landed"};
+constexpr int kCopyBytes = 16384;
 
 struct SelftestArgs {
     long long limit;                  // SM cycles
     unsigned long long limit_ns;
     const unsigned long long* count;  // zero
     const ulonglong2* pairs;          // 32, zero
+    const unsigned* source;           // kCopyBytes of 0x5a
     int* err;
     int* ran_out;                     // [wait]: 1 if it ran out, and the next one returned at once
     long long* info;                  // the trailing update's mark
 };
 
 __global__ void __launch_bounds__(32) wait_selftest_kernel(SelftestArgs a) {
-    __shared__ uint64_t bar;
+    __shared__ __align__(16) unsigned copied[kCopyBytes / 4];
+    __shared__ uint64_t bar, loaded;
     __shared__ Waits s_waits;
     volatile Waits* waits = &s_waits;
     const int lane = threadIdx.x, kind = blockIdx.x;
     if (lane == 0) {
         mbar_init(&bar, 1);  // nothing arrives
+        mbar_init(&loaded, 1);
         fence_barrier_init();
         s_waits.fail = 0;
         s_waits.limit = a.limit;
@@ -48,6 +53,22 @@ __global__ void __launch_bounds__(32) wait_selftest_kernel(SelftestArgs a) {
             default: return lane != 0 || mbar_wait_for(&bar, 0, a.limit_ns);
         }
     };
+    if (kind == kLanded) {
+        // a copy still in flight when a wait has run out is waited for all the same, and what
+        // never lands is not waited for without end
+        if (lane == 0) {
+            s_waits.fail = 1;
+            mbar_arrive_expect_tx(&loaded, kCopyBytes);
+            bulk_load(copied, a.source, kCopyBytes, &loaded);
+        }
+        __syncwarp();
+        bool in = landed(&loaded, 0, waits);
+        for (int e = lane; e < kCopyBytes / 4; e += 32) in = in && copied[e] == 0x5a5a5a5au;
+        const long long t0 = clock64();
+        in = __all_sync(0xffffffffu, in && !landed(&bar, 0, waits) && clock64() - t0 > a.limit);
+        if (lane == 0) a.ran_out[kind] = in;
+        return;
+    }
     bool out = !wait();
     __syncwarp();
     if (kind != kTimer) {
@@ -72,11 +93,13 @@ hs_status launch_bounded_wait_selftest(hs_ctx ctx, int64_t timeout_ns) {
     a.count = reinterpret_cast<unsigned long long*>(base + 256);
     a.err = reinterpret_cast<int*>(base + 512);
     a.pairs = reinterpret_cast<ulonglong2*>(base + 1024);
+    a.source = reinterpret_cast<unsigned*>(base + 4096);
     a.info = ctx->d_info;
     // the pivot record is lent to the test
     long long record = 0;
     HS_CUDA(cudaMemcpyAsync(&record, ctx->d_info, sizeof(record), cudaMemcpyDeviceToHost, s));
-    HS_CUDA(cudaMemsetAsync(base, 0, 2048, s));
+    HS_CUDA(cudaMemsetAsync(base, 0, 4096, s));
+    HS_CUDA(cudaMemsetAsync(base + 4096, 0x5a, kCopyBytes, s));
     HS_CUDA(cudaStreamSynchronize(s));
     set_i64_dev(ctx->d_info, INT64_MAX, s);
     ctx->launches += 2;

@@ -326,10 +326,7 @@ __global__ void __launch_bounds__(kThreads, 1) split_update_kernel(SplitArgs a) 
                 }
             }
             // no load may still be writing into shared memory when the CTA leaves
-            for (uint32_t h = g > kStages ? g - kStages : 0; h < g; ++h) {
-                const long long t0 = clock64();
-                while (!mbar_test(&full[h % kStages], (h / kStages) & 1) && clock64() - t0 < kWaitClk) {}
-            }
+            for (uint32_t h = g > kStages ? g - kStages : 0; h < g; ++h) landed(&full[h % kStages], (h / kStages) & 1, waits);
         }
     } else if (warp == 1) {
         const bool leader = elect_one();  // the whole warp walks the loop, so that descriptors stay in uniform registers

@@ -47,6 +47,7 @@ constexpr int kThreads = kCompute + 96;   // + copies, x in, r in
 // within that many steps (2 and 3 blocks, more for the chain to read: N=4096, bsz 128:
 // 49.5 -> 57.7 -> 66 us a sweep; N=16384, bsz 256: 184 -> 187 -> 203 us)
 constexpr int kBand = 1;
+constexpr long long kSettleClk = 100000;  // far longer than a store to another CTA of the cluster takes
 constexpr int kSlots = 3;  // x vectors kept (chain: kBand + 1, bulk: 3)
 
 struct SweepArgs {
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             // no copy may still be writing when the CTA leaves
             for (uint32_t h = n > (uint32_t)S ? n - S : 0; h < n; ++h)
-                thread_wait(&full[h % S], (h / S) & 1, waits);
+                landed(&full[h % S], (h / S) & 1, waits);
         }
         __syncwarp();
     } else if (warp == 9) {
@@ -331,6 +332,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     if (tid == 0 && s_waits.fail) atomicExch(a.err, 2);
     cluster_sync_all();  // no CTA leaves while a peer may still write into its memory
+    // after a wait ran out, peers' values may be on their way that nothing here has counted
+    if (s_waits.fail)
+        for (const long long t0 = clock64(); clock64() - t0 < kSettleClk;) {}
 }
 
 // columns of 128 bytes, all BSZ rows of a block

@@ -108,6 +108,15 @@ __device__ __forceinline__ bool suspended_wait_warp(uint64_t* bar, uint32_t pari
     return true;
 }
 
+// Before a CTA leaves: waits until a copy in flight has landed, also after another wait has run
+// out (then above all: the shared memory goes to the next CTA).  Bounded by itself.
+__device__ __forceinline__ bool landed(uint64_t* bar, uint32_t parity, const volatile Waits* w) {
+    const long long t0 = clock64();
+    while (!mbar_test(bar, parity))
+        if (clock64() - t0 > w->limit) return false;
+    return true;
+}
+
 // a warp's bounded wait for a counter in global memory to reach `want`; what was written
 // before it was counted up is then visible to lane 0
 __device__ __forceinline__ bool warp_count(const unsigned long long* count, unsigned long long want, int lane,

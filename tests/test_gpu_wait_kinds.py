@@ -21,3 +21,12 @@ def test_every_kind_of_wait_runs_out(hs, ctx):
         assert kind in text
     assert ctx.take_info() == 5
     assert ctx.take_info() == -1
+
+
+def test_copies_in_flight_are_waited_for_after_an_expiry(hs, ctx):
+    """A CTA that gives up must not leave while a copy still writes its shared memory: the wait
+    for it ignores the failure mark, and has a limit of its own."""
+    lib = hs._lib.load()
+    ctx.set_problem(128, 128)
+    assert hs._lib.STATUS_NAMES[lib.hs_selftest_bounded_wait(ctx.handle, 5_000_000)] == "HS_ERR_TIMEOUT"
+    assert "landed" in lib.hs_last_error().decode()
