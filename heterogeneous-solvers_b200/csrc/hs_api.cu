@@ -2,6 +2,7 @@
 // validation and the operator-level entry points of include/hs_b200.h.
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 
 #include "hs_internal.cuh"
@@ -30,6 +31,62 @@ hs_status require_ctx(hs_ctx ctx, const char* fn) {
     cudaError_t e = cudaSetDevice(ctx->device);
     if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
     return HS_OK;
+}
+
+namespace {
+struct DeviceTurns {
+    std::mutex m;
+    cudaEvent_t last = nullptr;  // recorded behind the last turn
+    int contexts = 0;
+};
+constexpr int kMaxDevices = 64;
+DeviceTurns g_turns[kMaxDevices];
+}  // namespace
+
+hs_status turns_join(int dev) {
+    HS_REQUIRE(dev >= 0 && dev < kMaxDevices, "device index out of range");
+    DeviceTurns& d = g_turns[dev];
+    std::lock_guard<std::mutex> lock(d.m);
+    if (d.contexts == 0) HS_CUDA(cudaEventCreateWithFlags(&d.last, cudaEventDisableTiming));
+    ++d.contexts;
+    return HS_OK;
+}
+
+void turns_leave(int dev) {
+    DeviceTurns& d = g_turns[dev];
+    std::lock_guard<std::mutex> lock(d.m);
+    if (--d.contexts == 0) {
+        cudaEventDestroy(d.last);
+        d.last = nullptr;
+    }
+}
+
+hs_status turn_mark(hs_ctx ctx, cudaStream_t s) {
+    DeviceTurns& d = g_turns[ctx->device];
+    {
+        std::lock_guard<std::mutex> lock(d.m);
+        ctx->turn_wait = d.contexts > 1;
+    }
+    if (ctx->turn_wait) HS_CUDA(cudaEventRecord(ctx->ev_turn, s));
+    return HS_OK;
+}
+
+hs_status turn_ready(hs_ctx ctx) {
+    if (ctx->turn_wait) HS_CUDA(cudaEventSynchronize(ctx->ev_turn));
+    return HS_OK;
+}
+
+Turn::Turn(hs_ctx ctx, cudaStream_t s) : dev_(ctx->device), s_(s) {
+    DeviceTurns& d = g_turns[dev_];
+    d.m.lock();
+    const cudaError_t e = cudaStreamWaitEvent(s, d.last, 0);
+    status = e == cudaSuccess ? HS_OK : cuda_fail(e, "the turns of kernels whose CTAs wait for one another");
+}
+
+Turn::~Turn() {
+    DeviceTurns& d = g_turns[dev_];
+    if (status == HS_OK) cudaEventRecord(d.last, s_);
+    d.m.unlock();
 }
 
 hs_status ensure_scratch(hs_ctx ctx, size_t bytes) {
@@ -232,11 +289,14 @@ hs_status hs_ctx_create(int device, void* stream, hs_ctx* out) {
     }
     HS_CUDA(cudaEventCreateWithFlags(&ctx->ev_a, cudaEventDisableTiming));
     HS_CUDA(cudaEventCreateWithFlags(&ctx->ev_b, cudaEventDisableTiming));
+    HS_CUDA(cudaEventCreateWithFlags(&ctx->ev_turn, cudaEventDisableTiming));
     HS_CUDA(cudaMalloc(&ctx->d_info, 2 * sizeof(long long)));
     HS_CUDA(cudaMallocHost(&ctx->h_pinned, 64 * sizeof(double)));
     set_i64_kernel<<<1, 1, 0, ctx->stream>>>(ctx->d_info, INT64_MAX);
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaStreamSynchronize(ctx->stream));
+    hs_status st = turns_join(device);
+    if (st != HS_OK) return st;
     *out = ctx;
     return HS_OK;
 }
@@ -245,6 +305,7 @@ hs_status hs_ctx_destroy(hs_ctx ctx) {
     if (!ctx) return HS_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    turns_leave(ctx->device);
     if (ctx->side) {
         cudaStreamSynchronize(ctx->side);
         cudaStreamDestroy(ctx->side);
@@ -255,6 +316,7 @@ hs_status hs_ctx_destroy(hs_ctx ctx) {
     }
     if (ctx->ev_a) cudaEventDestroy(ctx->ev_a);
     if (ctx->ev_b) cudaEventDestroy(ctx->ev_b);
+    if (ctx->ev_turn) cudaEventDestroy(ctx->ev_turn);
     for (auto& r : ctx->prof_pending) {
         cudaEventDestroy(r.start);
         cudaEventDestroy(r.stop);

@@ -52,6 +52,8 @@ struct hs_ctx_s {
     // takes SMs ahead of the trailing update's CTAs)
     cudaStream_t side_hi = nullptr;
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
+    cudaEvent_t ev_turn = nullptr;  // turn_mark's, while turn_wait
+    bool turn_wait = false;
 
     // > 0: matvec, dot and vector updates follow the reference CPU path's exact
     // accumulation order (separate multiply and add, dot products in this many
@@ -121,6 +123,35 @@ hs_status ensure_mixed(hs_ctx ctx, size_t bytes);
 hs_status ensure_gp(hs_ctx ctx, size_t bytes);
 hs_status ensure_hostws(hs_ctx ctx, size_t bytes);
 hs_status ensure_solvews(hs_ctx ctx, size_t bytes);
+
+// The CTAs of a sweep or of the persistent CG wait for one another.  Such a launch fits the
+// device alone, but two of them in different streams could each hold SMs that the other waits
+// for.  So they take turns on a device: each waits for the event of the one before it.  (A
+// cooperative launch would order the sweeps; together with clusters it cannot be launched under
+// a profiler, and it would not order them with CG's cooperative launch by any documented
+// rule.)
+class Turn {
+  public:
+    Turn(hs_ctx ctx, cudaStream_t s);  // `s` waits for the turn; hs_status in `status`
+    ~Turn();                           // the turn passes on once what was launched meanwhile is done
+    Turn(const Turn&) = delete;
+    Turn& operator=(const Turn&) = delete;
+    hs_status status;
+
+  private:
+    int dev_;
+    cudaStream_t s_;
+};
+// A turn that is queued behind a long factor would hold up those of every other stream until the
+// factor is done.  So with several contexts on the device the host waits, before it takes a
+// turn, for what was queued before turn_mark; short work may be queued in between (a solve's
+// inverse diagonal blocks: a wait for these as well costs N=16384 6 of 480 us).  With one
+// context there is no other stream to hold up, and both return at once.
+hs_status turn_mark(hs_ctx ctx, cudaStream_t s);
+hs_status turn_ready(hs_ctx ctx);
+// the contexts of a device: the first one makes its turns' event, the last one takes it away
+hs_status turns_join(int dev);
+void turns_leave(int dev);
 
 // scratch layout: [0, 32 KB) reduction partials, [32 KB, 48 KB) solver scalars,
 // [56 KB, 64 KB) small constants; matvec partial blocks start at 64 KB
@@ -261,7 +292,7 @@ hs_status launch_diag_inverses(hs_ctx ctx, const double* L, double* Y, double* T
 // a whole forward (out = L^-1 in) or backward (out = L^-T in) sweep over a packed factor in
 // one launch, given Y_k = L_kk^-T (k_sweep.cu; out must not be in).  ws: workspace whose
 // flags sweep_reset has cleared; epoch: a value no sweep since has used; *err = 2 on a
-// wait that ran out
+// wait that ran out.  The caller holds a Turn
 size_t sweep_workspace_bytes(int nb, int bsz);
 hs_status sweep_reset(hs_ctx ctx, void* ws, cudaStream_t s);
 hs_status launch_sweep_f64(hs_ctx ctx, const double* L, const double* Y, const double* in, double* out, int forward,

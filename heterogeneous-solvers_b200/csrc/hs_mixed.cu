@@ -142,6 +142,9 @@ int grid_n(int64_t n, int sms) {
 // reads b and writes L^-1 b into tmp; the backward sweep reads tmp and writes the
 // result into b.
 hs_status mixed_apply(hs_ctx ctx, MixedWork& w, double* b, double* tmp, cudaStream_t s) {
+    // (the solve has waited for its factor on the host: nothing long is queued before this)
+    Turn turn(ctx, s);
+    if (turn.status != HS_OK) return turn.status;
     hs_status st = launch_sweep_f32(ctx, w.A32, w.Y32, b, tmp, 1, ++w.epoch, w.sweep, w.err + 1, s);
     if (st != HS_OK) return st;
     return launch_sweep_f32(ctx, w.A32, w.Y32, tmp, b, 0, ++w.epoch, w.sweep, w.err + 1, s);

@@ -223,11 +223,17 @@ hs_status solve_driver(hs_ctx ctx, const double* L, double* b) {
         double* tmp = T + tq;
         int* err = reinterpret_cast<int*>(static_cast<char*>(ctx->solvews) + ybytes);
         void* ws = static_cast<char*>(ctx->solvews) + ybytes + 256;
+        if ((st = turn_mark(ctx, s)) != HS_OK) return st;
         if ((st = launch_diag_inverses(ctx, L, Y, T, s)) != HS_OK) return st;
         if ((st = sweep_reset(ctx, ws, s)) != HS_OK) return st;
         HS_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-        if ((st = launch_sweep_f64(ctx, L, Y, b, tmp, 1, 1u, ws, err, s)) != HS_OK) return st;
-        if ((st = launch_sweep_f64(ctx, L, Y, tmp, b, 0, 2u, ws, err, s)) != HS_OK) return st;
+        if ((st = turn_ready(ctx)) != HS_OK) return st;
+        {
+            Turn turn(ctx, s);
+            if (turn.status != HS_OK) return turn.status;
+            if ((st = launch_sweep_f64(ctx, L, Y, b, tmp, 1, 1u, ws, err, s)) != HS_OK) return st;
+            if ((st = launch_sweep_f64(ctx, L, Y, tmp, b, 0, 2u, ws, err, s)) != HS_OK) return st;
+        }
         int h_err = 0;
         HS_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
         HS_CUDA(cudaStreamSynchronize(s));

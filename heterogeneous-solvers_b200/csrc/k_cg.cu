@@ -405,6 +405,8 @@ hs_status run(hs_ctx ctx, CgArgs a, int grid, cudaStream_t s) {
     }
     void* args[] = {&a};
     ctx->launches += 1;
+    Turn turn(ctx, s);
+    if (turn.status != HS_OK) return turn.status;
     // cooperative: the CTAs wait for one another
     HS_CUDA(cudaLaunchCooperativeKernel((const void*)cg_kernel<BSZ>, dim3(grid), dim3(kThreads), args,
                                         cg_smem_bytes<BSZ>(), s));
@@ -442,6 +444,7 @@ hs_status cg_persistent(hs_ctx ctx, const double* A, const double* b, double* x,
     a.count = reinterpret_cast<unsigned long long*>(a.state + 1) + 16;  // a line of its own
     a.nb = nb;
     a.eps2 = eps * eps;
+    if ((st = turn_mark(ctx, s)) != HS_OK || (st = turn_ready(ctx)) != HS_OK) return st;
     HS_CUDA(cudaMemsetAsync(x, 0, n * sizeof(double), s));
     HS_CUDA(cudaMemsetAsync(a.d, 0, 2 * n * sizeof(double), s));
     HS_CUDA(cudaMemsetAsync(a.parts, 0, 2 * (size_t)grid * sizeof(double) + 512, s));

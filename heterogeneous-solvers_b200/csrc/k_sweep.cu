@@ -32,8 +32,6 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
-#include <mutex>
-
 #include "hs_internal.cuh"
 #include "hs_mixed.cuh"
 #include "stream_common.cuh"
@@ -358,41 +356,6 @@ hs_status cols_map(CUtensorMap* m, const T* base, int bsz, int64_t blocks) {
     return HS_OK;
 }
 
-// The CTAs of a sweep wait for one another and fit the device together, but two sweeps of
-// different streams could each hold a part of the SMs that the other waits for.  So the
-// sweeps of a device take turns: each waits for the event of the one before it.  (A
-// cooperative launch would do the same; together with clusters the profiler cannot launch
-// it.)
-class SweepTurn {
-  public:
-    SweepTurn(int dev, cudaStream_t s) : lock_(mutex()[dev]), slot_(&events()[dev]), s_(s) {
-        cudaError_t e = cudaSuccess;
-        if (!*slot_)
-            e = cudaEventCreateWithFlags(slot_, cudaEventDisableTiming);
-        else
-            e = cudaStreamWaitEvent(s, *slot_, 0);
-        status = e == cudaSuccess ? HS_OK : cuda_fail(e, "the turns of the sweeps");
-    }
-    hs_status taken() {
-        const cudaError_t e = cudaEventRecord(*slot_, s_);
-        return e == cudaSuccess ? HS_OK : cuda_fail(e, "the turns of the sweeps");
-    }
-    hs_status status;
-
-  private:
-    static std::mutex* mutex() {
-        static std::mutex m[64];
-        return m;
-    }
-    static cudaEvent_t* events() {  // one a device, for the life of the process
-        static cudaEvent_t e[64] = {};
-        return e;
-    }
-    std::lock_guard<std::mutex> lock_;
-    cudaEvent_t* slot_;
-    cudaStream_t s_;
-};
-
 template <int BSZ, typename T, bool FWD>
 hs_status launch_dir(hs_ctx ctx, const T* L, const T* Y, const double* in, double* out, unsigned epoch, void* ws,
                      int* err, cudaStream_t s) {
@@ -444,12 +407,7 @@ hs_status launch_dir(hs_ctx ctx, const T* L, const T* Y, const double* in, doubl
     HS_REQUIRE(cfg.dynamicSmemBytes <= kMaxSmem, "matrix too large for the single-launch sweep");
     prof_begin(ctx, s, HS_KERNEL_COLUPD);
     ctx->launches += 1;
-    {
-        SweepTurn turn(dev, s);
-        if (turn.status != HS_OK) return turn.status;
-        HS_CUDA(cudaLaunchKernelEx(&cfg, fn, m, a));
-        if ((st = turn.taken()) != HS_OK) return st;
-    }
+    HS_CUDA(cudaLaunchKernelEx(&cfg, fn, m, a));
     const double Tb = (double)nb * (nb - 1) / 2.0;
     prof_end(ctx, s, HS_KERNEL_COLUPD, 2.0 * (Tb + nb) * BSZ * BSZ, (Tb + nb) * sizeof(T) * BSZ * BSZ);
     return HS_OK;
