@@ -11,9 +11,10 @@ namespace hs {
 namespace {
 
 // one warp a wait
-enum { kThread, kWarp, kSuspended, kSuspendedWarp, kCount, kPairs, kTimer, kLanded, kWaitKinds };
+enum { kThread, kWarp, kSuspended, kSuspendedWarp, kCount, kPairs, kTimer, kLanded, kAbsent, kResident, kWaitKinds };
 const char* const kNames[kWaitKinds] = {"thread_wait", "warp_wait",  "suspended_wait", "suspended_wait_warp",
-                                        "warp_count",  "warp_pairs", "mbar_wait_for",  "landed"};
+                                        "warp_count",  "warp_pairs", "mbar_wait_for",  "landed",
+                                        "warp_wait with absent CTAs", "warp_wait with all CTAs"};
 constexpr int kCopyBytes = 16384;
 
 struct SelftestArgs {
@@ -30,7 +31,7 @@ struct SelftestArgs {
 __global__ void __launch_bounds__(32) wait_selftest_kernel(SelftestArgs a) {
     __shared__ __align__(16) unsigned copied[kCopyBytes / 4];
     __shared__ uint64_t bar, loaded;
-    __shared__ Waits s_waits;
+    __shared__ ResidentWaits s_waits;
     volatile Waits* waits = &s_waits;
     const int lane = threadIdx.x, kind = blockIdx.x;
     if (lane == 0) {
@@ -38,7 +39,9 @@ __global__ void __launch_bounds__(32) wait_selftest_kernel(SelftestArgs a) {
         mbar_init(&loaded, 1);
         fence_barrier_init();
         s_waits.fail = 0;
-        s_waits.limit = a.limit;
+        s_waits.limit = kind < kAbsent ? a.limit : a.limit / (kAbsentLimits + 1);
+        s_waits.resident = reinterpret_cast<const unsigned*>(a.count);  // zero
+        s_waits.ctas = kind == kAbsent ? 1 : 0;
     }
     __syncwarp();
     auto wait = [&]() -> bool {
@@ -67,6 +70,15 @@ __global__ void __launch_bounds__(32) wait_selftest_kernel(SelftestArgs a) {
         const long long t0 = clock64();
         in = __all_sync(0xffffffffu, in && !landed(&bar, 0, waits) && clock64() - t0 > a.limit);
         if (lane == 0) a.ran_out[kind] = in;
+        return;
+    }
+    if (kind >= kAbsent) {
+        // the limit again and again for CTAs that are absent, once more when all are there
+        const long long t0 = clock64();
+        bool out = !warp_wait(&bar, 0, static_cast<volatile ResidentWaits*>(&s_waits));
+        const long long limits = (clock64() - t0) / s_waits.limit;
+        out = out && (kind == kAbsent ? limits > kAbsentLimits : limits >= 2 && limits < kAbsentLimits / 2);
+        if (lane == 0) a.ran_out[kind] = out;
         return;
     }
     bool out = !wait();

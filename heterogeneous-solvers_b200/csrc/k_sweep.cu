@@ -21,7 +21,7 @@
 // Every sum has a fixed order (columns in order, lanes in a tree), so results are bitwise
 // reproducible.  x and r travel between chain and bulk through global memory as 16-byte
 // pairs (value, the sweep's epoch), stored and read whole: no fence, and a reader's poll
-// already has the value.  Every wait is bounded (kWaitClk): on expiry *err = 2 and the sweep
+// already has the value.  Every wait is bounded (kWaitClk from when all CTAs are resident): on expiry *err = 2 and the sweep
 // winds down.
 //
 // Measured a sweep (the kernel before: one CTA a row, chain through global flags): FP64
@@ -56,6 +56,7 @@ struct SweepArgs {
     ulonglong2* x;  // nb BSZ pairs: x from the chain to the bulk CTAs
     ulonglong2* r;  // nb BSZ pairs: right-hand sides from the bulk CTAs to the chain
     int* err;
+    unsigned* resident;  // two counters of resident CTAs, by the epoch's parity
     int nb;
     unsigned long long epoch;
 };
@@ -113,8 +114,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t* rrdy = rbar + 1;    // chain: [2] rslot filled
     uint64_t* rfree = rrdy + 2;   // chain: [2] rslot read
     double* acc = rslot + 64 + 64;  // bulk: running right-hand sides, [slice][32]
-    __shared__ Waits s_waits;
-    volatile Waits* waits = &s_waits;
+    __shared__ ResidentWaits s_waits;
+    volatile ResidentWaits* waits = &s_waits;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned rank = cluster_rank();
@@ -143,6 +144,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         fence_barrier_init();
         s_waits.fail = 0;
         s_waits.limit = kWaitClk;
+        s_waits.resident = a.resident + (a.epoch & 1);
+        s_waits.ctas = (int)gridDim.x;
         if (chain) {
             mbar_arrive_expect_tx(&xbar[0], BSZ * 8);
             mbar_arrive_expect_tx(rbar, BSZ * 8);
@@ -159,6 +162,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     __syncthreads();
     cluster_sync_all();  // every CTA's barriers are set up
+    // the CTAs count themselves in (after the barrier, whose release would wait for it); the next
+    // sweep's counter starts at zero
+    if (tid == kThreads - 1) {
+        atomicAdd(a.resident + (a.epoch & 1), 1u);
+        if (blockIdx.x == 0) a.resident[~a.epoch & 1] = 0;
+    }
 
     // the slice `q` of the off-diagonal block of (step t, step s < t), or of Y of step t
     auto copy = [&](uint32_t n, int t, int s, int q) {
@@ -369,6 +378,7 @@ hs_status launch_dir(hs_ctx ctx, const T* L, const T* Y, const double* in, doubl
     a.x = static_cast<ulonglong2*>(ws);
     a.r = a.x + (size_t)nb * BSZ;
     a.err = err;
+    a.resident = reinterpret_cast<unsigned*>(a.r + (size_t)nb * BSZ);
     a.nb = nb;
     a.epoch = epoch;
     CUtensorMap m;
@@ -427,7 +437,9 @@ hs_status launch_sweep(hs_ctx ctx, const T* L, const T* Y, const double* in, dou
 
 }  // namespace
 
-size_t sweep_workspace_bytes(int nb, int bsz) { return (size_t)2 * nb * bsz * sizeof(ulonglong2); }
+size_t sweep_workspace_bytes(int nb, int bsz) {
+    return (size_t)2 * nb * bsz * sizeof(ulonglong2) + 256;  // pairs, CTA counters
+}
 
 hs_status sweep_reset(hs_ctx ctx, void* ws, cudaStream_t s) {
     HS_CUDA(cudaMemsetAsync(ws, 0, sweep_workspace_bytes(ctx->nb, ctx->bsz), s));

@@ -19,6 +19,12 @@ struct __align__(8) Waits {
     int fail;
     long long limit;  // SM cycles
 };
+// the same where the launch's CTAs need not be resident together from the start
+struct __align__(8) ResidentWaits : Waits {
+    int ctas;                  // of the launch
+    const unsigned* resident;  // those counted in
+};
+constexpr int kAbsentLimits = 30;
 
 // a value and its epoch, stored and read whole (16 bytes)
 __device__ __forceinline__ void pair_store(ulonglong2* p, double v, unsigned long long epoch) {
@@ -55,52 +61,75 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-__device__ __forceinline__ bool out_of_time(const volatile Waits* w, long long t0) {
+__device__ __forceinline__ bool out_of_time(const volatile Waits* w, long long& t0, int&) {
     return w->fail || clock64() - t0 > w->limit;
 }
+// The limit is meant for CTAs that run: while some of the launch are not resident, because other
+// streams' kernels hold the SMs, it starts again (kAbsentLimits times at most), and once more
+// when all are.  `again`: how often so far; the result: the next, or -1.
+__device__ __noinline__ int begin_again(const volatile ResidentWaits* w, int again) {
+    if (again == kAbsentLimits) return -1;
+    return *reinterpret_cast<const volatile unsigned*>(w->resident) >= (unsigned)w->ctas ? kAbsentLimits : again + 1;
+}
+__device__ __forceinline__ bool out_of_time(const volatile ResidentWaits* w, long long& t0, int& again) {
+    if (w->fail) return true;
+    if (clock64() - t0 <= w->limit) return false;
+    again = begin_again(w, again);
+    t0 = clock64();
+    return again < 0;
+}
 
+constexpr int kTries = 16;  // between looks at the time, which would take longer than a try
 // a bounded wait by one thread.  The limit counts SM cycles: reading the global nanosecond
 // timer holds up the whole SM for longer than most waits here take.
-__device__ __forceinline__ bool thread_wait(uint64_t* bar, uint32_t parity, volatile Waits* w) {
+template <class W>
+__device__ __forceinline__ bool thread_wait(uint64_t* bar, uint32_t parity, volatile W* w) {
     if (mbar_test(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_test(bar, parity)) {
-        if (out_of_time(w, t0)) {
+    long long t0 = clock64();
+    int again = 0;
+    for (unsigned n = 1;; ++n) {
+        if (mbar_test(bar, parity)) return true;
+        if (n % kTries == 0 && out_of_time(w, t0, again)) {
             w->fail = 1;
             return false;
         }
     }
-    return true;
 }
 // the same for a whole warp, all lanes together: a wait by one lane leaves the warp split
 // afterwards (its code then ran six times slower until the next row)
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile Waits* w) {
+template <class W>
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile W* w) {
     if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
-    const long long t0 = clock64();
-    while (!__all_sync(0xffffffffu, mbar_test(bar, parity))) {
-        if (__any_sync(0xffffffffu, out_of_time(w, t0))) {
+    long long t0 = clock64();
+    int again = 0;
+    for (unsigned n = 1;; ++n) {
+        if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+        if (n % kTries == 0 && __any_sync(0xffffffffu, out_of_time(w, t0, again))) {
             w->fail = 1;
             return false;
         }
     }
-    return true;
 }
 // Both with the thread suspended between tries: for kernels whose tensor core reads operands
 // through the shared-memory port that polling warps would take.
-__device__ __forceinline__ bool suspended_wait(uint64_t* bar, uint32_t parity, volatile Waits* w) {
-    const long long t0 = clock64();
+template <class W>
+__device__ __forceinline__ bool suspended_wait(uint64_t* bar, uint32_t parity, volatile W* w) {
+    long long t0 = clock64();
+    int again = 0;
     while (!mbar_try_wait(bar, parity)) {
-        if (out_of_time(w, t0)) {
+        if (out_of_time(w, t0, again)) {
             w->fail = 1;
             return false;
         }
     }
     return true;
 }
-__device__ __forceinline__ bool suspended_wait_warp(uint64_t* bar, uint32_t parity, volatile Waits* w) {
-    const long long t0 = clock64();
+template <class W>
+__device__ __forceinline__ bool suspended_wait_warp(uint64_t* bar, uint32_t parity, volatile W* w) {
+    long long t0 = clock64();
+    int again = 0;
     while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
-        if (__any_sync(0xffffffffu, out_of_time(w, t0))) {
+        if (__any_sync(0xffffffffu, out_of_time(w, t0, again))) {
             w->fail = 1;
             return false;
         }
@@ -119,14 +148,16 @@ __device__ __forceinline__ bool landed(uint64_t* bar, uint32_t parity, const vol
 
 // a warp's bounded wait for a counter in global memory to reach `want`; what was written
 // before it was counted up is then visible to lane 0
+template <class W>
 __device__ __forceinline__ bool warp_count(const unsigned long long* count, unsigned long long want, int lane,
-                                           volatile Waits* w) {
-    const long long t0 = clock64();
+                                           volatile W* w) {
+    long long t0 = clock64();
+    int again = 0;
     for (;;) {
         unsigned long long have = 0;
         if (lane == 0) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(have) : "l"(count) : "memory");
         if (__shfl_sync(0xffffffffu, have, 0) >= want) return true;
-        if (__any_sync(0xffffffffu, out_of_time(w, t0))) {
+        if (__any_sync(0xffffffffu, out_of_time(w, t0, again))) {
             w->fail = 1;
             return false;
         }
@@ -136,10 +167,11 @@ __device__ __forceinline__ bool warp_count(const unsigned long long* count, unsi
 // lane l's pairs p[l + 32 q], q < M, once they carry the epoch; bounded as above.  While
 // they do not, only the last of each 32 is polled, and not at full rate: over a hundred CTAs
 // wait for the same vector, and polling all of it slowed the chain sixfold.
-template <int M>
-__device__ __forceinline__ bool warp_pairs(const ulonglong2* p, unsigned long long epoch, int lane, volatile Waits* w,
+template <int M, class W>
+__device__ __forceinline__ bool warp_pairs(const ulonglong2* p, unsigned long long epoch, int lane, volatile W* w,
                                            int* err, double (&v)[M]) {
-    const long long t0 = clock64();
+    long long t0 = clock64();
+    int again = 0;
     for (int n = 0;; ++n) {
         double one;
         bool done = lane >= M || pair_load(p + 32 * (lane % M) + 31, epoch, &one);
@@ -149,7 +181,7 @@ __device__ __forceinline__ bool warp_pairs(const ulonglong2* p, unsigned long lo
             if (__all_sync(0xffffffffu, done)) return true;
         }
         if ((n & 63) == 63 &&
-            __any_sync(0xffffffffu, out_of_time(w, t0) || *reinterpret_cast<volatile int*>(err) != 0)) {
+            __any_sync(0xffffffffu, out_of_time(w, t0, again) || *reinterpret_cast<volatile int*>(err) != 0)) {
             w->fail = 1;
             return false;
         }

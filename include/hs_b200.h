@@ -155,7 +155,8 @@ hs_status hs_ctx_take_info(hs_ctx ctx, int64_t* info);
  * reference counterpart): one warp for each kind of wait that the sweeps, CG and the
  * tensor-core kernels use waits for something that never happens, with a limit of
  * timeout_ns (1e6 .. 2e9; waits counted in SM cycles take 2 cycles a nanosecond, so up
- * to 2 GHz / clock times as long; in the solvers' kernels the limit is 4e9 cycles).
+ * to 2 GHz / clock times as long; in the solvers' kernels the limit is 4e9 cycles, in the
+ * sweeps from when all CTAs of the launch are resident).
  * Returns HS_ERR_TIMEOUT when all of them ran out, every later wait then returned at
  * once and the trailing update's mark came back from hs_ctx_take_info (the expected
  * outcome; the context and its pivot record stay as they were); HS_OK if a wait came

@@ -30,3 +30,13 @@ def test_copies_in_flight_are_waited_for_after_an_expiry(hs, ctx):
     ctx.set_problem(128, 128)
     assert hs._lib.STATUS_NAMES[lib.hs_selftest_bounded_wait(ctx.handle, 5_000_000)] == "HS_ERR_TIMEOUT"
     assert "landed" in lib.hs_last_error().decode()
+
+
+def test_limit_counts_from_when_every_cta_is_resident(hs, ctx):
+    """A sweep is no cooperative launch: while other streams' kernels hold SMs that it still
+    needs, its CTAs wait on; once all are resident the limit counts."""
+    lib = hs._lib.load()
+    ctx.set_problem(128, 128)
+    assert hs._lib.STATUS_NAMES[lib.hs_selftest_bounded_wait(ctx.handle, 100_000_000)] == "HS_ERR_TIMEOUT"
+    text = lib.hs_last_error().decode()
+    assert "absent CTAs" in text and "all CTAs" in text
