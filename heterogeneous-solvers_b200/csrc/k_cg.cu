@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
         const int len = (int)(seg_hi(j) - seg_lo(j));
         own += len > warp ? (len - warp + kWarps - 1) / kWarps : 0;
     }
-    const bool resident = own <= kStages;  // they all stay: read once
+    // copies go on (else the units all stay and are read once, or a wait for one has run out)
+    bool streaming = own > kStages;
     double* stage = ring + (size_t)warp * kStages * kUnit;
     uint64_t *full = s_full[warp], *read = s_read[warp];
 
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
         s_waits.limit = kWaitClk;
     }
     __syncthreads();
-    uint32_t issued = 0, taken = 0;
+    uint32_t issued = 0, m = 0;  // this warp's copies, and the next of them to be used
     // the unit of the next copy: the warp's units round and round
     int pj = ja;
     unsigned pu = lo + warp, phi = seg_hi(ja);
@@ -153,7 +154,6 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
 
     CgState st = *a.state;
     bool ok = true;
-    bool sound = true;  // no wait for a unit of this warp has run out: its copies go on
     const double* db[2] = {a.d, a.d + n};
 
     // sum over all CTAs of v (fixed order), a grid-wide barrier on the way
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
             return type == 0 ? fma(beta, __ldcg(dold + e), __ldcg(a.r + e)) : __ldcg(a.x + e);
         };
         double dq = 0.0;
-        int k = 0;  // this warp's units so far
+        if (!streaming) m = 0;  // the units are where they were
         for (int j = ja; j <= jb; ++j) {
             const unsigned u0 = column_unit(j), uhi = seg_hi(j);
             // the rows of v of a unit, read one unit ahead
@@ -215,12 +215,9 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
                 ca[e] = 0.0;
                 xj[e] = val((int64_t)j * BSZ + (e / 2 * 32 + lane) * 2 + (e & 1));
             }
-            for (; u < uhi; u += kWarps, ++k) {
-                const uint32_t m = resident ? (uint32_t)k : taken;
-                if (!resident || taken < (uint32_t)own)
-                    sound = sound && warp_wait(&full[m % kStages], (m / kStages) & 1, waits);
-                ++taken;
-                double* vr = s_rows[warp][k & 1];
+            for (; u < uhi; u += kWarps, ++m) {
+                streaming &= warp_wait(&full[m % kStages], (m / kStages) & 1, waits);
+                double* vr = s_rows[warp][m & 1];
                 if (lane < RW) vr[lane] = rv;
                 rv = rows(u + kWarps);
                 double v[RW * NC];
@@ -250,8 +247,10 @@ __global__ void __launch_bounds__(kThreads, 1) cg_kernel(CgArgs a) {
                     for (int e = 0; e < NC; ++e) ca[e] = fma(v[r * NC + e], d, ca[e]);
                 }
                 // only what has been read may be overwritten
-                sound = sound && (resident || warp_wait(&read[m % kStages], (m / kStages) & 1, waits));
-                if (!resident && sound) copy();
+                if (streaming) {
+                    streaming = warp_wait(&read[m % kStages], (m / kStages) & 1, waits);
+                    if (streaming) copy();
+                }
                 // row totals: row lane / (32 / RW)
                 const bool b4 = lane & 16, b3 = lane & 8;
                 double t;
