@@ -264,7 +264,7 @@ struct DiagFactor {
     double* L = nullptr;           // factor out
     int in_place = 0;              // L is the packed matrix's own block: zeros above the diagonal, padding rows kept
     int zeros = 1;                 // in place: also the zeros above the 32 x 32 diagonal blocks (0: the panel TRSM's)
-    double* Y = nullptr;           // L^-T, row major
+    double* Y = nullptr;           // L^-T, row major (in place with zeros: null for the factor alone, no scratch)
     int y_full = 0;                // Y: every zero below the diagonal (else those of its 64 x 64 diagonal blocks)
     double* T = nullptr;           // bsz 256: 128 x 128 doubles of scratch
     float *invHi = nullptr, *invLo = nullptr;  // L^-1 in FP32 and its low part under TF32
@@ -274,7 +274,7 @@ struct DiagFactor {
     int ctas = 8;                  // bsz 256: CTAs (one cluster) that share its products
 };
 hs_status launch_diag_factor(hs_ctx ctx, const DiagFactor& f, cudaStream_t s);
-// the factor's and the operators' form: in place, Y and T in the context's scratch
+// the factor's form: in place, Y and T in the context's scratch
 // (kDiagScratchBlocks blocks from kSmallScratch: Y, then T)
 constexpr size_t kDiagScratchBlocks = 2;
 inline DiagFactor diag_factor_in_place(hs_ctx ctx, double* blk) {

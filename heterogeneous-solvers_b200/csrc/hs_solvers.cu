@@ -92,7 +92,7 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
     const int64_t T = total_blocks(nb);
     cudaStream_t s = ctx->stream;
     auto diag_id = [&](int k) { return (int)(T - (int64_t)(nb - k) * (nb - k + 1) / 2); };
-    if ((bsz != 128 && bsz != 256) || !ctx->side_hi) {
+    if ((bsz != 128 && bsz != 256) || !ctx->side_hi || nb == 1) {
         for (int k = 0; k < nb; ++k) {
             const int blockID = diag_id(k);
             hs_status st = launch_potrf(ctx, A, blockID, k, s);
@@ -107,6 +107,7 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
         }
         return HS_OK;
     }
+    HS_REQUIRE(reinterpret_cast<uintptr_t>(A) % 16 == 0, "the matrix must be aligned to 16 bytes");
     // Tensor-core form with lookahead.  The panel TRSM is a product with
     // Y = L_kk^-T.  The chain of columns (bring column k up to date with panel k-1, factor
     // its diagonal block, TRSM) runs on the high-priority side stream, one launch after the

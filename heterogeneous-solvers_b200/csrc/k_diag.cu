@@ -45,7 +45,8 @@ struct DiagArgs {
     int pad_sqrt;         // L is in place: padding rows untouched but for sqrt of their diagonal entry, and
                           // zeros above the diagonal inside the 32 x 32 diagonal blocks
     int write_upper;      // L: the other zeros above the diagonal too
-    double* Y;            // L^-T row major
+    double* Y;            // L^-T row major (null: not written; bsz 256 then keeps that of the first 128 rows in
+                          // L's upper right quadrant until the zeros go there)
     int y_full;           // Y: all of its zeros; else only those beside its 64 x 64 diagonal blocks
     double* T;            // bsz 256: a 128 x 128 scratch block
     float *invHi, *invLo; // L^-1 in FP32 and its low part under TF32 truncation (null: not written)
@@ -432,7 +433,8 @@ __device__ __forceinline__ void store_panel(const Smem m, const Quad q, int p, i
     const int c0 = 32 * p;
     const int hi = lane >> 4, j = c0 + 2 * (lane & 15);  // 16 pairs of columns a row
     const int l0 = q.write_upper ? 0 : c0 / 2, nl = q.L ? kN / 2 - l0 : 0;
-    s1 = min(s1, nl + (q.y_full ? kN : ((p & 1) ? c0 + 32 : c0 + 64)) / 2);
+    if (q.Y) s1 = min(s1, nl + (q.y_full ? kN : ((p & 1) ? c0 + 32 : c0 + 64)) / 2);
+    else s1 = min(s1, nl);
     for (int u0 = s0 + w0; u0 < s1; u0 += 4 * nw) {
         double2 v[4];
 #pragma unroll
@@ -692,7 +694,9 @@ template <int BSZ>
 __global__ void __launch_bounds__(kThreads, 1) diag_factor_kernel(DiagArgs a) {
     const Smem m{};
     const unsigned rank = BSZ == 128 ? 0 : cluster_rank();
-    if (rank == 0) chain128<true>(m, a, quadrant(a, a.in64, a.in32, a.L, a.Y, 0, min(a.valid, kN)));
+    // rows of the upper right quadrant are padding only if L21 has none but padding
+    double* Y11 = BSZ == 128 || a.Y ? a.Y : (a.valid > kN ? a.L + kN : nullptr);
+    if (rank == 0) chain128<true>(m, a, quadrant(a, a.in64, a.in32, a.L, Y11, 0, min(a.valid, kN)));
     if constexpr (BSZ == 256) {
         constexpr int ld = 256, MT = kMT;
         const unsigned nranks = cluster_size();
@@ -704,7 +708,7 @@ __global__ void __launch_bounds__(kThreads, 1) diag_factor_kernel(DiagArgs a) {
         cluster_sync();
         // L21 = A21 Y11, strip by strip of rows through shared memory (in place); Y11 is
         // upper triangular: columns 8 cg .. need k < 8 (cg + 1)
-        for (int st = rank; st < kStrips; st += nranks) {
+        for (int st = rank; st < (Y11 ? kStrips : 0); st += nranks) {
             const int i0 = st * kStrip;
             double* F = m.S;  // the chain is done with it
             __syncthreads();
@@ -715,7 +719,7 @@ __global__ void __launch_bounds__(kThreads, 1) diag_factor_kernel(DiagArgs a) {
             }
             __syncthreads();
             for_groups(warp, true, [&](int cg) {
-                const double* pb = a.Y + (size_t)2 * t * ld + 8 * cg + g;
+                const double* pb = Y11 + (size_t)2 * t * ld + 8 * cg + g;
 #pragma unroll
                 for (int mi = 0; mi < MT; ++mi) acc[mi][0] = acc[mi][1] = 0.0;
 #pragma unroll 4
@@ -768,6 +772,12 @@ __global__ void __launch_bounds__(kThreads, 1) diag_factor_kernel(DiagArgs a) {
         // A22's chain on the first CTA; meanwhile (afterwards, when it is alone) the others
         // form T = Y11 L21^T
         if (rank == 0) chain128<true>(m, a, quadrant(a, a.L, nullptr, a.L, a.Y, kN, valid2));
+        if (!a.Y) {
+            for (int e = rank * kThreads + threadIdx.x; e < min(a.valid, kN) * (kN / 2); e += nranks * kThreads)
+                *reinterpret_cast<double2*>(a.L + (size_t)(e / (kN / 2)) * ld + kN + 2 * (e % (kN / 2))) =
+                    make_double2(0.0, 0.0);
+            return;
+        }
         if (nranks == 1)
             inverse_corner_t(a.Y, L21, a.T, ld, valid2, 0, 1, warp, lane);
         else if (rank != 0)
@@ -852,6 +862,7 @@ hs_status launch_diag_factor(hs_ctx ctx, const DiagFactor& f, cudaStream_t s) {
     if (st != HS_OK) return st;
     const int bsz = ctx->bsz;
     HS_REQUIRE(bsz == 128 || bsz == 256, "the on-chip diagonal block needs matrixBlockSize 128 or 256");
+    HS_REQUIRE(f.Y || (f.in_place && f.zeros), "the inverse is left out in place only");
     DiagArgs a{};
     a.in64 = f.in64;
     a.in32 = f.in32;

@@ -505,11 +505,12 @@ static hs_status potrf_impl(hs_ctx ctx, double* A, int blockID, int blockRow, cu
     const long long row_base = (long long)blockRow * bsz;
     const int64_t rem = ctx->N - row_base;
     const int valid = rem <= 0 ? 0 : (rem < bsz ? (int)rem : bsz);
-    if (bsz == 128 || bsz == 256) {
-        const size_t bb = (size_t)bsz * bsz;
-        st = ensure_scratch(ctx, kSmallScratch + kDiagScratchBlocks * bb * sizeof(double));
-        if (st != HS_OK) return st;
-        DiagFactor f = diag_factor_in_place(ctx, blk);
+    // The on-chip block reads and writes 16 bytes at a time; a matrix that is aligned to its
+    // entries only takes the kernels of the other block sizes.
+    if ((bsz == 128 || bsz == 256) && reinterpret_cast<uintptr_t>(blk) % 16 == 0) {
+        DiagFactor f;
+        f.in64 = f.L = blk;
+        f.in_place = 1;
         f.row_base = row_base;
         return launch_diag_factor(ctx, f, s);
     }
