@@ -92,7 +92,7 @@ Turn::~Turn() {
 hs_status ensure_scratch(hs_ctx ctx, size_t bytes) {
     if (ctx->scratch_bytes >= bytes) return HS_OK;
     size_t want = bytes + bytes / 8;
-    if (want < 1024 * 1024) want = 1024 * 1024;
+    if (want < kScratchLeast) want = kScratchLeast;
     HS_CUDA(cudaStreamSynchronize(ctx->stream));
     if (ctx->side) HS_CUDA(cudaStreamSynchronize(ctx->side));
     if (ctx->side_hi) HS_CUDA(cudaStreamSynchronize(ctx->side_hi));

@@ -159,6 +159,10 @@ constexpr size_t kSmallScratch = 64 * 1024;
 constexpr size_t kScalarOffset = 32 * 1024;
 constexpr size_t kConstOffset = 56 * 1024;
 constexpr int kMaxPartials = 4096;
+// the least that ensure_scratch allocates, and what of it can be asked for without its margin
+// of an eighth passing the least
+constexpr size_t kScratchLeast = 1024 * 1024;
+constexpr size_t kScratchSmall = kScratchLeast / 9 * 8;
 
 // FP64 tensor-core step: d (8 x 8, two entries a lane) += a (8 x 4, one entry) b (4 x 8,
 // one entry); lane l holds a[l/4][l%4], b[l%4][l/4], d[l/4][2(l%4) .. +1]

@@ -268,8 +268,11 @@ hs_status hs_gp_predict(hs_ctx ctx, const double* X, const double* X_test, int64
     const int64_t N = ctx->N, tiles = (N_test + kPredTile - 1) / kPredTile, steps = (N + kPredTile - 1) / kPredTile;
     HS_REQUIRE(tiles < (1LL << 31), "N_test too large");
     // enough ranges of training points for just under six waves of two CTAs an SM (a wave
-    // that is partly empty then costs little), each of at least two steps
-    int64_t splits = std::max<int64_t>(1, std::min<int64_t>({12LL * ctx->num_sms / tiles, steps / 2, 512}));
+    // that is partly empty then costs little), each of at least two steps.  Their parts fit
+    // the scratch that a context has anyway: growing it costs a first call more than the
+    // last few ranges give (N=16384, 5000 test points: 22 -> 21 ranges)
+    const int64_t room = (int64_t)((kScratchSmall - kSmallScratch) / sizeof(double)) / N_test;
+    int64_t splits = std::max<int64_t>(1, std::min<int64_t>({12LL * ctx->num_sms / tiles, steps / 2, 512, room}));
     const int64_t range = (steps + splits - 1) / splits * kPredTile;
     splits = (N + range - 1) / range;
     st = ensure_scratch(ctx, kSmallScratch + (splits > 1 ? (size_t)splits * N_test * sizeof(double) : 0));
