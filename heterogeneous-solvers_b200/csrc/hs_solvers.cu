@@ -215,7 +215,7 @@ hs_status solve_driver(hs_ctx ctx, const double* L, double* b) {
         // reference's 2 nb dependent launches a sweep are latency-bound
         const size_t bb = (size_t)ctx->bsz * ctx->bsz;
         const int64_t n = (int64_t)nb * ctx->bsz;
-        const size_t tq = (size_t)nb * 128 * 128;  // a quadrant a block
+        const size_t tq = ctx->bsz == 256 ? (size_t)nb * 128 * 128 : 0;  // a quadrant a block of 256
         const size_t ybytes = ((size_t)nb * bb + tq + (size_t)n) * sizeof(double);
         hs_status st = ensure_solvews(ctx, ybytes + 256 + sweep_workspace_bytes(nb, ctx->bsz));
         if (st != HS_OK) return st;
