@@ -268,8 +268,9 @@ struct DiagFactor {
     double* L = nullptr;           // factor out
     int in_place = 0;              // L is the packed matrix's own block: zeros above the diagonal, padding rows kept
     int zeros = 1;                 // in place: also the zeros above the 32 x 32 diagonal blocks (0: the panel TRSM's)
-    double* Y = nullptr;           // L^-T, row major (in place with zeros: null for the factor alone, no scratch)
-    int y_full = 0;                // Y: every zero below the diagonal (else those of its 64 x 64 diagonal blocks)
+    // L^-T, row major, with the zeros beside its 64 x 64 diagonal blocks only (in place with
+    // zeros: null for the factor alone, no scratch)
+    double* Y = nullptr;
     double* T = nullptr;           // bsz 256: 128 x 128 doubles of scratch
     float *invHi = nullptr, *invLo = nullptr;  // L^-1 in FP32 and its low part under TF32
     int zero_upper = 0;            // invHi / invLo: also the zeros above the diagonal

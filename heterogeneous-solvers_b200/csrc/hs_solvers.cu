@@ -112,9 +112,8 @@ hs_status factor_driver(hs_ctx ctx, double* A) {
     // Y = L_kk^-T.  The chain of columns (bring column k up to date with panel k-1, factor
     // its diagonal block, TRSM) runs on the high-priority side stream, one launch after the
     // other; the rest of panel k's update, columns k+2 on, runs beside it on the caller's
-    // stream.  Every block sees the same operations in the same order as without
-    // lookahead.  (With the column update on the caller's stream, the chain crossed streams
-    // twice a column.)
+    // stream.  Every block sees its panels in the same order as without lookahead.  (With the
+    // column update on the caller's stream, the chain crossed streams twice a column.)
     const size_t bb = (size_t)bsz * bsz;
     // Large updates go to the INT8 tensor cores (if the digits' workspace can be had).  Panels
     // of 256 one by one from a tile an SM on (a factor at N = 9973: 13.3 -> 8.6 ms).  Two panels

@@ -47,7 +47,7 @@ struct DiagArgs {
     int write_upper;      // L: the other zeros above the diagonal too
     double* Y;            // L^-T row major (null: not written; bsz 256 then keeps that of the first 128 rows in
                           // L's upper right quadrant until the zeros go there)
-    int y_full;           // Y: all of its zeros; else only those beside its 64 x 64 diagonal blocks
+    int y_full;           // Y: all of its zeros (the inverses alone); else only those beside its 64 x 64 diagonal blocks
     double* T;            // bsz 256: a 128 x 128 scratch block
     float *invHi, *invLo; // L^-1 in FP32 and its low part under TF32 truncation (null: not written)
     int zero_upper;       // invHi / invLo: also write the part above the diagonal
@@ -783,7 +783,7 @@ __global__ void __launch_bounds__(kThreads, 1) diag_factor_kernel(DiagArgs a) {
         else if (rank != 0)
             inverse_corner_t(a.Y, L21, a.T, ld, valid2, (int)rank - 1, (int)nranks - 1, warp, lane);
         cluster_sync();
-        inverse_corner_y(a.Y, a.T, ld, a.y_full, rank, nranks, warp, lane, [&](int j, int i, double2 v) {
+        inverse_corner_y(a.Y, a.T, ld, 0, rank, nranks, warp, lane, [&](int j, int i, double2 v) {
             // rows j of the upper right quadrant
             if (a.write_upper && j < a.valid)
                 *reinterpret_cast<double2*>(a.L + (size_t)j * ld + kN + i) = make_double2(0.0, 0.0);
@@ -870,7 +870,6 @@ hs_status launch_diag_factor(hs_ctx ctx, const DiagFactor& f, cudaStream_t s) {
     a.pad_sqrt = f.in_place;
     a.write_upper = f.in_place && f.zeros;
     a.Y = f.Y;
-    a.y_full = f.y_full;
     a.T = f.T;
     a.invHi = f.invHi;
     a.invLo = f.invLo;

@@ -412,17 +412,17 @@ __global__ void __launch_bounds__(256, 1) trsm_dmma_kernel(double* A, int64_t fi
     dmma_tile_t<ROWS, BSZ, 32, ROWS * BSZ / 256, 3, 1>(B, BSZ, B, BSZ, Y, BSZ, BSZ, false, 0, smem);
 }
 
-// L_rk <- L_rk Y_k^T for every off-diagonal block, one CTA per ROWS rows of a block
-template <int BSZ, int ROWS>
+// L_rk <- L_rk Y_k^T for every off-diagonal block, one CTA per 64 rows of a block
+template <int BSZ>
 __global__ void __launch_bounds__(256, 1) scale_panels_kernel(double* L, int nb, const double* __restrict__ Y) {
     extern __shared__ __align__(16) double smem[];
-    constexpr int kSlabs = BSZ / ROWS;
+    constexpr int kRows = 64, kSlabs = BSZ / kRows;
     const int64_t pair = blockIdx.x / kSlabs;  // (r, k), r > k: triangle of nb - 1 columns
     int i, k;
     block_coords(pair, nb - 1, &i, &k);
-    double* B = L + ((size_t)block_id(i + 1, k, nb) * BSZ + (size_t)(blockIdx.x % kSlabs) * ROWS) * BSZ;
-    dmma_tile_t<ROWS, BSZ, 32, ROWS * BSZ / 256, 3, 2>(B, BSZ, B, BSZ, Y + (size_t)k * BSZ * BSZ, BSZ, BSZ, false, 0,
-                                                       smem);
+    double* B = L + ((size_t)block_id(i + 1, k, nb) * BSZ + (size_t)(blockIdx.x % kSlabs) * kRows) * BSZ;
+    dmma_tile_t<kRows, BSZ, 32, kRows * BSZ / 256, 3, 2>(B, BSZ, B, BSZ, Y + (size_t)k * BSZ * BSZ, BSZ, BSZ, false, 0,
+                                                         smem);
 }
 
 // scalar fallback (any bsz): one thread per output element; SYRK follows
@@ -467,9 +467,9 @@ hs_status set_attrs() {
                                  TrsmTile<128, 32>::kSmem));
     HS_CUDA(cudaFuncSetAttribute(trsm_dmma_kernel<256, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  TrsmTile<256, 32>::kSmem));
-    HS_CUDA(cudaFuncSetAttribute(scale_panels_kernel<128, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HS_CUDA(cudaFuncSetAttribute(scale_panels_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  TrsmTile<128, 64>::kSmem));
-    HS_CUDA(cudaFuncSetAttribute(scale_panels_kernel<256, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HS_CUDA(cudaFuncSetAttribute(scale_panels_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  TrsmTile<256, 64>::kSmem));
     HS_CUDA(cudaFuncSetAttribute(trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem(256)));
     HS_CUDA(cudaFuncSetAttribute(potrf_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -569,9 +569,9 @@ hs_status launch_scale_panels(hs_ctx ctx, double* L, const double* Y, cudaStream
     prof_begin(ctx, s, HS_KERNEL_ADJOINT);
     ctx->launches += 1;
     if (bsz == 256)
-        scale_panels_kernel<256, 64><<<(unsigned)grid, 256, TrsmTile<256, 64>::kSmem, s>>>(L, nb, Y);
+        scale_panels_kernel<256><<<(unsigned)grid, 256, TrsmTile<256, 64>::kSmem, s>>>(L, nb, Y);
     else
-        scale_panels_kernel<128, 64><<<(unsigned)grid, 256, TrsmTile<128, 64>::kSmem, s>>>(L, nb, Y);
+        scale_panels_kernel<128><<<(unsigned)grid, 256, TrsmTile<128, 64>::kSmem, s>>>(L, nb, Y);
     HS_CHECK_LAUNCH("scale_panels");
     prof_end(ctx, s, HS_KERNEL_ADJOINT, blocks * n * n * n, 2.0 * blocks * n * n * 8.0);
     return HS_OK;

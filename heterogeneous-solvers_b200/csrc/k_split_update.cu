@@ -14,11 +14,14 @@
 // integer matrix multiplication unit", 2024.)
 //
 // Error of one update, in units of the rows' scales: the digits' 2^-57 a factor, levels
-// past 7 at most 2^-64 a product and the last unit 2^-57; then a rounding of the product and
-// one of C.  The FP64 pipe's chain rounds 64 times at 2^-53 |C|.  Measured, max |A - L L^T| /
-// sqrt(a_ii a_jj) of a factor at N = 4800 (Wishart): 7.6e-15 -> 2.4e-15.  Scale_i scale_j <=
-// 16 max|P_i| max|P_j| <= 16 sqrt(A_ii A_jj), so the factor keeps the plain form's backward
-// error bound relative to sqrt(A_ii A_jj).
+// past 7 at most 1.26 x 2^-64 a product (five products of 2^14 x 2^-80 at level 8) and the
+// last unit 2^-57; then a rounding of the product and one of C.  The FP64 pipe's chain rounds
+// 64 times at 2^-53 |C|.  Measured, max |A - L L^T| / sqrt(a_ii a_jj) of a factor at N = 4800
+// (Wishart): 7.6e-15 -> 2.4e-15.  Scale_i scale_j <= 16.2 max|P_i| max|P_j| <= 16.2 sqrt(A_ii
+// A_jj) (a row's scale is at most 4 / 0.994 times its largest entry), so the factor keeps the
+// plain form's backward error bound relative to sqrt(A_ii A_jj).  It does not keep the plain
+// form's bound by entries, |L| |L|^T: what lies more than 2^-56 below the largest entry of a
+// row's panel (of both, where two go at once) does not enter the product.
 #include "hs_internal.cuh"
 #include "stream_common.cuh"
 #include "tc_common.cuh"

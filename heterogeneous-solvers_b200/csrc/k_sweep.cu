@@ -102,9 +102,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     extern __shared__ uint8_t sweep_smem[];
     // the ring starts at the same offset in every CTA of the cluster
     uint8_t* ring = sweep_smem + ((1024u - (smem_u32(sweep_smem) & 1023u)) & 1023u);
-    constexpr int slots = kSlots;
     double* xs = reinterpret_cast<double*>(ring + (size_t)S * C::kTile);  // x vectors, [slot][BSZ]
-    double* rv = xs + slots * BSZ;                                        // chain: r of the step
+    double* rv = xs + kSlots * BSZ;                                       // chain: r of the step
     double* rslot = rv + BSZ;                                             // chain: the bulk's part of r, [2][32]
     uint64_t* full = reinterpret_cast<uint64_t*>(rslot + 64);
     uint64_t* empty = full + S;
