@@ -93,14 +93,20 @@ hs_status ensure_scratch(hs_ctx ctx, size_t bytes) {
     if (ctx->scratch_bytes >= bytes) return HS_OK;
     size_t want = bytes + bytes / 8;
     if (want < kScratchLeast) want = kScratchLeast;
+    const hs_status st = release_scratch(ctx);
+    if (st != HS_OK) return st;
+    HS_CUDA(cudaMalloc(&ctx->scratch, want));
+    ctx->scratch_bytes = want;
+    return HS_OK;
+}
+
+hs_status release_scratch(hs_ctx ctx) {
     HS_CUDA(cudaStreamSynchronize(ctx->stream));
     if (ctx->side) HS_CUDA(cudaStreamSynchronize(ctx->side));
     if (ctx->side_hi) HS_CUDA(cudaStreamSynchronize(ctx->side_hi));
     if (ctx->scratch) HS_CUDA(cudaFree(ctx->scratch));
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
-    HS_CUDA(cudaMalloc(&ctx->scratch, want));
-    ctx->scratch_bytes = want;
     return HS_OK;
 }
 

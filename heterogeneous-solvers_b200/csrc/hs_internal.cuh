@@ -118,6 +118,8 @@ void prof_end(hs_ctx ctx, cudaStream_t s, int kernel, double flops, double bytes
 // makes sure at least `bytes` of scratch are available (stream-ordered safe:
 // the old buffer is released after a stream sync)
 hs_status ensure_scratch(hs_ctx ctx, size_t bytes);
+// gives it back (no call keeps anything there for the next one)
+hs_status release_scratch(hs_ctx ctx);
 hs_status ensure_work(hs_ctx ctx, size_t bytes);
 hs_status ensure_mixed(hs_ctx ctx, size_t bytes);
 hs_status ensure_gp(hs_ctx ctx, size_t bytes);

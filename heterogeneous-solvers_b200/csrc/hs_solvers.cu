@@ -208,16 +208,28 @@ hs_status solve_driver(hs_ctx ctx, const double* L, double* b) {
     const int nb = ctx->nb;
     const int64_t T = total_blocks(nb);
     cudaStream_t s = ctx->stream;
-    if ((ctx->bsz == 128 || ctx->bsz == 256) && nb > 1) {
+    const size_t bb = block_elems(ctx);
+    const int64_t n = (int64_t)nb * ctx->bsz;
+    const size_t tq = ctx->bsz == 256 ? (size_t)nb * 128 * 128 : 0;  // a quadrant a block of 256
+    const size_t ybytes = ((size_t)nb * bb + tq + (size_t)n) * sizeof(double);
+    bool whole = (ctx->bsz == 128 || ctx->bsz == 256) && nb > 1;
+    if (whole) {
+        // A matrix that leaves no room for the workspace is solved block by block below; but
+        // first what the factor's digits took is given back.
+        const size_t bytes = ybytes + 256 + sweep_workspace_bytes(nb, ctx->bsz);
+        hs_status st = ensure_solvews(ctx, bytes);
+        if (st == HS_ERR_OOM && ctx->scratch_bytes > kScratchLeast) {
+            if ((st = release_scratch(ctx)) != HS_OK) return st;
+            st = ensure_solvews(ctx, bytes);
+        }
+        if (st != HS_OK && st != HS_ERR_OOM) return st;
+        whole = st == HS_OK;
+    }
+    if (whole) {
         // both sweeps as single launches over the FP64 factor, with the diagonal solves as
         // products with Y_k = L_kk^-T formed for all blocks in one batched launch first; the
         // reference's 2 nb dependent launches a sweep are latency-bound
-        const size_t bb = (size_t)ctx->bsz * ctx->bsz;
-        const int64_t n = (int64_t)nb * ctx->bsz;
-        const size_t tq = ctx->bsz == 256 ? (size_t)nb * 128 * 128 : 0;  // a quadrant a block of 256
-        const size_t ybytes = ((size_t)nb * bb + tq + (size_t)n) * sizeof(double);
-        hs_status st = ensure_solvews(ctx, ybytes + 256 + sweep_workspace_bytes(nb, ctx->bsz));
-        if (st != HS_OK) return st;
+        hs_status st;
         double* Y = static_cast<double*>(ctx->solvews);
         double* T = Y + (size_t)nb * bb;
         double* tmp = T + tq;

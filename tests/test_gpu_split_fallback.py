@@ -113,3 +113,37 @@ def test_mixed_gradient_through_the_int8_inverse(hs, ctx, prec):
     exact = hs.gp_nlml_grad(ctx, X, y, theta)[1]
     for got in grads:
         assert np.linalg.norm(got - exact) <= 5e-2 * np.linalg.norm(exact)
+
+
+def test_solve_without_room_for_its_workspace(hs):
+    """The solve's workspace (18 MB here) comes after the factor's digits (30 MB), which are given
+    back for it; where even that does not help, the solve goes block by block without one."""
+    N, bsz = 7168, 256
+    X, y = _data(N)
+    A = hs.SymmetricMatrix(N, bsz, device="cuda:0")
+    b = hs.RightHandSide(N, bsz, device="cuda:0")
+    K = torch.exp(-2.0 * torch.cdist(X, X, compute_mode="donot_use_mm_for_euclid_dist").square())
+    K.diagonal().add_(SN2)
+    with hs.Context(device=0, N=N, matrixBlockSize=bsz) as warm:
+        hs.MatrixGenerator.assemble(warm, A.matrixData, X, 0.5, SF2, SN2)
+        hs.TriangularSystemSolver(A, hs.Cholesky(A, warm).solve_heterogeneous().A_gpu, b, warm).solve()
+        for k in (0, 1):  # loads the operators' kernels
+            hs.MatrixVectorOperations.triangularSolveBlockVector(warm, A.matrixData, b.rightHandSideData, 0, 0, k)
+            hs.MatrixVectorOperations.matrixVectorColumnUpdate(warm, A.matrixData, b.rightHandSideData, 1 - k, 1, k,
+                                                               hs.block_id(k, k, N // bsz), N // bsz, k)
+    solved = []
+    for with_digits in (True, False):
+        with hs.Context(device=0, N=N, matrixBlockSize=bsz) as c:
+            if with_digits:
+                hs.MatrixGenerator.assemble(c, A.matrixData, X, 0.5, SF2, SN2)
+                hs.Cholesky(A, c).solve_heterogeneous()
+            b.rightHandSideData.copy_(y)
+            with Full(6 << 20):
+                before = c.launch_count()
+                hs.TriangularSystemSolver(A, A.matrixData, b, c).solve()
+                solved.append((b.rightHandSideData.clone(), c.launch_count() - before))
+    (x, few), (blockwise, many) = solved
+    assert few <= 4 and many >= 2 * (N // bsz)
+    for v in (x, blockwise):
+        r = torch.linalg.norm(K @ v - y)
+        assert r <= 8 * N * 2.0 ** -52 * torch.linalg.norm(K) * torch.linalg.norm(v)
