@@ -214,6 +214,7 @@ hs_status solve_driver(hs_ctx ctx, const double* L, double* b) {
     const size_t ybytes = ((size_t)nb * bb + tq + (size_t)n) * sizeof(double);
     bool whole = (ctx->bsz == 128 || ctx->bsz == 256) && nb > 1;
     if (whole) {
+        HS_REQUIRE(reinterpret_cast<uintptr_t>(L) % 16 == 0, "the factor must be aligned to 16 bytes");
         // A matrix that leaves no room for the workspace is solved block by block below; but
         // first what the factor's digits took is given back.
         const size_t bytes = ybytes + 256 + sweep_workspace_bytes(nb, ctx->bsz);

@@ -418,6 +418,7 @@ hs_status cg_persistent(hs_ctx ctx, const double* A, const double* b, double* x,
                         int64_t* iters_out, double* dnew_out, double* d0_out) {
     const int nb = ctx->nb, bsz = ctx->bsz;
     HS_REQUIRE(bsz == 128 || bsz == 256, "the persistent CG supports matrixBlockSize 128 or 256");
+    HS_REQUIRE(reinterpret_cast<uintptr_t>(A) % 16 == 0, "the matrix must be aligned to 16 bytes");
     cudaStream_t s = ctx->stream;
     const int64_t n = (int64_t)nb * bsz;
     CgArgs a{};

@@ -50,11 +50,15 @@ def test_factor_of_one_block_at_any_alignment(hs, ctx, bsz, N):
     _check(A.matrixData, M, K, N, bsz)
 
 
-def test_larger_factor_wants_16_bytes(hs, ctx):
+def test_several_blocks_want_16_bytes(hs, ctx):
+    """Refused on the host (the copies into shared memory always needed it)."""
     A = hs.SymmetricMatrix(300, 128, device="cuda:0")
     A.matrixData = torch.zeros(A.matrixData.numel() + 1, dtype=torch.float64, device="cuda")[1:]
-    with pytest.raises(hs.HSError, match="16 bytes"):
-        hs.Cholesky(A, ctx).solve_heterogeneous()
+    b = hs.RightHandSide(300, 128, device="cuda:0")
+    for call in (hs.Cholesky(A, ctx).solve_heterogeneous, hs.TriangularSystemSolver(A, A.matrixData, b, ctx).solve,
+                 hs.CG(A, b, ctx).solveHeterogeneous):
+        with pytest.raises(hs.HSError, match="16 bytes"):
+            call()
 
 
 @pytest.mark.parametrize("bsz,N", [(128, 128), (256, 256)])
