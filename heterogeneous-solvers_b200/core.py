@@ -477,8 +477,8 @@ def cholesky_adjoint(ctx, L, Abar):
 
 def gp_nlml_grad(ctx, X, y, theta, n_ell=None, precision=None, tol=1e-14):
     """GP negative log marginal likelihood and its gradient with respect to
-    theta = [log l_1..log l_n_ell, log sf2, log sn2] (FP64 factor, reverse-mode
-    Cholesky and an on-the-fly dK/dtheta contraction).  X (N x d) and y (N)
+    theta = [log l_1..log l_n_ell, log sf2, log sn2] (FP64 factor, inverse and
+    an on-the-fly dK/dtheta contraction).  X (N x d) and y (N)
     may be host or device float64 arrays; returns (nlml, grad ndarray, report).
     With ``precision`` ("tf32x3", "bf16x3" or "f16x3") the factor is the
     mixed-precision one (hs_gp_nlml_grad_mixed): alpha refined in FP64 to the

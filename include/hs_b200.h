@@ -86,12 +86,13 @@ typedef enum hs_kernel_id {
     HS_KERNEL_UPDATE = 0,    /* SYRK + GEMM trailing update (FP64) */
     HS_KERNEL_POTRF = 1,
     HS_KERNEL_TRSM = 2,
-    HS_KERNEL_SYMV = 3,      /* symmetric block matvec, both phases */
+    HS_KERNEL_SYMV = 3,      /* symmetric block matvec, both phases; a CG launch of blocks of 128 or
+                                256 runs many iterations: flops and bytes of all its passes */
     HS_KERNEL_TRSV = 4,
     HS_KERNEL_COLUPD = 5,
     HS_KERNEL_ASSEMBLE = 6,
     HS_KERNEL_VECTOR = 7,    /* vector ops, dots, CG updates */
-    HS_KERNEL_ADJOINT = 8,   /* reverse-mode Cholesky block products (FP64 DMMA) */
+    HS_KERNEL_ADJOINT = 8,   /* block products of the reverse-mode Cholesky and of the inverse */
     HS_KERNEL_GRAD = 9,      /* GP gradient contraction */
     HS_KERNEL_UPDATE_SIDE = 10, /* mixed factor: trailing-update launches on the look-ahead stream
                                    (flops are counted where the tiles are: the in-group updates
@@ -245,11 +246,23 @@ hs_status hs_rbf_assemble(hs_ctx ctx, double* A, const double* X, int d, const d
 /* Cholesky::solve_heterogeneous with the whole matrix on the GPU
  * (src/solver/cholesky/Cholesky.cpp:413-493): A (packed, device) is overwritten
  * by L.  *info (host, may be NULL) = -1 on success, else the global row of the
- * first non-positive pivot (then HS_ERR_NOT_SPD). */
+ * first non-positive pivot (then HS_ERR_NOT_SPD).
+ * With blocks of 128 or 256 A must be aligned to 16 bytes (one block alone to 8), and the
+ * large trailing updates run in fixed point: each row of a panel (of two at once, where
+ * that pays) as 56-bit numbers with one power-of-two scale, products exact in integers,
+ * one rounding to FP64.  The backward error keeps its bound relative to sqrt(a_ii a_jj), and
+ * measured no larger than that of FP64 products; what lies more than 2^-56 below the
+ * largest entry of its row's panel does not enter a product, so the tighter entrywise bound
+ * |L| |L|^T does not hold.  Their workspace (up to 3.6 KB a row) stays with the context
+ * (hs_ctx_release_buffers); where it cannot be had the updates take FP64 products, and the
+ * result other bits. */
 hs_status hs_cholesky_factor(hs_ctx ctx, double* A, int64_t* info);
 
 /* TriangularSystemSolver::solve (TriangularSystemSolver.cpp:15-105): b <- L^-T L^-1 b
- * in place (device). */
+ * in place (device).  L aligned to 16 bytes with blocks of 128 or 256.  Solves and
+ * hs_cg_solve of several contexts of a device take turns (their kernels' CTAs wait for one
+ * another); with several contexts the call first waits on the host for what is queued
+ * before it. */
 hs_status hs_cholesky_solve(hs_ctx ctx, const double* L, double* b);
 
 /* CG::solveHeterogeneous with the whole matrix on the GPU (src/solver/cg/CG.cpp:38-163):
@@ -367,9 +380,10 @@ hs_status hs_cholesky_adjoint(hs_ctx ctx, const double* L, double* Abar);
  *   *nlml = 1/2 y^T K^-1 y + 1/2 log|K| + N/2 log 2pi
  *   grad[q] = dNLML/dtheta_q = 1/2 tr((K^-1 - alpha alpha^T) dK/dtheta_q)
  * (host, n_ell + 2 values; may be NULL).  FP64 factor on the tensor cores,
- * the gradient through hs_cholesky_adjoint of sum log L_ii and an on-the-fly
+ * the gradient through K^-1 (from 13 block rows of 256 on by the fixed-point products of
+ * hs_cholesky_factor, else in FP64) and an on-the-fly
  * contraction that recomputes dK/dtheta from X (nothing of size N^2 besides L
- * and its adjoint is stored; that workspace is kept by the context between
+ * and K^-1 is stored; that workspace is kept by the context between
  * calls, see hs_ctx_release_buffers).  d <= 32; matrixBlockSize 128 or 256.  Returns
  * HS_ERR_NOT_SPD when K(theta) has no Cholesky factor. */
 typedef struct hs_gp_report {
@@ -383,7 +397,7 @@ hs_status hs_gp_nlml_grad(hs_ctx ctx, const double* X, const double* y, int d, c
 /* The same NLML and gradient through the mixed-precision factor (no reference
  * counterpart): the factor of hs_mixed_solve with `precision` (HS_PRECISION_*),
  * alpha = K^-1 y refined in FP64 to the backward error `tol`, log|K| from the
- * factor's FP64 diagonal blocks, and the FP64 reverse sweep run on the mixed
+ * factor's FP64 diagonal blocks, and the inverse from the mixed
  * factor widened to FP64.  alpha (hence the data-fit term) has FP64 accuracy;
  * log|K| and the trace term 1/2 tr(K^-1 dK/dtheta) carry the error of the
  * low-precision factor (K~ = L~ L~^T = K + E gives log|K~| - log|K| =
